@@ -936,7 +936,7 @@ def main():
     ap.add_argument("--cpu-threads", type=int, default=0, help="reference arm: host threads (default: all)")
     ap.add_argument("--ncu-case", action="store_true", help="build + warm-up ticks only (for ncu captures)")
     ap.add_argument("--ncu-density", type=int, default=-1,
-                    help="ncu case: density kernel (0 walk, 1 grouped; default: the handle's)")
+                    help="ncu case: density value of the tuning (0 or 1, the same kernel; default: the handle's)")
     ap.add_argument("--ncu-block", type=int, default=0,
                     help="ncu case of dam10m: an N^3 fluid block in the same tank (bins still doubled)")
     args = ap.parse_args()

@@ -275,11 +275,9 @@ vxl_status vxl_sph_reactions_all(vxl_sph_handle* h, vxl_sph_reaction* out, uint3
 /* Launch shape of the particle passes: threads per block (128 or 256), slots per tile
  * (a multiple of 128, at least one block) and the scheduling: waves = 0 runs one block
  * per tile, waves = k > 0 runs k x the occupancy limit of persistent blocks that draw
- * tiles from a counter. density selects the density kernel of scenes without provider
- * walls: VXL_SPH_DENSITY_WALK (one thread per particle walking its own cells, threads
- * ordered by cell octant) or VXL_SPH_DENSITY_GROUPED (eight lanes per cell octant sharing
- * one staged stream of candidates); both give the same results. Default {256, 256, 0,
- * WALK}. */
+ * tiles from a counter. density once chose between two density kernels with the same
+ * results; both values are accepted and reported back, and run the one walk there is
+ * now. Default {256, 256, 0, WALK}. */
 #define VXL_SPH_DENSITY_WALK 0u
 #define VXL_SPH_DENSITY_GROUPED 1u
 typedef struct vxl_sph_tuning {
@@ -293,8 +291,7 @@ typedef struct vxl_sph_tuning {
 vxl_status vxl_sph_set_tuning(vxl_sph_handle* h, const vxl_sph_tuning* t);
 vxl_status vxl_sph_get_tuning(vxl_sph_handle* h, vxl_sph_tuning* t);
 /* Autotuner: times every candidate shape on the handle's own scenes (`trials` substeps
- * each, from a snapshot of the state that is restored afterwards) and keeps the fastest;
- * then times the other density kernels at that shape and keeps the fastest.
+ * each, from a snapshot of the state that is restored afterwards) and keeps the fastest.
  * Results are identical for every shape; only the time differs. */
 vxl_status vxl_sph_autotune(vxl_sph_handle* h, float dt_tick, uint32_t trials, vxl_sph_tuning* best);
 

@@ -23,7 +23,8 @@ struct GridBox {
   float bin;
   uint32_t nx, ny, nz;
   uint32_t total;
-  uint32_t pad[3];
+  uint32_t reach_q;  // candidate filter: the squared reach in cell units of 1/64 bin (sub_word below)
+  uint32_t pad[2];
 };
 
 // Constants of one scene, computed on the host exactly as FluidSystem::new does
@@ -66,6 +67,42 @@ __device__ __forceinline__ uint32_t cell_index(const GridBox& g, float x, float 
   bin_of(g, x, y, z, cx, cy, cz);
   uint32_t idx = (cx * g.ny + cy) * g.nz + cz;
   return min(idx, g.total - 1u);
+}
+
+// Cell of the engine's own table: z outermost, x innermost. The neighbour walk takes its 27
+// cells in (dz, dy, dx) order, so in this order the three cells of a (dz, dy) row are one
+// run of slots, in walk order. (The reference's table has x outermost; the export converts.)
+__device__ __forceinline__ uint32_t cell_slot(const GridBox& g, float x, float y, float z) {
+  uint32_t cx, cy, cz;
+  bin_of(g, x, y, z, cx, cy, cz);
+  return min((cz * g.ny + cy) * g.nx + cx, g.total - 1u);
+}
+
+// Candidate filter of the density walk. A slot's position inside its cell, in 1/64 of a bin
+// (0..63 per axis), is kept in three 32-bit words, one for each residue p of an observer's x
+// cell modulo 3: seen from there the slot's cell is the left, middle or right one of a row, so
+// word p holds b = (64 ((cx - p + 1) mod 3) + x - 96, y - 32, z - 32) as signed bytes and
+// floor(|b|^2 / 90) in byte 3 (|b|^2 <= 11264: at most 125). A particle at sub-cell position q
+// in a cell of residue p sees the whole row at offset (dy, dz) from A = (q.x - 32, q.y - 64 dy
+// - 32, q.z - 64 dz - 32), and |b - A|^2 = 2 (|b|^2 / 2 - A.b) + |A|^2: with M = (-A, 45) as signed
+// bytes, one four-way byte dot product per candidate, word . M <= |b|^2 / 2 - A.b, decides
+// |b - A|^2 <= T conservatively. A slot the filter drops is farther than sqrt(T); one it keeps is
+// tested exactly. T = (64 h / bin + 2.5)^2: flooring two positions moves their difference by
+// less than 1 per axis (sqrt(3) in all), and the f32 rounding of (v - o) * inv by at most 0.19
+// per axis and particle at the largest grid (16,384 cells of 64). Positions outside the grid's
+// cells are clamped into the last one, which never moves two particles apart, so the filter
+// stays conservative there.
+constexpr uint32_t kSubUnits = 64;
+constexpr uint32_t kSubNorm = 45;  // |b|^2 / 2 is kept in multiples of this
+
+__device__ __forceinline__ int axis_sub(float o, float v, float inv, uint32_t c) {
+  const float f = (v - o) * inv * (float)kSubUnits - (float)c * (float)kSubUnits;  // power-of-two scaling: exact
+  return (int)fminf(fmaxf(f, 0.0f), (float)(kSubUnits - 1));
+}
+
+__device__ __forceinline__ uint32_t sub_word(int bx, int by, int bz) {
+  const uint32_t norm = (uint32_t)(bx * bx + by * by + bz * bz) / (2 * kSubNorm);
+  return (uint32_t)(bx & 255) | ((uint32_t)(by & 255) << 8) | ((uint32_t)(bz & 255) << 16) | (norm << 24);
 }
 
 // Tait EOS with the free-surface clamp: crates/vxl-phys-fluid/src/fluid_force.rs:11-29.
@@ -117,6 +154,8 @@ __device__ inline bool grid_box(float lox, float loy, float loz, float hix, floa
   g.ny = dims[1];
   g.nz = dims[2];
   g.total = dims[0] * dims[1] * dims[2];
+  const float reach = (float)kSubUnits * (h / bin) + 2.5f;  // at most 66.5: bin >= h
+  g.reach_q = (uint32_t)ceilf(reach * reach);
   return ok;
 }
 

@@ -33,14 +33,13 @@ inline uint32_t blocks_for(uint64_t n, int t = kThreads) { return (uint32_t)((n 
 
 enum KernelId : int {
   KID_CELLOFF, KID_KEYS, KID_SCAN_PARTIAL, KID_SCAN_FINAL, KID_PLACE, KID_CANON,
-  KID_DENSITY, KID_FORCE, KID_BFORCE, KID_REACT_LONG, KID_REACT_SPANS, KID_SCALE, KID_HALFMASK, KID_WALLS,
+  KID_DENSITY, KID_FORCE, KID_BFORCE, KID_REACT_LONG, KID_REACT_SPANS, KID_SCALE, KID_WALLS,
   KID_GROUPS, KID_COUNT
 };
 const char* const kKernelNames[KID_COUNT] = {
     "k_celloff", "k_keys", "k_scan_partial", "k_scan_final", "k_place", "k_canon",
-    "k_density", "k_force", "k_bforce", "k_react_long", "k_react_spans", "k_scale", "k_halfmask", "k_walls",
+    "k_density", "k_force", "k_bforce", "k_react_long", "k_react_spans", "k_scale", "k_walls",
     "k_groups"};
-constexpr int kSegWarps = 8;  // warps per block of the grouped density pass
 
 constexpr size_t kSceneHostBytes = offsetof(SceneDev, g);
 
@@ -91,9 +90,8 @@ namespace vxl {
 
 uint64_t Engine::bytes_per_slot(uint32_t nbr_cap) {
   // pos, vel (x2), orig, slot_of, cellrank, items, rc, press, acc, xsph, bforce, bpos,
-  // neighbour list + count, staging, half masks, density thread orders (walls variant and
-  // grouped pass), density segments
-  return 4 * 16 + 4 + 4 + 8 + 8 + 8 + 4 + 16 + 16 + 16 + 16 + (uint64_t)nbr_cap * 2 + 4 + 32 + 1 + 4 + 4 + 8;
+  // neighbour list + count, staging, candidate-filter words, density thread order
+  return 4 * 16 + 4 + 4 + 8 + 8 + 8 + 4 + 16 + 16 + 16 + 16 + (uint64_t)nbr_cap * 2 + 4 + 32 + 12 + 4;
 }
 
 uint64_t Engine::bytes_per_cell() { return 12; }  // counts, start, wet
@@ -170,13 +168,12 @@ vxl_status Engine::alloc_all() {
   A(dalloc((float4**)&bpos_, n));
   A(dalloc(&nbr_, (size_t)nbr_cap_ * n));
   A(dalloc(&nbr_n_, n));
-  A(dalloc(&halves_, 4 * (n / 32 + 2)));
+  wstride_ = (uint32_t)((n + 32 + 3) & ~size_t(3));  // the walk reads whole 16-byte groups, up to 32 words past the end
+  A(dalloc(&words_, 3ull * wstride_));
   A(dalloc(&stage_, 8 * n));
   A(dalloc(&counts_, cell_cap_ + 1));
   A(dalloc(&wet_, cell_cap_ + 1));
-  A(dalloc(&xorder_, slot_cap_));
   A(dalloc(&order_, slot_cap_));
-  A(dalloc((uint2**)&segs_, slot_cap_));
   A(dalloc(&start_, cell_cap_ + 1));
   A(dalloc(&partial_, cell_cap_ / kScanTile + 2));
   A(dalloc(&sc_d_, scene_cap_));
@@ -206,7 +203,7 @@ void Engine::free_all() {
   if (graph_) cudaGraphExecDestroy(graph_);
   graph_ = nullptr;
   void* d[] = {pos_[0], pos_[1], vel_[0], vel_[1], orig_, slot_of_, cellrank_, items_, rc_, press_, acc_, xsph_,
-               bforce_, bpos_, nbr_, nbr_n_, halves_, xorder_, order_, segs_, stage_, counts_, wet_, start_, partial_, sc_d_, tiles_d_, ctl_d_, spans_d_,
+               bforce_, bpos_, nbr_, nbr_n_, words_, order_, stage_, counts_, wet_, start_, partial_, sc_d_, tiles_d_, ctl_d_, spans_d_,
                longs_d_, breact_d_};
   for (void* p : d)
     if (p) cudaFree(p);
@@ -291,9 +288,6 @@ void Engine::set_tuning(const Tuning& t) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_f, k_e_force<256>, 256, 0);
   }
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_b, k_e_bforce, 128, 0);
-  int occ_s = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_e_density_seg<kSegWarps>, kSegWarps * 32, 0);
-  grid_seg_ = sms * std::max(1, occ_s);
   cudaGetLastError();
   // waves == 0: one block per tile (the grid is sized from the tile count at launch)
   grid_density_ = sms * std::max(1, occ_d) * (int)tuning_.waves;
@@ -1146,25 +1140,29 @@ vxl_status Engine::export_grid(uint32_t q, uint32_t* items, uint32_t* start, uin
     info->dims[2] = rec.g.nz;
     info->total = total;
   }
-  uint32_t* tmp = (uint32_t*)stage_;
-  if (start) {
-    if (start_cap < total + 1) return set_error(VXL_SIZE_MISMATCH, "start buffer smaller than cells + 1");
-    // the scene's slice of the global table, rebased to scene-local slots on the host
-    CU(cudaMemcpyAsync(start, start_ + rec.cell_off, (total + 1) * 4, cudaMemcpyDeviceToHost, stream_));
-    CU(cudaStreamSynchronize(stream_));
-    for (uint64_t c = 0; c <= total; ++c) start[c] -= rec.base;
+  if (start && start_cap < total + 1) return set_error(VXL_SIZE_MISMATCH, "start buffer smaller than cells + 1");
+  if (!start && !(items && n) && !(bins && n)) return VXL_OK;
+  uint32_t* ref_start = nullptr;  // the table in the reference's cell order
+  if (cudaMalloc((void**)&ref_start, (total + 1) * 4) != cudaSuccess) {
+    cudaGetLastError();
+    return set_error(VXL_OUT_OF_MEMORY, "no device memory for the exported table");
   }
-  if (items && n) {
-    k_e_export_items<<<blocks_for(n), kThreads, 0, stream_>>>(orig_, si.base, n, tmp);
-    CU(cudaMemcpyAsync(items, tmp, (size_t)n * 4, cudaMemcpyDeviceToHost, stream_));
-    CU(cudaStreamSynchronize(stream_));
-  }
-  if (bins && n) {
-    k_e_export_bins<<<blocks_for(std::max<uint64_t>(total, 1)), kThreads, 0, stream_>>>(start_, orig_, sc_d_, q, tmp);
-    CU(cudaMemcpyAsync(bins, tmp, (size_t)n * 4, cudaMemcpyDeviceToHost, stream_));
-    CU(cudaStreamSynchronize(stream_));
-  }
-  CU(cudaGetLastError());
+  uint32_t* d_items = (uint32_t*)stage_;
+  uint32_t* d_bins = d_items + n;
+  const uint32_t blocks = blocks_for(total + 1);
+  k_e_export_counts<<<blocks, kThreads, 0, stream_>>>(start_, sc_d_, q, ref_start);
+  k_e_export_scan<<<1, 1024, 0, stream_>>>(ref_start, (uint32_t)(total + 1));
+  if (n)
+    k_e_export_table<<<blocks, kThreads, 0, stream_>>>(start_, orig_, sc_d_, q, ref_start, items ? d_items : nullptr,
+                                                       bins ? d_bins : nullptr);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && start)
+    e = cudaMemcpyAsync(start, ref_start, (total + 1) * 4, cudaMemcpyDeviceToHost, stream_);
+  if (e == cudaSuccess && items && n) e = cudaMemcpyAsync(items, d_items, (size_t)n * 4, cudaMemcpyDeviceToHost, stream_);
+  if (e == cudaSuccess && bins && n) e = cudaMemcpyAsync(bins, d_bins, (size_t)n * 4, cudaMemcpyDeviceToHost, stream_);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
+  cudaFree(ref_start);
+  if (e != cudaSuccess) return set_error(VXL_CUDA_ERROR, std::string("export: ") + cudaGetErrorString(e));
   return VXL_OK;
 }
 
@@ -1420,26 +1418,17 @@ void Engine::enqueue_substep(bool with_reactions) {
   join_side_only();
   LAUNCH(KID_CELLOFF, k_e_celloff<<<1, 1024, 0, st>>>(sc_d_, S, ctl_d_, (uint32_t)cell_cap_));
   LAUNCH(KID_KEYS, k_e_keys<<<key_blocks, kThreads, 0, st>>>(p0, sc_d_, tiles_d_, ntiles_, ctl_d_, counts_,
-                                                             (uint2*)cellrank_, halves_,
-                                                             (uint32_t)(4 * (used_ / 32 + 1)), wet_));
+                                                             (uint2*)cellrank_, wet_));
   LAUNCH(KID_SCAN_PARTIAL, k_e_scan_partial<<<148 * 4, kScanThreads, 0, st>>>(counts_, ctl_d_, partial_, start_));
   LAUNCH(KID_SCAN_FINAL, k_e_scan_final<<<148 * 4, kScanThreads, 0, st>>>(counts_, ctl_d_, partial_, start_));
   LAUNCH(KID_PLACE, k_e_place<<<key_blocks, kThreads, 0, st>>>((const uint2*)cellrank_, start_, orig_, tiles_d_,
                                                                ntiles_, ctl_d_, (uint2*)items_));
   LAUNCH(KID_CANON, k_e_canon<<<148 * 8, 256, 0, st>>>((const uint2*)items_, start_, ctl_d_, p0, v0, (float4*)pos_[1],
                                                        (float4*)vel_[1], orig_, slot_of_));
-  // half-cell masks and the thread order of the density pass: for the provider-wall variant
-  // the masks, then x halves first per cell; otherwise the masks with the octant-major order
-  // per chunk of a tile (and the segments of the grouped kernel) in one pass
-  if (walls_any_) {
-    LAUNCH(KID_HALFMASK, k_e_halfmask<<<key_blocks, kThreads, 0, st>>>(p1, sc_d_, tiles_d_, ntiles_, ctl_d_, halves_));
-    LAUNCH(KID_HALFMASK, k_e_xorder<<<148 * 8, kThreads, 0, st>>>(start_, ctl_d_, halves_, xorder_));
-  } else {
-    LAUNCH(KID_GROUPS, k_e_groups<<<key_blocks, kGroupChunk, 0, st>>>(p1, sc_d_, tiles_d_, ntiles_, ctl_d_, order_,
-                                                                      (uint2*)segs_, halves_));
-  }
+  // the candidate-filter words, and at doubled bins the density pass's thread order
+  LAUNCH(KID_GROUPS, k_e_groups<<<key_blocks, kGroupChunk, 0, st>>>(p1, sc_d_, tiles_d_, ntiles_, ctl_d_, order_, words_,
+                                                                    wstride_));
   const uint32_t stride = (uint32_t)slot_cap_;
-  const uint32_t* walk_order = order_;
   const bool rec = record_;
   const uint32_t per_tile = std::max<uint32_t>(ntiles_, 1);
   const uint32_t gd = grid_density_ ? (uint32_t)grid_density_ : per_tile;
@@ -1448,24 +1437,20 @@ void Engine::enqueue_substep(bool with_reactions) {
   if (walls_any_) {  // provider walls: the variant with mirror ghosts
     if (tuning_.block == 128)
       LAUNCH(KID_DENSITY, k_e_density<128, true><<<gd, 128, 0, st>>>(
-                              p1, start_, sc_d_, tiles_d_, ntiles_, ctl_d_, halves_, (float2*)rc_, press_, nbr_, nbr_n_,
-                              nbr_cap_, stride, wet_, xorder_, prov_d_, wplanes_d_, orig_, ctab(0)));
+                              p1, start_, sc_d_, tiles_d_, ntiles_, ctl_d_, words_, wstride_, (float2*)rc_, press_, nbr_, nbr_n_,
+                              nbr_cap_, stride, wet_, order_, prov_d_, wplanes_d_, orig_, ctab(0)));
     else
       LAUNCH(KID_DENSITY, k_e_density<256, true><<<gd, 256, 0, st>>>(
-                              p1, start_, sc_d_, tiles_d_, ntiles_, ctl_d_, halves_, (float2*)rc_, press_, nbr_, nbr_n_,
-                              nbr_cap_, stride, wet_, xorder_, prov_d_, wplanes_d_, orig_, ctab(0)));
-  } else if (tuning_.density == 1) {
-    LAUNCH(KID_DENSITY, k_e_density_seg<kSegWarps><<<grid_seg_, kSegWarps * 32, 0, st>>>(
-                            p1, start_, sc_d_, ctl_d_, halves_, order_, (const uint2*)segs_, (float2*)rc_, press_, nbr_,
-                            nbr_n_, nbr_cap_, stride, wet_));
+                              p1, start_, sc_d_, tiles_d_, ntiles_, ctl_d_, words_, wstride_, (float2*)rc_, press_, nbr_, nbr_n_,
+                              nbr_cap_, stride, wet_, order_, prov_d_, wplanes_d_, orig_, ctab(0)));
   } else if (tuning_.block == 128) {
-    LAUNCH(KID_DENSITY, k_e_density<128><<<gd, 128, 0, st>>>(p1, start_, sc_d_, tiles_d_, ntiles_, ctl_d_, halves_,
+    LAUNCH(KID_DENSITY, k_e_density<128><<<gd, 128, 0, st>>>(p1, start_, sc_d_, tiles_d_, ntiles_, ctl_d_, words_, wstride_,
                                                              (float2*)rc_, press_, nbr_, nbr_n_, nbr_cap_, stride, wet_,
-                                                             walk_order));
+                                                             order_));
   } else {
-    LAUNCH(KID_DENSITY, k_e_density<256><<<gd, 256, 0, st>>>(p1, start_, sc_d_, tiles_d_, ntiles_, ctl_d_, halves_,
+    LAUNCH(KID_DENSITY, k_e_density<256><<<gd, 256, 0, st>>>(p1, start_, sc_d_, tiles_d_, ntiles_, ctl_d_, words_, wstride_,
                                                              (float2*)rc_, press_, nbr_, nbr_n_, nbr_cap_, stride, wet_,
-                                                             walk_order));
+                                                             order_));
   }
   // Reaction branch on the side stream: it reads only the sorted buffer, the densities and
   // the lists, so it runs beside the force pass (which writes the other buffer).
@@ -1747,31 +1732,6 @@ vxl_status Engine::autotune(float dt_tick, uint32_t trials, Tuning* best, float*
           best_t = tuning_;
         }
       }
-  // the other density kernels at the best shape (provider-wall scenes use their own variant)
-  for (uint32_t dv = 0; st == VXL_OK && !walls_any_ && dv < 2; ++dv) {
-    if (dv == best_t.density) continue;
-    Tuning other = best_t;
-    other.density = dv;
-    st = copy_all(false);
-    if (st != VXL_OK) break;
-    set_tuning(other);
-    enqueue_substep(false);
-    cudaEventRecord(e0, stream_);
-    for (uint32_t r = 0; r < trials; ++r) enqueue_substep(false);
-    join_side();
-    cudaEventRecord(e1, stream_);
-    if (cudaStreamSynchronize(stream_) != cudaSuccess) {
-      st = set_error(VXL_CUDA_ERROR, "autotune trial failed");
-      break;
-    }
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    ms /= (float)trials;
-    if (ms < best_v) {
-      best_v = ms;
-      best_t = tuning_;
-    }
-  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (st == VXL_OK) st = copy_all(false);

@@ -14,32 +14,33 @@
 // [cell_off_q, cell_off_q + cells_q), assigned in scene order. A particle's key is
 // cell_off_q + its cell, so one counting sort over the global cells is a segmented sort
 // that keeps each scene inside its slot range, and inside every cell the slots ascend by
-// reference index: the reference's table (crates/vxl-phys-fluid/src/grid.rs:29-76).
-// Walking a scene's 27 cells in the reference's (dz, dy, dx) order over those ranges
-// visits neighbours in the order of UniformGrid::for_neighbors_in (grid.rs:115-155),
-// so every per-particle sum matches the reference's CPU path bit for bit.
+// reference index: the reference's cells (crates/vxl-phys-fluid/src/grid.rs:29-76), but in
+// z-major order (cell_slot; the reference's table has x outermost, which the export
+// restores). Walking a scene's 27 cells in the reference's (dz, dy, dx) order visits
+// neighbours in the order of UniformGrid::for_neighbors_in (grid.rs:115-155), so every
+// per-particle sum matches the reference's CPU path bit for bit, and the three cells of a
+// (dz, dy) row are one run of slots.
 //
 // Work list. The particle kernels run persistent blocks over a list of tiles
 // (scene, first slot, count): a block takes the next tile from an atomic counter, so the
 // scene of a tile is uniform and scenes of very different sizes balance across SMs.
 //
 // Substep: gridbox (per scene) -> cell offsets -> keys -> scan -> place -> canon ->
-// density + EOS (+ neighbour lists) -> force + XSPH + integrate -> boundary reactions ->
+// filter words -> density + EOS (+ neighbour lists) -> force + XSPH + integrate -> boundary reactions ->
 // per-span reduction.
 #pragma once
 
 #include "sph_device.cuh"
 
 // Resident threads per SM the density and force passes are compiled for (register
-// budget = 65536 / this).
+// budget = 65536 / this). Density at 768 / 1024 / 1280: 0.352 / 0.291 / 0.288 ms on the 1M dam
+// break, 5.0 / 4.2 / 4.1 ms on the 10M one with queues of 12 windows (below), and 1280 has no
+// room for longer ones.
 #ifndef VXL_DENSITY_THREADS_PER_SM
-#define VXL_DENSITY_THREADS_PER_SM 2048
+#define VXL_DENSITY_THREADS_PER_SM 1024
 #endif
 #ifndef VXL_FORCE_THREADS_PER_SM
 #define VXL_FORCE_THREADS_PER_SM 1280
-#endif
-#ifndef VXL_DENSITY_SEG_THREADS_PER_SM
-#define VXL_DENSITY_SEG_THREADS_PER_SM 1024  // 64 registers, no spills: 11.4 vs 15.0 ms at 1536 on dam10m
 #endif
 
 
@@ -113,7 +114,6 @@ struct EngineCtl {
   uint32_t cells;  // sum of the scenes' cells this substep
   uint32_t err;
   uint32_t slow_gathers;
-  uint32_t doubled;  // some scene's bins are at least 2h this substep (half-cell masks needed)
   uint32_t epoch;    // substep counter: wet[c] == epoch marks cells holding fluid this substep
   uint32_t work[kWorkSlots];
 };
@@ -123,7 +123,7 @@ struct EngineCtl {
 // closer than 0.2 h", "the separation moved a particle".
 enum WorkId : int {
   kWorkDensity = 0, kWorkForce = 1, kWorkBforce = 2, kWorkScan = 3,
-  kWorkPushed = 4, kWorkTrigger = 5, kWorkMoved = 6, kWorkSegs = 7
+  kWorkPushed = 4, kWorkTrigger = 5, kWorkMoved = 6
 };
 
 // Provider walls (analytic ProviderColliders queried on the device). A plane of a FACES
@@ -165,6 +165,13 @@ constexpr int kScanThreads = 256;
 constexpr int kCanonSmem = 1024;
 constexpr int kCanonWindow = kCanonSmem / 2;  // window path: keys + segment table in one warp's buffer
 constexpr int kBGatherCap = 64;
+// Density walk: windows queued per thread. h-sized bins need 9 or 10 (a row each), 2h bins
+// about 20. 12 / 14 / 18 / 22 on the 10M dam break: 4.20 / 4.03 / 3.81 / 3.90 ms (shorter queues are
+// emptied more often, longer ones leave less L1); the 1M one 0.29 ms with each.
+#ifndef VXL_WALK_QUEUE
+#define VXL_WALK_QUEUE 18
+#endif
+constexpr uint32_t kWalkQueue = VXL_WALK_QUEUE;
 constexpr uint32_t kListPrefetch = 4;  // force pass: list entries fetched into L2 this far ahead
 
 // Block-level ordered-uint min/max of (x, y, z), one atomic per component into acc.
@@ -405,11 +412,7 @@ __global__ void k_e_slot_of(const uint32_t* __restrict__ orig, uint32_t* __restr
 __global__ void k_e_celloff(SceneDev* __restrict__ sc, uint32_t nscenes, EngineCtl* ctl, uint32_t cell_cap) {
   __shared__ uint32_t sh[1024];
   __shared__ unsigned long long carry;
-  __shared__ uint32_t doubled;
-  if (threadIdx.x == 0) {
-    carry = 0;
-    doubled = 0;
-  }
+  if (threadIdx.x == 0) carry = 0;
   if (threadIdx.x < kWorkSlots) ctl->work[threadIdx.x] = 0;  // persistent-pass counters of this substep
   if (threadIdx.x == 0) ctl->epoch = ctl->epoch + 1u;
   __syncthreads();
@@ -434,7 +437,6 @@ __global__ void k_e_celloff(SceneDev* __restrict__ sc, uint32_t nscenes, EngineC
         s.fbox[a] = 0xffffffffu;
         s.fbox[3 + a] = 0u;
       }
-      if (g.bin >= 2.0f * s.k.h) doubled = 1;
       v = g.total;
     }
     sh[threadIdx.x] = v;
@@ -452,7 +454,6 @@ __global__ void k_e_celloff(SceneDev* __restrict__ sc, uint32_t nscenes, EngineC
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    ctl->doubled = doubled;
     if (carry > (unsigned long long)cell_cap) {
       atomicOr(&ctl->err, kErrCellCap);
       ctl->cells = 0;
@@ -467,13 +468,9 @@ __global__ void k_e_celloff(SceneDev* __restrict__ sc, uint32_t nscenes, EngineC
 // makes the final order deterministic. Cells holding a fluid particle get wet[c] = epoch.
 __global__ void k_e_keys(const float4* __restrict__ pos, const SceneDev* __restrict__ sc,
                          const TileDev* __restrict__ tiles, uint32_t ntiles, const EngineCtl* __restrict__ ctl,
-                         uint32_t* __restrict__ counts, uint2* __restrict__ cellrank, uint32_t* __restrict__ halves,
-                         uint32_t half_words, uint32_t* __restrict__ wet) {
+                         uint32_t* __restrict__ counts, uint2* __restrict__ cellrank, uint32_t* __restrict__ wet) {
   if (ctl->err & kErrCellCap) return;
   const uint32_t epoch = ctl->epoch;
-  if (ctl->doubled)  // clear the half-cell masks that k_e_halfmask fills after the sort
-    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < half_words; w += gridDim.x * blockDim.x)
-      halves[w] = 0u;
   for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const TileDev td = tiles[t];
     const GridBox g = sc[td.scene].g;
@@ -484,7 +481,7 @@ __global__ void k_e_keys(const float4* __restrict__ pos, const SceneDev* __restr
       uint32_t c = 0xffffffffu;
       if (valid) {
         const float4 p = pos[td.first + i];
-        c = off + cell_index(g, p.x, p.y, p.z);
+        c = off + cell_slot(g, p.x, p.y, p.z);
         if (p.w > 0.0f) wet[c] = epoch;
       }
       const uint32_t active = __ballot_sync(0xffffffffu, valid);
@@ -742,97 +739,61 @@ __global__ void k_e_canon(const uint2* __restrict__ items, const uint32_t* __res
   }
 }
 
-// Walk the 27 cells around position p (cell (cx, cy, cz)) in the reference order
-// (dz outer, dy, dx inner; crates/vxl-phys-fluid/src/grid.rs:123-153), calling f(j) for
-// every slot j in them — except cells whose nominal box lies farther than h from p.
-// Such a cell holds no particle with r2 <= h2, so skipping it changes neither the set nor
-// the order of accepted neighbours. The test is conservative: per-axis gaps to the
-// neighbouring cell faces are clamped at 0 and compared with (h + bin/1024)^2, a margin
-// far above the f32 rounding of cell faces and bin assignment. `start` is the scene's
-// slice of the global cell table. With kSkipSelf, slot `self` is left out of the walk (it
-// can only lie in the centre cell, so only that cell's loop tests for it). kCompact walks
-// the same cells in the same order from a 27-bit mask built up front: fewer live registers
-// (measured: the force pass's fallback walk and the boundary gather run 9-10% faster with
-// it), but slower as the density pass's main loop (0.64 vs 0.47 ms on the 1M scene).
-template <bool kSkipSelf = false, bool kCompact = false, class F>
-__device__ __forceinline__ void walk27(const GridBox& g, const uint32_t* __restrict__ start, float px, float py,
-                                       float pz, uint32_t cx, uint32_t cy, uint32_t cz, float h, F&& f,
-                                       uint32_t self = ~0u) {
+// Squared gaps from a particle at p in cell c to the faces of that cell, per axis (0 where p
+// lies beyond the face), and the squared reach: a neighbouring cell whose gaps sum above it
+// holds no particle with r2 <= h2. The margin bin / 1024 on h is far above the f32 rounding of
+// cell faces and bin assignment.
+struct CellGaps {
+  float xl, xr, yl, yr, zl, zr, reach2;
+};
+
+__device__ __forceinline__ CellGaps cell_gaps(const GridBox& g, float px, float py, float pz, uint32_t cx, uint32_t cy,
+                                              uint32_t cz, float h) {
   const float lx = g.minx + (float)cx * g.bin, ly = g.miny + (float)cy * g.bin, lz = g.minz + (float)cz * g.bin;
-  const float gxl = fmaxf(px - lx, 0.0f), gxr = fmaxf(lx + g.bin - px, 0.0f);
-  const float gyl = fmaxf(py - ly, 0.0f), gyr = fmaxf(ly + g.bin - py, 0.0f);
-  const float gzl = fmaxf(pz - lz, 0.0f), gzr = fmaxf(lz + g.bin - pz, 0.0f);
+  const float xl = fmaxf(px - lx, 0.0f), xr = fmaxf(lx + g.bin - px, 0.0f);
+  const float yl = fmaxf(py - ly, 0.0f), yr = fmaxf(ly + g.bin - py, 0.0f);
+  const float zl = fmaxf(pz - lz, 0.0f), zr = fmaxf(lz + g.bin - pz, 0.0f);
   const float reach = h + g.bin * (1.0f / 1024.0f);
-  const float reach2 = reach * reach;
-  if constexpr (kCompact) {
-    uint32_t vm = 0;
-#pragma unroll
-    for (int dz = -1; dz <= 1; ++dz) {
-      const bool zok = dz < 0 ? cz > 0 : (dz > 0 ? cz + 1 < g.nz : true);
-      const float gz = dz < 0 ? gzl : (dz > 0 ? gzr : 0.0f);
-      const float dz2 = gz * gz;
-#pragma unroll
-      for (int dy = -1; dy <= 1; ++dy) {
-        const bool yok = dy < 0 ? cy > 0 : (dy > 0 ? cy + 1 < g.ny : true);
-        const float gy = dy < 0 ? gyl : (dy > 0 ? gyr : 0.0f);
-        const float dyz2 = dz2 + gy * gy;
-#pragma unroll
-        for (int dx = -1; dx <= 1; ++dx) {
-          const bool xok = dx < 0 ? cx > 0 : (dx > 0 ? cx + 1 < g.nx : true);
-          const float gx = dx < 0 ? gxl : (dx > 0 ? gxr : 0.0f);
-          if (zok && yok && xok && !(dyz2 + gx * gx > reach2)) vm |= 1u << ((dz + 1) * 9 + (dy + 1) * 3 + (dx + 1));
-        }
-      }
+  return CellGaps{xl * xl, xr * xr, yl * yl, yr * yr, zl * zl, zr * zr, reach * reach};
+}
+
+// Slots [j0, j1) of the row of cells at offset (dy, dz) from cell (cx, cy, cz): those of its up
+// to three cells in the grid that lie within reach. Empty when none does. `start` is the
+// scene's slice of the cell table.
+__device__ __forceinline__ bool cell_row(const GridBox& g, const uint32_t* __restrict__ start, const CellGaps& w,
+                                         uint32_t cx, uint32_t cy, uint32_t cz, int dy, int dz, uint32_t& j0,
+                                         uint32_t& j1) {
+  const int z = (int)cz + dz, y = (int)cy + dy;
+  const float gap = (dz < 0 ? w.zl : (dz > 0 ? w.zr : 0.0f)) + (dy < 0 ? w.yl : (dy > 0 ? w.yr : 0.0f));
+  if (z < 0 || z >= (int)g.nz || y < 0 || y >= (int)g.ny || gap > w.reach2) return false;
+  const uint32_t c = ((uint32_t)z * g.ny + (uint32_t)y) * g.nx + cx;
+  j0 = start[c - (cx > 0 && !(gap + w.xl > w.reach2) ? 1u : 0u)];
+  j1 = start[c + (cx + 1 < g.nx && !(gap + w.xr > w.reach2) ? 2u : 1u)];
+  return j0 < j1;
+}
+
+// Walk the 27 cells around position p (cell (cx, cy, cz)) in the reference order (dz outer,
+// dy, dx inner; crates/vxl-phys-fluid/src/grid.rs:123-153), calling f(j) for every slot j in
+// them, the particle's own among them, except cells farther than h from p (skipping them
+// changes neither the set nor the order of accepted neighbours).
+template <class F>
+__device__ __forceinline__ void walk27(const GridBox& g, const uint32_t* __restrict__ start, float px, float py,
+                                       float pz, uint32_t cx, uint32_t cy, uint32_t cz, float h, F&& f) {
+  const CellGaps w = cell_gaps(g, px, py, pz, cx, cy, cz, h);
+#pragma unroll 1
+  for (int dz = -1; dz <= 1; ++dz)
+#pragma unroll 1
+    for (int dy = -1; dy <= 1; ++dy) {
+      uint32_t j, j1;
+      if (cell_row(g, start, w, cx, cy, cz, dy, dz, j, j1))
+        for (; j < j1; ++j) f(j);
     }
-    const int nz = (int)g.nz, nyz = (int)(g.ny * g.nz);
-    const int centre = (int)(((cx * g.ny) + cy) * g.nz + cz);
-    while (vm) {
-      const int d = __ffs(vm) - 1;
-      vm &= vm - 1u;
-      const int dzp = d / 9, rem = d - 9 * dzp, dyp = rem / 3, dxp = rem - 3 * dyp;
-      const uint32_t idx = (uint32_t)(centre + (dxp - 1) * nyz + (dyp - 1) * nz + (dzp - 1));
-      const uint32_t j1 = start[idx + 1];
-      if (kSkipSelf && d == 13) {
-        for (uint32_t j = start[idx]; j < j1; ++j)
-          if (j != self) f(j);
-      } else {
-        for (uint32_t j = start[idx]; j < j1; ++j) f(j);
-      }
-    }
-  } else {
-    for (int dz = -1; dz <= 1; ++dz) {
-      const int z = (int)cz + dz;
-      if (z < 0 || z >= (int)g.nz) continue;
-      const float gz = dz < 0 ? gzl : (dz > 0 ? gzr : 0.0f);
-      const float dz2 = gz * gz;
-      for (int dy = -1; dy <= 1; ++dy) {
-        const int y = (int)cy + dy;
-        if (y < 0 || y >= (int)g.ny) continue;
-        const float gy = dy < 0 ? gyl : (dy > 0 ? gyr : 0.0f);
-        const float dyz2 = dz2 + gy * gy;
-        for (int dx = -1; dx <= 1; ++dx) {
-          const int x = (int)cx + dx;
-          if (x < 0 || x >= (int)g.nx) continue;
-          const float gx = dx < 0 ? gxl : (dx > 0 ? gxr : 0.0f);
-          if (dyz2 + gx * gx > reach2) continue;
-          const uint32_t idx = ((uint32_t)x * g.ny + (uint32_t)y) * g.nz + (uint32_t)z;
-          const uint32_t j1 = start[idx + 1];
-          if (kSkipSelf && dz == 0 && dy == 0 && dx == 0) {
-            for (uint32_t j = start[idx]; j < j1; ++j)
-              if (j != self) f(j);
-          } else {
-            for (uint32_t j = start[idx]; j < j1; ++j) f(j);
-          }
-        }
-      }
-    }
-  }
 }
 
 // Compact neighbour-list entries. Every neighbour of a particle in cell (cx, cy, cz) lies in
-// one of the three x-planes x = cx - 1, cx, cx + 1 of its 27 cells, and inside plane x its
-// slot is at least the first slot of cell (x, max(cy - 1, 0), max(cz - 1, 0)) — cell indices
-// grow with x, y, z and the table is sorted by cell — and below the next plane's first
+// one of the three z-planes z = cz - 1, cz, cz + 1 of its 27 cells, and inside plane z its
+// slot is at least the first slot of cell (max(cx - 1, 0), max(cy - 1, 0), z) — the table is
+// sorted by cell, z outermost, x innermost — and below the next plane's first
 // slot. A list entry is (plane << 14) | (slot - plane's first slot), 16 bits; a neighbour
 // 16,384 or more slots past its plane's first slot cannot be encoded, and its list is then
 // marked unusable (bit 31 of the count) so that the consumers walk the cells again.
@@ -841,25 +802,17 @@ constexpr uint32_t kListOffBits = 14;
 constexpr uint32_t kListOffMask = (1u << kListOffBits) - 1u;
 
 struct ListPlanes {
-  uint32_t b0, b1, b2;  // first slot of plane cx - 1 (= b1 at the grid's edge), cx, cx + 1 (~0u if none)
+  uint32_t b0, b1, b2;  // first slot of plane cz - 1 (= b1 at the grid's edge), cz, cz + 1 (~0u if none)
 };
 
 __device__ __forceinline__ ListPlanes list_planes(const GridBox& g, const uint32_t* __restrict__ cst, uint32_t cx,
                                                   uint32_t cy, uint32_t cz) {
-  const uint32_t ylo = cy > 0 ? cy - 1 : 0, zlo = cz > 0 ? cz - 1 : 0;
-  const uint32_t yz = ylo * g.nz + zlo, nyz = g.ny * g.nz;
+  const uint32_t xy = (cy > 0 ? cy - 1 : 0) * g.nx + (cx > 0 ? cx - 1 : 0), nxy = g.nx * g.ny;
   ListPlanes lp;
-  lp.b1 = cst[cx * nyz + yz];
-  lp.b0 = cx > 0 ? cst[(cx - 1) * nyz + yz] : lp.b1;
-  lp.b2 = cx + 1 < g.nx ? cst[(cx + 1) * nyz + yz] : 0xffffffffu;
+  lp.b1 = cst[cz * nxy + xy];
+  lp.b0 = cz > 0 ? cst[(cz - 1) * nxy + xy] : lp.b1;
+  lp.b2 = cz + 1 < g.nz ? cst[(cz + 1) * nxy + xy] : 0xffffffffu;
   return lp;
-}
-
-// Entry of neighbour slot j, or 0xffffffff if it cannot be encoded.
-__device__ __forceinline__ uint32_t list_encode(const ListPlanes& lp, uint32_t j) {
-  const uint32_t pl = (j >= lp.b1 ? 1u : 0u) + (j >= lp.b2 ? 1u : 0u);
-  const uint32_t off = j - (pl == 0u ? lp.b0 : (pl == 1u ? lp.b1 : lp.b2));
-  return off > kListOffMask ? 0xffffffffu : (pl << kListOffBits) | off;
 }
 
 __device__ __forceinline__ uint32_t list_decode(const ListPlanes& lp, uint32_t e) {
@@ -867,286 +820,80 @@ __device__ __forceinline__ uint32_t list_decode(const ListPlanes& lp, uint32_t e
   return (pl == 0u ? lp.b0 : (pl == 1u ? lp.b1 : lp.b2)) + (e & kListOffMask);
 }
 
-// Half-cell masks of the sorted slots, for the density walk: for each aligned block of 32
-// slots, halves[4 * (s >> 5) + a] has bit (s & 31) set iff slot s lies at or above the
-// midplane of its own cell along axis a (x, y, z). One thread per slot over tiles;
-// lanes that share a block and axis combine their bits before one atomicOr.
-__global__ void k_e_halfmask(const float4* __restrict__ pos, const SceneDev* __restrict__ sc,
-                             const TileDev* __restrict__ tiles, uint32_t ntiles, const EngineCtl* __restrict__ ctl,
-                             uint32_t* __restrict__ halves) {
-  if ((ctl->err & kErrCellCap) || !ctl->doubled) return;
-  const int lane = threadIdx.x & 31;
-  for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const TileDev td = tiles[t];
-    const GridBox g = sc[td.scene].g;
-    if (g.bin < 2.0f * sc[td.scene].k.h) continue;  // the density pass walks this scene unmasked
-    const float hb = g.bin * 0.5f;
-    for (uint32_t b0 = 0; b0 < td.count; b0 += blockDim.x) {
-      const uint32_t i = b0 + threadIdx.x;
-      const bool valid = i < td.count;
-      uint32_t blk = 0xffffffffu, bit = 0, hx = 0, hy = 0, hz = 0;
-      if (valid) {
-        const uint32_t s = td.first + i;
-        const float4 p = pos[s];
-        uint32_t cx, cy, cz;
-        bin_of(g, p.x, p.y, p.z, cx, cy, cz);
-        hx = p.x >= g.minx + (float)cx * g.bin + hb;
-        hy = p.y >= g.miny + (float)cy * g.bin + hb;
-        hz = p.z >= g.minz + (float)cz * g.bin + hb;
-        blk = s >> 5;
-        bit = 1u << (s & 31);
-      }
-      const uint32_t active = __ballot_sync(0xffffffffu, valid);
-      if (valid) {
-        const uint32_t peers = __match_any_sync(active, blk);
-        const uint32_t mx = __reduce_or_sync(peers, hx ? bit : 0u);
-        const uint32_t my = __reduce_or_sync(peers, hy ? bit : 0u);
-        const uint32_t mz = __reduce_or_sync(peers, hz ? bit : 0u);
-        if (lane == __ffs(peers) - 1) {
-          if (mx) atomicOr(&halves[4 * blk], mx);
-          if (my) atomicOr(&halves[4 * blk + 1], my);
-          if (mz) atomicOr(&halves[4 * blk + 2], mz);
+// walk27 through the candidate filter (sph_device.cuh): the same rows in the same order and in
+// each row the same slots in ascending order, except the slot `self` and those the filter
+// shows to lie farther than h. words holds the slots' filter words for the particle's residue
+// (padded by 32 past the last slot), tested eight per step; what is left comes out a window at a
+// time, push(m, base, plane): bit t of m (not 0) is slot base + t, plane its z-plane (dz + 1).
+// Called by whole warps (`active`: this lane walks); row() follows each row, converged.
+// A candidate costs a dp4a and a funnel shift (39 pairs per clock and SM) instead of a 16-byte
+// gather and eight float operations; what binds the walk is its work per row, which is why
+// the rows are runs of slots and the words are kept per residue. Density pass, before (cells
+// one by one, every candidate gathered and tested exactly) and after: 0.475 -> 0.295 ms on the
+// 1M dam break (h-sized bins), 0.84 -> 0.58 ms on a 1.4M pool and 5.5 -> 3.8 ms on the 10M one
+// (2h bins), 75 -> 36 us at 16k particles. With the words of one frame per cell, 27 cells and a
+// window each, 0.43 / 0.65 / 4.2 ms.
+template <class P, class R>
+__device__ __forceinline__ void walk27_q(const GridBox& g, const uint32_t* __restrict__ start,
+                                         const uint32_t* __restrict__ words, float px, float py, float pz, uint32_t cx,
+                                         uint32_t cy, uint32_t cz, float h, uint32_t self, bool active, P&& push,
+                                         R&& row) {
+  const CellGaps w = cell_gaps(g, px, py, pz, cx, cy, cz, h);
+  const int ax = axis_sub(g.minx, px, g.inv, cx) - 32, ay = axis_sub(g.miny, py, g.inv, cy) - 32,
+            az = axis_sub(g.minz, pz, g.inv, cz) - 32;
+  const uint32_t Mx = (uint32_t)(-ax & 255) | (kSubNorm << 24);
+  const int Tx = (int)g.reach_q - ax * ax;
+#pragma unroll 1
+  for (int dz = -1; dz <= 1; ++dz)
+#pragma unroll 1
+    for (int dy = -1; dy <= 1; ++dy) {
+      uint32_t j0, j1;
+      if (active && cell_row(g, start, w, cx, cy, cz, dy, dz, j0, j1)) {
+        const int my = (int)kSubUnits * dy - ay, mz = (int)kSubUnits * dz - az;
+        const int M = (int)(Mx | ((uint32_t)(my & 255) << 8) | ((uint32_t)(mz & 255) << 16));
+        const int over = -((Tx - (my * my + mz * mz)) >> 1) - 1;  // kept: word . M + over < 0
+        uint32_t low = ~0u << (j0 & 3u);
+        for (uint32_t base = j0 & ~3u; base < j1; base += 32) {
+          // eight words at a time from the last to the first, each sign bit shifted in from
+          // below: bit t of m is slot base + t
+          uint32_t m = 0;
+          const int4* w0 = reinterpret_cast<const int4*>(words + base);
+          const int4* wp = w0 + 2 * ((min(j1 - base, 32u) + 7u) / 8u);
+          do {
+            wp -= 2;
+            const int4 wb = wp[1], wa = wp[0];
+            m = __funnelshift_l((uint32_t)__dp4a(wb.w, M, over), m, 1);
+            m = __funnelshift_l((uint32_t)__dp4a(wb.z, M, over), m, 1);
+            m = __funnelshift_l((uint32_t)__dp4a(wb.y, M, over), m, 1);
+            m = __funnelshift_l((uint32_t)__dp4a(wb.x, M, over), m, 1);
+            m = __funnelshift_l((uint32_t)__dp4a(wa.w, M, over), m, 1);
+            m = __funnelshift_l((uint32_t)__dp4a(wa.z, M, over), m, 1);
+            m = __funnelshift_l((uint32_t)__dp4a(wa.y, M, over), m, 1);
+            m = __funnelshift_l((uint32_t)__dp4a(wa.x, M, over), m, 1);
+          } while (wp != w0);
+          m &= low;
+          low = ~0u;
+          if (j1 - base < 32u) m &= (1u << (j1 - base)) - 1u;
+          if (dz == 0 && dy == 0 && self - base < 32u) m &= ~(1u << (self - base));
+          if (m) push(m, base, (uint32_t)(dz + 1));
         }
       }
+      row();
     }
-  }
 }
 
-// Thread order of the half-culled density walk: within each cell, the slots in the lower x
-// half first, then those in the upper half (each group in slot order), from the half-cell
-// masks. At 2h bins a particle's reachable halves follow from the halves it lies in, so a
-// warp whose lanes share their x half skips the x-side cells its lanes cannot reach together
-// (every lane in the lower half leaves the +x cells out) instead of idling through them.
-// order[p] is the slot the density pass processes at position p; it permutes each cell's own
-// slots, so every slot is processed once and each result is unchanged. One warp per cell.
-__global__ void k_e_xorder(const uint32_t* __restrict__ start, const EngineCtl* __restrict__ ctl,
-                           const uint32_t* __restrict__ halves, uint32_t* __restrict__ order) {
-  if ((ctl->err & kErrCellCap) || !ctl->doubled) return;
-  const uint32_t total = ctl->cells;
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t lt = (1u << lane) - 1u;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < total; c += nw) {
-    const uint32_t b = start[c], n = start[c + 1] - b;
-    uint32_t nlow = 0;
-    for (uint32_t k0 = 0; k0 < n; k0 += 32) {
-      const uint32_t sl = b + k0 + lane;
-      const bool valid = k0 + lane < n;
-      const bool up = valid && ((halves[4 * (sl >> 5)] >> (sl & 31)) & 1u);
-      nlow += __popc(__ballot_sync(0xffffffffu, valid && !up));
-    }
-    uint32_t lo = 0, hi = 0;
-    for (uint32_t k0 = 0; k0 < n; k0 += 32) {
-      const uint32_t sl = b + k0 + lane;
-      const bool valid = k0 + lane < n;
-      const bool up = valid && ((halves[4 * (sl >> 5)] >> (sl & 31)) & 1u);
-      const uint32_t ml = __ballot_sync(0xffffffffu, valid && !up);
-      const uint32_t mh = __ballot_sync(0xffffffffu, up);
-      if (valid) order[b + (up ? nlow + hi + __popc(mh & lt) : lo + __popc(ml & lt))] = sl;
-      lo += __popc(ml);
-      hi += __popc(mh);
-    }
-  }
-}
-
-// Per axis, which halves of the three cells (d = -1, 0, +1) along it a particle at p can
-// reach: bit 2 (d + 1) for the lower half, bit 2 (d + 1) + 1 for the upper half. A half is
-// dropped only when the gap from p to its nominal interval exceeds `reach` (h plus a
-// margin far above the rounding of cell faces and midplanes). `last`: p's cell is the last
-// on this axis, whose upper half also holds the particles clamped into it from beyond the
-// grid (an axis at the 16,384-cell cap), p possibly among them: that half has no upper face.
-// (No particle lies below the grid's lower corner, the scene AABB's minimum.)
-__device__ __forceinline__ uint32_t half_reach_bits(float p, float l, float B, float reach, bool last) {
-  const float hb = B * 0.5f;
-  const float gm_lo = fmaxf(p - (l - hb), 0.0f);
-  const float gm_hi = fmaxf(p - l, 0.0f);
-  const float g0_lo = fmaxf(fmaxf(l - p, p - (l + hb)), 0.0f);
-  const float g0_hi = fmaxf(fmaxf((l + hb) - p, last ? 0.0f : p - (l + B)), 0.0f);
-  const float gp_lo = fmaxf((l + B) - p, 0.0f);
-  const float gp_hi = fmaxf((l + B + hb) - p, 0.0f);
-  return (gm_lo <= reach ? 1u : 0u) | (gm_hi <= reach ? 2u : 0u) | (g0_lo <= reach ? 4u : 0u) |
-         (g0_hi <= reach ? 8u : 0u) | (gp_lo <= reach ? 16u : 0u) | (gp_hi <= reach ? 32u : 0u);
-}
-
-// Slot mask of the particles in a block whose half along one axis is reachable.
-__device__ __forceinline__ uint32_t half_select(uint32_t two_bits, uint32_t upper) {
-  return two_bits == 3u ? 0xffffffffu : (two_bits == 2u ? upper : ~upper);
-}
-
-// walk27 with half-cell culling: the same cells in the same order, and inside each cell
-// the same slots in ascending order, except slots lying in a half-cell (along any axis)
-// farther than h from p — they cannot be accepted, so the accepted set and its order are
-// unchanged. Used when the grid's bins are at least 2h (the reference's cell budget
-// doubled them), where a particle reaches only about a quarter of the 27 cells' slots.
-template <class F>
-__device__ __forceinline__ void walk27_half(const GridBox& g, const uint32_t* __restrict__ start,
-                                            const uint32_t* __restrict__ halves, float px, float py, float pz,
-                                            uint32_t cx, uint32_t cy, uint32_t cz, float h, F&& f) {
-  const float B = g.bin;
-  const float lx = g.minx + (float)cx * B, ly = g.miny + (float)cy * B, lz = g.minz + (float)cz * B;
-  const float gxl = fmaxf(px - lx, 0.0f), gxr = fmaxf(lx + B - px, 0.0f);
-  const float gyl = fmaxf(py - ly, 0.0f), gyr = fmaxf(ly + B - py, 0.0f);
-  const float gzl = fmaxf(pz - lz, 0.0f), gzr = fmaxf(lz + B - pz, 0.0f);
-  const float reach = h + B * (1.0f / 1024.0f);
-  const float reach2 = reach * reach;
-  const uint32_t bxs = half_reach_bits(px, lx, B, reach, cx + 1 == g.nx);
-  const uint32_t bys = half_reach_bits(py, ly, B, reach, cy + 1 == g.ny);
-  const uint32_t bzs = half_reach_bits(pz, lz, B, reach, cz + 1 == g.nz);
-  for (int dz = -1; dz <= 1; ++dz) {
-    const int z = (int)cz + dz;
-    if (z < 0 || z >= (int)g.nz) continue;
-    const float gz = dz < 0 ? gzl : (dz > 0 ? gzr : 0.0f);
-    const float dz2 = gz * gz;
-    const uint32_t zsel = (bzs >> (2 * (dz + 1))) & 3u;
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int y = (int)cy + dy;
-      if (y < 0 || y >= (int)g.ny) continue;
-      const float gy = dy < 0 ? gyl : (dy > 0 ? gyr : 0.0f);
-      const float dyz2 = dz2 + gy * gy;
-      const uint32_t ysel = (bys >> (2 * (dy + 1))) & 3u;
-      for (int dx = -1; dx <= 1; ++dx) {
-        const int x = (int)cx + dx;
-        if (x < 0 || x >= (int)g.nx) continue;
-        const float gx = dx < 0 ? gxl : (dx > 0 ? gxr : 0.0f);
-        if (dyz2 + gx * gx > reach2) continue;
-        const uint32_t xsel = (bxs >> (2 * (dx + 1))) & 3u;
-        if (!xsel || !ysel || !zsel) continue;
-        const uint32_t idx = ((uint32_t)x * g.ny + (uint32_t)y) * g.nz + (uint32_t)z;
-        const uint32_t j0 = start[idx], j1 = start[idx + 1];
-        for (uint32_t base = j0 & ~31u; base < j1; base += 32) {
-          const uint4 hm = *reinterpret_cast<const uint4*>(halves + 4 * (base >> 5));
-          uint32_t m = half_select(xsel, hm.x) & half_select(ysel, hm.y) & half_select(zsel, hm.z);
-          if (j0 > base) m &= ~0u << (j0 - base);
-          if (j1 < base + 32) m &= (1u << (j1 - base)) - 1u;
-          while (m) {
-            const uint32_t j = base + (uint32_t)(__ffs(m) - 1);
-            m &= m - 1u;
-            f(j);
-          }
-        }
-      }
-    }
-  }
-}
-
-// walk27 / walk27_half with a hook per cell and the slot `skip` left out: f(j) for every
-// candidate in the same order; before a cell's candidates, fc(plane, end) with the cell's
-// x-plane (dx + 1) and its end slot.
-template <class FC, class F>
-__device__ __forceinline__ void walk27_c(const GridBox& g, const uint32_t* __restrict__ start, float px, float py,
-                                         float pz, uint32_t cx, uint32_t cy, uint32_t cz, float h, uint32_t skip,
-                                         FC&& fc, F&& f) {
-  const float lx = g.minx + (float)cx * g.bin, ly = g.miny + (float)cy * g.bin, lz = g.minz + (float)cz * g.bin;
-  const float gxl = fmaxf(px - lx, 0.0f), gxr = fmaxf(lx + g.bin - px, 0.0f);
-  const float gyl = fmaxf(py - ly, 0.0f), gyr = fmaxf(ly + g.bin - py, 0.0f);
-  const float gzl = fmaxf(pz - lz, 0.0f), gzr = fmaxf(lz + g.bin - pz, 0.0f);
-  const float reach = h + g.bin * (1.0f / 1024.0f);
-  const float reach2 = reach * reach;
-  for (int dz = -1; dz <= 1; ++dz) {
-    const int z = (int)cz + dz;
-    if (z < 0 || z >= (int)g.nz) continue;
-    const float gz = dz < 0 ? gzl : (dz > 0 ? gzr : 0.0f);
-    const float dz2 = gz * gz;
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int y = (int)cy + dy;
-      if (y < 0 || y >= (int)g.ny) continue;
-      const float gy = dy < 0 ? gyl : (dy > 0 ? gyr : 0.0f);
-      const float dyz2 = dz2 + gy * gy;
-      for (int dx = -1; dx <= 1; ++dx) {
-        const int x = (int)cx + dx;
-        if (x < 0 || x >= (int)g.nx) continue;
-        const float gx = dx < 0 ? gxl : (dx > 0 ? gxr : 0.0f);
-        if (dyz2 + gx * gx > reach2) continue;
-        const uint32_t idx = ((uint32_t)x * g.ny + (uint32_t)y) * g.nz + (uint32_t)z;
-        const uint32_t j1 = start[idx + 1];
-        fc((uint32_t)(dx + 1), j1);
-        for (uint32_t j = start[idx]; j < j1; ++j)
-          if (j != skip) f(j);
-      }
-    }
-  }
-}
-
-template <class FC, class F>
-__device__ __forceinline__ void walk27_half_c(const GridBox& g, const uint32_t* __restrict__ start,
-                                              const uint32_t* __restrict__ halves, float px, float py, float pz,
-                                              uint32_t cx, uint32_t cy, uint32_t cz, float h, uint32_t skip,
-                                              FC&& fc, F&& f) {
-  const float B = g.bin;
-  const float lx = g.minx + (float)cx * B, ly = g.miny + (float)cy * B, lz = g.minz + (float)cz * B;
-  const float gxl = fmaxf(px - lx, 0.0f), gxr = fmaxf(lx + B - px, 0.0f);
-  const float gyl = fmaxf(py - ly, 0.0f), gyr = fmaxf(ly + B - py, 0.0f);
-  const float gzl = fmaxf(pz - lz, 0.0f), gzr = fmaxf(lz + B - pz, 0.0f);
-  const float reach = h + B * (1.0f / 1024.0f);
-  const float reach2 = reach * reach;
-  const uint32_t bxs = half_reach_bits(px, lx, B, reach, cx + 1 == g.nx);
-  const uint32_t bys = half_reach_bits(py, ly, B, reach, cy + 1 == g.ny);
-  const uint32_t bzs = half_reach_bits(pz, lz, B, reach, cz + 1 == g.nz);
-  for (int dz = -1; dz <= 1; ++dz) {
-    const int z = (int)cz + dz;
-    if (z < 0 || z >= (int)g.nz) continue;
-    const float gz = dz < 0 ? gzl : (dz > 0 ? gzr : 0.0f);
-    const float dz2 = gz * gz;
-    const uint32_t zsel = (bzs >> (2 * (dz + 1))) & 3u;
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int y = (int)cy + dy;
-      if (y < 0 || y >= (int)g.ny) continue;
-      const float gy = dy < 0 ? gyl : (dy > 0 ? gyr : 0.0f);
-      const float dyz2 = dz2 + gy * gy;
-      const uint32_t ysel = (bys >> (2 * (dy + 1))) & 3u;
-      for (int dx = -1; dx <= 1; ++dx) {
-        const int x = (int)cx + dx;
-        if (x < 0 || x >= (int)g.nx) continue;
-        const float gx = dx < 0 ? gxl : (dx > 0 ? gxr : 0.0f);
-        if (dyz2 + gx * gx > reach2) continue;
-        const uint32_t xsel = (bxs >> (2 * (dx + 1))) & 3u;
-        if (!xsel || !ysel || !zsel) continue;
-        const uint32_t idx = ((uint32_t)x * g.ny + (uint32_t)y) * g.nz + (uint32_t)z;
-        const uint32_t j0 = start[idx], j1 = start[idx + 1];
-        fc((uint32_t)(dx + 1), j1);
-        // windows of 32 slots from the cell's own first slot, the half masks read across two
-        // aligned words: lanes of one octant in different cells of similar contents then
-        // take the same number of trips through each window
-        for (uint32_t base = j0; base < j1; base += 32) {
-          const uint32_t sh = base & 31u;
-          const uint4 lo = *reinterpret_cast<const uint4*>(halves + 4 * (base >> 5));
-          const uint4 hi = *reinterpret_cast<const uint4*>(halves + 4 * (base >> 5) + 4);
-          const uint32_t ux = __funnelshift_r(lo.x, hi.x, sh), uy = __funnelshift_r(lo.y, hi.y, sh),
-                         uz = __funnelshift_r(lo.z, hi.z, sh);
-          uint32_t m = half_select(xsel, ux) & half_select(ysel, uy) & half_select(zsel, uz);
-          if (j1 < base + 32) m &= (1u << (j1 - base)) - 1u;
-          if (skip - base < 32u) m &= ~(1u << (skip - base));  // once per window, not per candidate
-          while (m) {
-            f(base + (uint32_t)(__ffs(m) - 1));
-            m &= m - 1u;
-          }
-        }
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------- grouped density walk
+// ---------------------------------------------------------------- filter words and walk order
 //
-// Particles of one cell reach the same neighbour cells; when the cell budget has doubled
-// the bins to 2h or more, particles of one octant of a cell (the same half along x, y and
-// z) also reach the same half-cells. The grouped density pass lets eight lanes of a warp
-// share one stream of candidates: k_e_groups orders each chunk of a tile (up to
-// kGroupChunk slots) by octant (a stable counting sort, so the slots of an octant stay
-// ascending) into order[], then cuts the runs of equal (cell, octant) into segments of at
-// most kSegLanes positions, appended to segs[] as (first position in order[], count |
-// scene << 4); ctl->work[kWorkSegs] counts them. The order of segments in segs[] is
-// immaterial: each particle's sums are formed by one lane alone.
-//
-// The per-particle walk runs in order[] too: a warp whose lanes share one octant walks one
-// culled cell set. Octants follow one another in Gray-code order (0 1 3 2 6 7 5 4), so a
-// warp that straddles two octants walks the union of two sets that differ along one axis
-// only (12 cells instead of 8; up to 27 for octants apart in all three). A chunk holds 8
-// octant runs, 7 boundaries over kGroupChunk / 32 warps; chunks of 512 slots (tiles of 512)
-// let fewer warps straddle, but cost the grouping pass about as much as they save.
-
-constexpr uint32_t kSegLanes = 8;   // lanes (particles) per segment; four segments per warp
-constexpr uint32_t kSegQueue = 64;  // candidate ring per segment (pending never exceeds 7 + 32)
+// k_e_groups writes every slot's candidate-filter words from its sorted position, and for
+// scenes whose cell budget doubled the bins to 2h or more the order in which the density
+// pass takes the slots: each chunk of a tile (up to kGroupChunk slots) by octant of the
+// cell (the half along x, y and z; a stable counting sort into order[]). At 2h bins a
+// particle reaches the cells on its own octant's side only, so a warp whose lanes share one
+// octant walks one set of cells. Octants follow one another in Gray-code order (0 1 3 2 6
+// 7 5 4), so a warp that straddles two octants walks the union of two sets that differ along
+// one axis only (12 cells instead of 8; up to 27 for octants apart in all three). A chunk
+// holds 8 octant runs, 7 boundaries over kGroupChunk / 32 warps; chunks of 512 slots (tiles
+// of 512) let fewer warps straddle, but cost the grouping pass about as much as they save.
 #ifndef VXL_GROUP_CHUNK
 #define VXL_GROUP_CHUNK 256
 #endif
@@ -1156,15 +903,13 @@ static_assert(kGroupChunk % 128 == 0 && kGroupChunk <= 1024, "chunk: 128..1024 s
 __device__ __forceinline__ uint32_t octant_rank(uint32_t oct) { return oct ^ (oct >> 1) ^ (oct >> 2); }
 
 __global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restrict__ pos, const SceneDev* __restrict__ sc,
-                                                          const TileDev* __restrict__ tiles, uint32_t ntiles, EngineCtl* ctl,
-                                                          uint32_t* __restrict__ order, uint2* __restrict__ segs,
-                                                          uint32_t* __restrict__ halves) {
+                                                          const TileDev* __restrict__ tiles, uint32_t ntiles,
+                                                          const EngineCtl* __restrict__ ctl, uint32_t* __restrict__ order,
+                                                          uint32_t* __restrict__ words, uint32_t wstride) {
   if (ctl->err & kErrCellCap) return;
   constexpr uint32_t kW = kGroupChunk / 32;  // warps
   constexpr uint32_t kV = 8 * kW / 32;       // (rank, warp) counts per lane of the scan
   __shared__ uint32_t s_cnt[8 * kW];         // [octant rank][warp]: slots per octant in each warp
-  __shared__ uint32_t s_cell[kGroupChunk], s_oct[kGroupChunk];
-  __shared__ uint32_t s_last[kW], s_nseg[kW], s_segbase;
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u;
   // the block's chunks one after another, each one's positions loaded while the previous
@@ -1185,328 +930,59 @@ __global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restri
     }
     if (t < ntiles && c1 + threadIdx.x < tn.count) pn = pos[tn.first + c1 + threadIdx.x];
     const GridBox g = sc[td.scene].g;
-    const bool half = g.bin >= 2.0f * sc[td.scene].k.h;
+    const bool half = g.bin >= 2.0f * sc[td.scene].k.h;  // uniform over the block
     const float hb = g.bin * 0.5f;
-    {
-      const uint32_t n = min(kGroupChunk, td.count - c0);
-      const uint32_t i = threadIdx.x;
-      const bool valid = i < n;
-      uint32_t cell = 0, oct = 0;
-      if (valid) {
-        uint32_t cx, cy, cz;
-        bin_of(g, p.x, p.y, p.z, cx, cy, cz);
-        cell = (cx * g.ny + cy) * g.nz + cz;
-        if (half)
-          oct = (p.x >= g.minx + (float)cx * g.bin + hb ? 1u : 0u) | (p.y >= g.miny + (float)cy * g.bin + hb ? 2u : 0u) |
-                (p.z >= g.minz + (float)cz * g.bin + hb ? 4u : 0u);
-      }
-      // the half-cell masks of the density walk (what k_e_halfmask writes for the scenes
-      // with provider walls): bit (s & 31) of halves[4 (s >> 5) + a] for the upper half
-      if (half) {
-        const uint32_t active = __ballot_sync(0xffffffffu, valid);
-        if (valid) {
-          const uint32_t s = td.first + c0 + i;
-          const uint32_t blk = s >> 5, bit = 1u << (s & 31);
-          const uint32_t peers = __match_any_sync(active, blk);
-          const uint32_t mx = __reduce_or_sync(peers, (oct & 1u) ? bit : 0u);
-          const uint32_t my = __reduce_or_sync(peers, (oct & 2u) ? bit : 0u);
-          const uint32_t mz = __reduce_or_sync(peers, (oct & 4u) ? bit : 0u);
-          if (lane == __ffs(peers) - 1) {
-            if (mx) atomicOr(&halves[4 * blk], mx);
-            if (my) atomicOr(&halves[4 * blk + 1], my);
-            if (mz) atomicOr(&halves[4 * blk + 2], mz);
-          }
-        }
-      }
-      const uint32_t key = octant_rank(oct);
-      uint32_t rank = 0;
+    const uint32_t i = threadIdx.x;
+    const bool valid = i < min(kGroupChunk, td.count - c0);
+    uint32_t oct = 0;
+    if (valid) {
+      uint32_t cx, cy, cz;
+      bin_of(g, p.x, p.y, p.z, cx, cy, cz);
+      const int bx = axis_sub(g.minx, p.x, g.inv, cx), by = axis_sub(g.miny, p.y, g.inv, cy) - 32,
+                bz = axis_sub(g.minz, p.z, g.inv, cz) - 32;
+      uint32_t side = (cx + 1) % 3;  // (cx - p + 1) mod 3, p = 0, 1, 2
 #pragma unroll
-      for (uint32_t o = 0; o < 8; ++o) {
-        const uint32_t b = __ballot_sync(0xffffffffu, valid && key == o);
-        if (lane == 0) s_cnt[o * kW + w] = __popc(b);
-        if (valid && key == o) rank = __popc(b & lt);
+      for (uint32_t q = 0; q < 3; ++q) {
+        words[(size_t)q * wstride + td.first + c0 + i] = sub_word((int)(kSubUnits * side) + bx - 96, by, bz);
+        side = side ? side - 1 : 2;
       }
-      __syncthreads();
-      if (w == 0) {  // exclusive scan of the 8 * kW counts in (rank, warp) order
-        uint32_t v[kV], tot = 0;
-#pragma unroll
-        for (uint32_t k = 0; k < kV; ++k) {
-          v[k] = s_cnt[lane * kV + k];
-          tot += v[k];
-        }
-        uint32_t incl = tot;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-          const uint32_t u = __shfl_up_sync(0xffffffffu, incl, off);
-          if ((int)lane >= off) incl += u;
-        }
-        uint32_t ex = incl - tot;
-#pragma unroll
-        for (uint32_t k = 0; k < kV; ++k) {
-          s_cnt[lane * kV + k] = ex;
-          ex += v[k];
-        }
-      }
-      __syncthreads();
-      if (valid) {
-        const uint32_t q = s_cnt[key * kW + w] + rank;
-        order[td.first + c0 + q] = td.first + c0 + i;
-        s_cell[q] = cell;
-        s_oct[q] = oct;
-      }
-      __syncthreads();
-      // runs of equal (cell, octant) in the new order, cut into segments of kSegLanes
-      const bool head = valid && (i == 0 || s_cell[i] != s_cell[i - 1] || s_oct[i] != s_oct[i - 1]);
-      const uint32_t hbal = __ballot_sync(0xffffffffu, head);
-      if (lane == 0) s_last[w] = hbal ? w * 32 + 31 - __clz(hbal) : 0xffffffffu;
-      __syncthreads();
-      uint32_t run0 = 0;
-      const uint32_t le = hbal & (0xffffffffu >> (31 - lane));
-      if (le) {
-        run0 = w * 32 + 31 - __clz(le);
-      } else {
-        for (int k = (int)w - 1; k >= 0; --k)
-          if (s_last[k] != 0xffffffffu) {
-            run0 = s_last[k];
-            break;
-          }
-      }
-      const bool shead = valid && ((i - run0) % kSegLanes == 0u);
-      uint32_t cnt = 0;
-      if (shead) {
-        cnt = 1;
-        while (cnt < kSegLanes && i + cnt < n && s_cell[i + cnt] == s_cell[i] && s_oct[i + cnt] == s_oct[i]) ++cnt;
-      }
-      const uint32_t sb = __ballot_sync(0xffffffffu, shead);
-      if (lane == 0) s_nseg[w] = __popc(sb);
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        uint32_t tot = 0;
-        for (uint32_t k = 0; k < kW; ++k) {
-          const uint32_t v = s_nseg[k];
-          s_nseg[k] = tot;
-          tot += v;
-        }
-        s_segbase = atomicAdd(&ctl->work[kWorkSegs], tot);
-      }
-      __syncthreads();
-      if (shead) segs[s_segbase + s_nseg[w] + __popc(sb & lt)] = make_uint2(td.first + c0 + i, cnt | (td.scene << 4));
-      __syncthreads();
+      if (half)
+        oct = (p.x >= g.minx + (float)cx * g.bin + hb ? 1u : 0u) | (p.y >= g.miny + (float)cy * g.bin + hb ? 2u : 0u) |
+              (p.z >= g.minz + (float)cz * g.bin + hb ? 4u : 0u);
     }
-  }
-}
-
-// Density (poly6 with self term) + Tait EOS over the segments of k_e_groups: the same
-// sums as k_e_density (crates/vxl-phys-fluid/src/fluid_density.rs:17-70) for scenes
-// without provider walls. Lanes 8k..8k+7 of a warp hold the particles of one segment,
-// which share their cell. The segment's cells are the union of its lanes' culled 27-cell
-// sets (and, at 2h bins, of their reachable half-cells) — for each lane a superset of its
-// own walk that adds only particles farther than h — taken in the reference's (dz, dy, dx)
-// order and, inside a cell, in ascending slot order (crates/vxl-phys-fluid/src/grid.rs:
-// 115-155). The segment's eight lanes append the candidate slots to a ring in shared
-// memory (each lane four bits of a 32-slot window), load eight of them at a time into a
-// staging row, and every lane then tests its own particle against the row in order, so
-// each lane accepts exactly its walk's neighbours in its walk's order: the sums, the EOS
-// and the recorded neighbour list are those of k_e_density, bit for bit. Segments of one
-// warp advance in lock step, eight candidates per round.
-template <int kWarps>
-__global__ void __launch_bounds__(kWarps * 32, VXL_DENSITY_SEG_THREADS_PER_SM / (kWarps * 32)) k_e_density_seg(
-    const float4* __restrict__ pos, const uint32_t* __restrict__ start, const SceneDev* __restrict__ sc,
-    const EngineCtl* __restrict__ ctl, const uint32_t* __restrict__ halves, const uint32_t* __restrict__ order,
-    const uint2* __restrict__ segs, float2* __restrict__ rc, float* __restrict__ press_out, uint16_t* __restrict__ nbr,
-    uint32_t* __restrict__ nbr_n, uint32_t cap, uint32_t stride, const uint32_t* __restrict__ wet) {
-  if (ctl->err & kErrCellCap) return;
-  __shared__ uint32_t s_queue[kWarps][4][kSegQueue];
-  __shared__ float4 s_pos[kWarps][4 * (kSegLanes + 1)];  // rows padded by one: segments hit different banks
-  __shared__ uint32_t s_j[kWarps][4 * (kSegLanes + 1)];
-  const uint32_t nseg = ctl->work[kWorkSegs];
-  const uint32_t epoch = ctl->epoch;
-  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint32_t seg = lane >> 3, sl = lane & 7u;
-  uint32_t* queue = s_queue[w][seg];
-  float4* stp = &s_pos[w][seg * (kSegLanes + 1)];
-  uint32_t* stj = &s_j[w][seg * (kSegLanes + 1)];
-  const uint32_t nwarps = gridDim.x * kWarps;
-  for (uint32_t g0 = (blockIdx.x * kWarps + w) * 4; g0 < nseg; g0 += nwarps * 4) {
-    const uint32_t sid = g0 + seg;
-    const uint2 rec = sid < nseg ? segs[sid] : make_uint2(0u, 0u);
-    const uint32_t nseg_lanes = rec.y & 15u;
-    const bool act = sl < nseg_lanes;
-    const SceneDev& S = sc[rec.y >> 4];
-    const GridBox g = S.g;
-    const float h = S.k.h, h2 = S.k.h2, k6 = S.k.k6;
-    const bool half = halves != nullptr && g.bin >= 2.0f * h;
-    uint32_t s = 0;
-    float4 pi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    uint32_t cx = 0, cy = 0, cz = 0;
-    if (act) {
-      s = order[rec.x + sl];
-      pi = pos[s];
-      bin_of(g, pi.x, pi.y, pi.z, cx, cy, cz);
+    if (!half) continue;
+    const uint32_t key = octant_rank(oct);
+    uint32_t rank = 0;
+#pragma unroll
+    for (uint32_t o = 0; o < 8; ++o) {
+      const uint32_t b = __ballot_sync(0xffffffffu, valid && key == o);
+      if (lane == 0) s_cnt[o * kW + w] = __popc(b);
+      if (valid && key == o) rank = __popc(b & lt);
     }
-    const bool fluid_i = pi.w > 0.0f;
-    // this lane's cells: in the grid and not farther than h (conservatively, as walk27),
-    // and at 2h bins with some reachable half along every axis (as walk27_half)
-    uint32_t cm = 0, bxs = 0, bys = 0, bzs = 0;
-    if (act) {
-      const float lx = g.minx + (float)cx * g.bin, ly = g.miny + (float)cy * g.bin, lz = g.minz + (float)cz * g.bin;
-      const float gxl = fmaxf(pi.x - lx, 0.0f), gxr = fmaxf(lx + g.bin - pi.x, 0.0f);
-      const float gyl = fmaxf(pi.y - ly, 0.0f), gyr = fmaxf(ly + g.bin - pi.y, 0.0f);
-      const float gzl = fmaxf(pi.z - lz, 0.0f), gzr = fmaxf(lz + g.bin - pi.z, 0.0f);
-      const float reach = h + g.bin * (1.0f / 1024.0f);
-      const float reach2 = reach * reach;
-      if (half) {
-        bxs = half_reach_bits(pi.x, lx, g.bin, reach, cx + 1 == g.nx);
-        bys = half_reach_bits(pi.y, ly, g.bin, reach, cy + 1 == g.ny);
-        bzs = half_reach_bits(pi.z, lz, g.bin, reach, cz + 1 == g.nz);
-      } else {
-        bxs = bys = bzs = 63u;
+    __syncthreads();
+    if (w == 0) {  // exclusive scan of the 8 * kW counts in (rank, warp) order
+      uint32_t v[kV], tot = 0;
+#pragma unroll
+      for (uint32_t k = 0; k < kV; ++k) {
+        v[k] = s_cnt[lane * kV + k];
+        tot += v[k];
       }
+      uint32_t incl = tot;
 #pragma unroll
-      for (int dz = -1; dz <= 1; ++dz) {
-        const bool zok = (dz < 0 ? cz > 0 : (dz > 0 ? cz + 1 < g.nz : true)) && ((bzs >> (2 * (dz + 1))) & 3u);
-        const float gz = dz < 0 ? gzl : (dz > 0 ? gzr : 0.0f);
-        const float dz2 = gz * gz;
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, off);
+        if ((int)lane >= off) incl += u;
+      }
+      uint32_t ex = incl - tot;
 #pragma unroll
-        for (int dy = -1; dy <= 1; ++dy) {
-          const bool yok = (dy < 0 ? cy > 0 : (dy > 0 ? cy + 1 < g.ny : true)) && ((bys >> (2 * (dy + 1))) & 3u);
-          const float gy = dy < 0 ? gyl : (dy > 0 ? gyr : 0.0f);
-          const float dyz2 = dz2 + gy * gy;
-#pragma unroll
-          for (int dx = -1; dx <= 1; ++dx) {
-            const bool xok = (dx < 0 ? cx > 0 : (dx > 0 ? cx + 1 < g.nx : true)) && ((bxs >> (2 * (dx + 1))) & 3u);
-            const float gx = dx < 0 ? gxl : (dx > 0 ? gxr : 0.0f);
-            if (zok && yok && xok && !(dyz2 + gx * gx > reach2)) cm |= 1u << ((dz + 1) * 9 + (dy + 1) * 3 + (dx + 1));
-          }
-        }
+      for (uint32_t k = 0; k < kV; ++k) {
+        s_cnt[lane * kV + k] = ex;
+        ex += v[k];
       }
     }
-    // A segment of boundary particles only sums fluid neighbours: with no fluid in its
-    // cell's 27 cells (none marked wet this substep) it has nothing to walk. The segment's
-    // lanes share the cell, so they test the 27 cells together.
-    const uint32_t seg_mask = 0xffu << (8 * seg);
-    const bool seg_fluid = (__ballot_sync(0xffffffffu, act && fluid_i) & seg_mask) != 0u;
-    const uint32_t lead = seg * 8;
-    const uint32_t ccx = __shfl_sync(0xffffffffu, cx, lead), ccy = __shfl_sync(0xffffffffu, cy, lead),
-                   ccz = __shfl_sync(0xffffffffu, cz, lead);
-    bool wet_seen = seg_fluid;
-    if (!seg_fluid && nseg_lanes) {
-      const uint32_t* wc = wet + S.cell_off;
-      for (uint32_t d = sl; d < 27u; d += 8u) {
-        const int dz = (int)(d / 9) - 1, dy = (int)((d / 3) % 3) - 1, dx = (int)(d % 3) - 1;
-        const int x = (int)ccx + dx, y = (int)ccy + dy, z = (int)ccz + dz;
-        if (x >= 0 && x < (int)g.nx && y >= 0 && y < (int)g.ny && z >= 0 && z < (int)g.nz &&
-            wc[((uint32_t)x * g.ny + (uint32_t)y) * g.nz + (uint32_t)z] == epoch)
-          wet_seen = true;
-      }
-    }
-    const bool seg_wet = (__ballot_sync(0xffffffffu, wet_seen) & seg_mask) != 0u;
-    if (!seg_wet) cm = 0;
-#pragma unroll
-    for (uint32_t o = 1; o < 8; o <<= 1) {
-      cm |= __shfl_xor_sync(0xffffffffu, cm, o);
-      bxs |= __shfl_xor_sync(0xffffffffu, bxs, o);
-      bys |= __shfl_xor_sync(0xffffffffu, bys, o);
-      bzs |= __shfl_xor_sync(0xffffffffu, bzs, o);
-    }
-    const uint32_t nz = g.nz, nyz = g.ny * g.nz;
-    const uint32_t centre = (ccx * g.ny + ccy) * g.nz + ccz;
-    const uint32_t* cst = start + S.cell_off;
-    float sum = fluid_i ? S.k.w0 : 0.0f;
-    float sum_b = 0.0f;
-    uint32_t cnt = 0, bad = 0;
-    uint16_t* wp = nbr + s;  // next list entry: nbr[cnt * stride + s]
-    const ListPlanes lp = list_planes(g, cst, ccx, ccy, ccz);
-    // segment walk state (equal on the segment's lanes)
-    uint32_t ucm = cm, blk = 0, jb = 0, je = 0, xs = 3, ys = 3, zs = 3, qh = 0, qt = 0;
-    for (;;) {
-      while (qt - qh < kSegLanes) {
-        if (blk >= je) {
-          if (!ucm) break;
-          const uint32_t d = __ffs(ucm) - 1;
-          ucm &= ucm - 1u;
-          const uint32_t dzp = d / 9, dyp = (d / 3) % 3, dxp = d % 3;
-          const uint32_t idx = centre + dxp * nyz + dyp * nz + dzp - (nyz + nz + 1u);
-          jb = cst[idx];
-          je = cst[idx + 1];
-          blk = half ? (jb & ~31u) : jb;
-          xs = (bxs >> (2 * dxp)) & 3u;
-          ys = (bys >> (2 * dyp)) & 3u;
-          zs = (bzs >> (2 * dzp)) & 3u;
-          continue;
-        }
-        uint32_t m;
-        if (half) {
-          const uint4 hm = *reinterpret_cast<const uint4*>(halves + 4 * (blk >> 5));
-          m = half_select(xs, hm.x) & half_select(ys, hm.y) & half_select(zs, hm.z);
-          if (jb > blk) m &= ~0u << (jb - blk);
-          if (je < blk + 32u) m &= (1u << (je - blk)) - 1u;
-        } else {
-          const uint32_t left = je - blk;
-          m = left >= 32u ? ~0u : (1u << left) - 1u;
-        }
-        const uint32_t nib = (m >> (4 * sl)) & 15u;
-        uint32_t at = qt + __popc(m & ((1u << (4 * sl)) - 1u));
-        const uint32_t j4 = blk + 4 * sl;
-        if (nib & 1u) queue[(at++) & (kSegQueue - 1)] = j4;
-        if (nib & 2u) queue[(at++) & (kSegQueue - 1)] = j4 + 1;
-        if (nib & 4u) queue[(at++) & (kSegQueue - 1)] = j4 + 2;
-        if (nib & 8u) queue[at & (kSegQueue - 1)] = j4 + 3;
-        qt += __popc(m);
-        blk += 32u;
-      }
-      const uint32_t nc = min(qt - qh, kSegLanes);
-      if (!__any_sync(0xffffffffu, nc != 0u)) break;
-      __syncwarp();
-      if (sl < nc) {
-        const uint32_t j = queue[(qh + sl) & (kSegQueue - 1)];
-        stj[sl] = j;
-        stp[sl] = pos[j];
-      }
-      __syncwarp();
-#pragma unroll
-      for (uint32_t c = 0; c < kSegLanes; ++c) {
-        if (c < nc) {
-          const uint32_t j = stj[c];
-          const float4 pj = stp[c];
-          if (act && j != s) {
-            const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-            const float r2 = dx * dx + dy * dy + dz * dz;
-            if (r2 <= h2) {
-              const float tt = h2 - r2;
-              const float wv = k6 * tt * tt * tt;
-              bool keep = true;
-              if (fluid_i) {
-                if (pj.w > 0.0f) sum += wv;
-                else sum_b += (-pj.w) * wv;
-              } else if (pj.w > 0.0f) {
-                sum += pj.w * wv;
-              } else {
-                keep = false;
-              }
-              if (keep) {
-                if (cnt < cap) {
-                  const uint32_t e = list_encode(lp, j);
-                  bad |= e >> 31;
-                  __stcs(wp, (unsigned short)e);  // streaming store: the list is read once, by the force pass
-                  wp += stride;
-                }
-                ++cnt;
-              }
-            }
-          }
-        }
-      }
-      qh += nc;
-      __syncwarp();
-    }
-    if (act) {
-      nbr_n[s] = cnt | (bad ? kListBad : 0u);
-      const float rho = fluid_i ? (S.k.mass * sum + sum_b) : ((-pi.w) * S.k.w0 + sum);
-      const float p = tait(S.k, rho);
-      rc[s] = make_float2(rho, p / (rho * rho));
-      if (press_out) press_out[s] = p;
-    }
+    __syncthreads();
+    if (valid) order[td.first + c0 + s_cnt[key * kW + w] + rank] = td.first + c0 + i;
+    __syncthreads();
   }
 }
 
@@ -1590,13 +1066,18 @@ __device__ __forceinline__ void provider_contacts(const ProviderDev& pr, const W
 template <int kBlock, bool kWalls = false>
 __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k_e_density(
     const float4* __restrict__ pos, const uint32_t* __restrict__ start, const SceneDev* __restrict__ sc,
-    const TileDev* __restrict__ tiles, uint32_t ntiles, EngineCtl* ctl, const uint32_t* __restrict__ halves,
-    float2* __restrict__ rc, float* __restrict__ press_out, uint16_t* __restrict__ nbr,
+    const TileDev* __restrict__ tiles, uint32_t ntiles, EngineCtl* ctl, const uint32_t* __restrict__ words,
+    uint32_t wstride, float2* __restrict__ rc, float* __restrict__ press_out, uint16_t* __restrict__ nbr,
     uint32_t* __restrict__ nbr_n, uint32_t cap, uint32_t stride, const uint32_t* __restrict__ wet,
-    const uint32_t* __restrict__ xorder, const ProviderDev* __restrict__ prov = nullptr,
+    const uint32_t* __restrict__ order, const ProviderDev* __restrict__ prov = nullptr,
     const WallPlaneDev* __restrict__ wplanes = nullptr, const uint32_t* __restrict__ orig = nullptr,
     ContactTableDev ctm = ContactTableDev{nullptr, nullptr, nullptr}) {
   if (ctl->err & kErrCellCap) return;
+  // Windows of kept candidates (mask, first slot | plane << 30), a column per thread: the walk
+  // queues them and the warp takes the exact tests from the queue together, so that its lanes,
+  // whose windows hold different counts, run one loop of about equal length instead of
+  // waiting for one another in every window.
+  __shared__ uint2 s_win[kWalkQueue][kBlock];
   for (uint32_t t = first_tile(&ctl->work[kWorkDensity], ntiles); t < ntiles; t = following_tile(&ctl->work[kWorkDensity], ntiles)) {
     const TileDev td = tiles[t];
     const SceneDev& S = sc[td.scene];
@@ -1604,10 +1085,12 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
     const SphConst& k = S.k;
     const uint32_t* cst = start + S.cell_off;
     const float h = k.h, h2 = k.h2, k6 = k.k6, w0 = k.w0, mass = k.mass;
-    const bool half_walk = halves != nullptr && g.bin >= 2.0f * h;  // uniform over the tile
+    const bool ordered = g.bin >= 2.0f * h;  // uniform over the tile: octant order (k_e_groups)
     const uint32_t epoch = ctl->epoch;
-    for (uint32_t i = threadIdx.x; i < td.count; i += kBlock) {
-      const uint32_t s = half_walk ? xorder[td.first + i] : td.first + i;
+    for (uint32_t i0 = threadIdx.x & ~31u; i0 < td.count; i0 += kBlock) {  // whole warps (lanes past the tile idle)
+      const uint32_t i = i0 + (threadIdx.x & 31u);
+      const bool valid = i < td.count;
+      const uint32_t s = valid ? (ordered ? order[td.first + i] : td.first + i) : td.first;
       const float4 pi = pos[s];
       const bool fluid_i = pi.w > 0.0f;
       uint32_t cx, cy, cz;
@@ -1617,6 +1100,7 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
       uint32_t cnt = 0, bad = 0;
       uint16_t* wp = nbr + s;  // next list entry: nbr[cnt * stride + s]
       const ListPlanes lp = list_planes(g, cst, cx, cy, cz);
+      uint32_t kadd = 0;  // list entry of slot j in the window being taken: j + kadd
       float wpt[kWalls ? 3 * kMaxWallPlanes : 1], wn[kWalls ? 3 * kMaxWallPlanes : 1];
       uint32_t np = 0;
       if (kWalls && fluid_i) {
@@ -1638,8 +1122,7 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
                             });
         }
       }
-      auto visit = [&](uint32_t j) {  // j != s (the callers skip it)
-        const float4 pj = pos[j];
+      auto visit = [&](uint32_t j, const float4& pj) {  // j != s (the walk leaves it out)
         const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
         const float r2 = dx * dx + dy * dy + dz * dz;
         if (r2 <= h2) {
@@ -1671,9 +1154,7 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
           }
           if (rec) {
             if (cnt < cap) {
-              const uint32_t e = list_encode(lp, j);
-              bad |= e >> 31;
-              __stcs(wp, (unsigned short)e);  // streaming store: the list is read once, by the force pass
+              __stcs(wp, (unsigned short)(j + kadd));  // streaming store: the list is read once, by the force pass
               wp += stride;
             }
             ++cnt;
@@ -1683,7 +1164,7 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
       // A boundary particle sums fluid neighbours only: with no fluid particle in its 27
       // cells (none marked wet this substep) its walk would accept nothing.
       bool dry = false;
-      if (!fluid_i) {
+      if (!fluid_i && valid) {
         const uint32_t* wc = wet + S.cell_off;
         dry = true;
         for (int dz = -1; dz <= 1; ++dz) {
@@ -1695,16 +1176,13 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
             for (int dx = -1; dx <= 1; ++dx) {
               const int x = (int)cx + dx;
               if (x < 0 || x >= (int)g.nx) continue;
-              if (wc[((uint32_t)x * g.ny + (uint32_t)y) * g.nz + (uint32_t)z] == epoch) dry = false;
+              if (wc[((uint32_t)z * g.ny + (uint32_t)y) * g.nx + (uint32_t)x] == epoch) dry = false;
             }
           }
         }
       }
-      // Without provider walls: the same test and sums as `visit`, with the list entry
-      // formed from the walked cell's plane offset (kadd, set by cellhook before each cell).
-      uint32_t kadd = 0;
-      auto visit1 = [&](uint32_t j) {  // j != s (the walks skip it)
-        const float4 pj = pos[j];
+      // Without provider walls: the same test and sums as `visit`.
+      auto visit1 = [&](uint32_t j, const float4& pj) {
         const float ddx = pi.x - pj.x, ddy = pi.y - pj.y, ddz = pi.z - pj.z;
         const float r2 = ddx * ddx + ddy * ddy + ddz * ddz;
         if (r2 <= h2) {
@@ -1726,30 +1204,53 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
           }
         }
       };
-      // list entries of the cell about to be walked: (plane << 14) + slot - plane's first slot,
-      // the plane's first slot being that of cell (cx + pl - 1, max(cy - 1, 0), max(cz - 1, 0));
-      // a cell reaching 2^14 slots past it marks the list unusable (consumers walk again)
-      auto cellhook = [&](uint32_t pl, uint32_t jend) {
-        const uint32_t pb = cst[(cx + pl - 1u) * (g.ny * g.nz) + (cy > 0 ? cy - 1 : 0) * g.nz + (cz > 0 ? cz - 1 : 0)];
-        kadd = (pl << kListOffBits) - pb;
-        bad |= (jend > pb && jend - 1u - pb > kListOffMask) ? 1u : 0u;
+      // Take the queued windows, the next candidate's position loaded while the current one is
+      // tested. List entries are (plane << 14) + slot - plane's first slot; a slot 2^14 or more
+      // past it marks the list unusable (consumers walk again).
+      uint32_t nq = 0;
+      const uint32_t full = kWalkQueue - (ordered ? 6u : 2u);  // a row adds one window or two, at 2h bins four to six
+      auto drain = [&]() {
+        uint32_t m = 0, base = 0, ka = 0, k = 0;
+        auto next = [&]() -> uint32_t {
+          if (m == 0u) {
+            if (k == nq) return ~0u;
+            const uint2 win = s_win[k][threadIdx.x];
+            ++k;
+            m = win.x;
+            base = win.y & 0x3fffffffu;
+            const uint32_t pl = win.y >> 30;
+            ka = (pl << kListOffBits) - (pl == 0u ? lp.b0 : (pl == 1u ? lp.b1 : lp.b2));
+          }
+          const uint32_t j = base + (uint32_t)(__ffs(m) - 1);
+          m &= m - 1u;
+          return j;
+        };
+        uint32_t j = next();
+        float4 pj = j != ~0u ? pos[j] : pi;
+        while (j != ~0u) {
+          kadd = ka;
+          const uint32_t jn = next();
+          const float4 pn = jn != ~0u ? pos[jn] : pj;
+          if constexpr (kWalls) visit(j, pj);
+          else visit1(j, pj);
+          j = jn;
+          pj = pn;
+        }
+        nq = 0;
       };
-      if (dry) {
-      } else if (half_walk) {
-        if constexpr (kWalls) {
-          walk27_half(g, cst, halves, pi.x, pi.y, pi.z, cx, cy, cz, h, [&](uint32_t j) {
-            if (j != s) visit(j);
+      walk27_q(
+          g, cst, words + (size_t)(cx % 3) * wstride, pi.x, pi.y, pi.z, cx, cy, cz, h, s, valid && !dry,
+          [&](uint32_t m, uint32_t base, uint32_t pl) {
+            if (nq == kWalkQueue) drain();  // a crowded row
+            const uint32_t pb = pl == 0u ? lp.b0 : (pl == 1u ? lp.b1 : lp.b2);
+            bad |= base + 31u - (uint32_t)__clz(m) - pb > kListOffMask ? 1u : 0u;
+            s_win[nq++][threadIdx.x] = make_uint2(m, base | (pl << 30));
+          },
+          [&]() {
+            if (__any_sync(0xffffffffu, nq > full)) drain();
           });
-        } else {
-          walk27_half_c(g, cst, halves, pi.x, pi.y, pi.z, cx, cy, cz, h, s, cellhook, visit1);
-        }
-      } else {
-        if constexpr (kWalls) {
-          walk27<true>(g, cst, pi.x, pi.y, pi.z, cx, cy, cz, h, visit, s);
-        } else {
-          walk27_c(g, cst, pi.x, pi.y, pi.z, cx, cy, cz, h, s, cellhook, visit1);
-        }
-      }
+      drain();
+      if (!valid) continue;
       nbr_n[s] = cnt | (bad ? kListBad : 0u);
       const float rho = fluid_i ? (mass * sum + sum_b) : ((-pi.w) * w0 + sum);
       const float p = tait(k, rho);
@@ -1853,7 +1354,7 @@ __global__ void __launch_bounds__(kBlock, VXL_FORCE_THREADS_PER_SM / kBlock) k_e
               pair(j, pj, dx, dy, dz, dx * dx + dy * dy + dz * dz);
             }
           } else {
-            walk27<false, true>(g, start + S.cell_off, pi.x, pi.y, pi.z, cx, cy, cz, h, [&](uint32_t j) {
+            walk27(g, start + S.cell_off, pi.x, pi.y, pi.z, cx, cy, cz, h, [&](uint32_t j) {
               if (j == s) return;
               const float4 pj = pos[j];
               const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
@@ -2224,7 +1725,7 @@ __global__ void __launch_bounds__(128) k_e_bforce(
         const ListPlanes lp = list_planes(g, cst, cx, cy, cz);
         for (uint32_t q = 0; q < cnt; ++q) insert(list_decode(lp, nbr[(size_t)q * stride + s]));
       } else {
-        walk27<false, true>(g, cst, pj.x, pj.y, pj.z, cx, cy, cz, k.h, [&](uint32_t ii) {
+        walk27(g, cst, pj.x, pj.y, pj.z, cx, cy, cz, k.h, [&](uint32_t ii) {
           const float4 p = pos[ii];
           if (!(p.w > 0.0f)) return;
           const float dx = p.x - pj.x, dy = p.y - pj.y, dz = p.z - pj.z;
@@ -2253,7 +1754,7 @@ __global__ void __launch_bounds__(128) k_e_bforce(
         bool first = true;
         for (;;) {
           uint32_t best = 0xffffffffu, best_slot = 0;
-          walk27<false, true>(g, cst, pj.x, pj.y, pj.z, cx, cy, cz, k.h, [&](uint32_t ii) {
+          walk27(g, cst, pj.x, pj.y, pj.z, cx, cy, cz, k.h, [&](uint32_t ii) {
             const float4 p = pos[ii];
             if (!(p.w > 0.0f)) return;
             const uint32_t o = orig[ii];
@@ -2553,17 +2054,65 @@ __global__ void k_e_read_fields(const float2* __restrict__ rc, const float* __re
   }
 }
 
-// Per-particle cell (scene-local cell index) of one scene, from its slice of the table.
-__global__ void k_e_export_bins(const uint32_t* __restrict__ start, const uint32_t* __restrict__ orig,
-                                const SceneDev* __restrict__ sc, uint32_t scene, uint32_t* __restrict__ bins) {
+// One scene's table in the reference's cell order (x outermost, z innermost), from the
+// engine's (z outermost): per reference cell its count, then, with the exclusive scan of the
+// counts in ref_start, each cell's particles (scene-local index) and each particle's cell.
+__device__ __forceinline__ uint32_t engine_cell(const GridBox& g, uint32_t c) {
+  const uint32_t z = c % g.nz, xy = c / g.nz, y = xy % g.ny, x = xy / g.ny;
+  return (z * g.ny + y) * g.nx + x;
+}
+
+__global__ void k_e_export_counts(const uint32_t* __restrict__ start, const SceneDev* __restrict__ sc, uint32_t scene,
+                                  uint32_t* __restrict__ ref_start) {
+  const SceneDev& S = sc[scene];
+  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c > S.cells) return;
+  const uint32_t e = S.cell_off + (c < S.cells ? engine_cell(S.g, c) : 0u);
+  ref_start[c] = c < S.cells ? start[e + 1] - start[e] : 0u;
+}
+
+// Exclusive scan in place, one block.
+__global__ void __launch_bounds__(1024) k_e_export_scan(uint32_t* __restrict__ v, uint32_t n) {
+  __shared__ uint32_t ws[32];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t carry = 0;
+  for (uint32_t b0 = 0; b0 < n; b0 += 1024) {
+    const uint32_t i = b0 + threadIdx.x;
+    const uint32_t x = i < n ? v[i] : 0u;
+    uint32_t incl = x;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+      if ((int)lane >= off) incl += y;
+    }
+    __syncthreads();
+    if (lane == 31) ws[w] = incl;
+    __syncthreads();
+    uint32_t before = carry;
+    for (uint32_t k = 0; k < 32; ++k) {
+      if (k < w) before += ws[k];
+      carry += ws[k];
+    }
+    if (i < n) v[i] = before + incl - x;
+  }
+}
+
+__global__ void k_e_export_table(const uint32_t* __restrict__ start, const uint32_t* __restrict__ orig,
+                                 const SceneDev* __restrict__ sc, uint32_t scene,
+                                 const uint32_t* __restrict__ ref_start, uint32_t* __restrict__ items,
+                                 uint32_t* __restrict__ bins) {
   const SceneDev& S = sc[scene];
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= S.cells) return;
-  const uint32_t gc = S.cell_off + c;
-  for (uint32_t q = start[gc]; q < start[gc + 1]; ++q) bins[orig[q] - S.base] = c;
+  const uint32_t e = S.cell_off + engine_cell(S.g, c);
+  uint32_t at = ref_start[c];
+  for (uint32_t q = start[e]; q < start[e + 1]; ++q) {
+    const uint32_t o = orig[q] - S.base;
+    if (items) items[at++] = o;
+    if (bins) bins[o] = c;
+  }
 }
 
-// One scene's slice of the cell table, rebased to the scene's first slot.
 // Contact table entries by global reference index: ent[ids[e]] = e + 1 (ent zeroed before).
 __global__ void k_e_ctab_scatter(const uint32_t* __restrict__ ids, uint32_t n, uint32_t* __restrict__ ent) {
   const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2605,18 +2154,13 @@ __global__ void k_e_export_nbr_entries(const float4* __restrict__ pos, const uin
   }
   const bool fluid_i = pi.w > 0.0f;
   const float h2 = S.k.h2;
-  walk27<true>(g, start + S.cell_off, pi.x, pi.y, pi.z, cx, cy, cz, S.k.h, [&](uint32_t j) {
+  walk27(g, start + S.cell_off, pi.x, pi.y, pi.z, cx, cy, cz, S.k.h, [&](uint32_t j) {
+    if (j == s) return;
     const float4 pj = pos[j];
     const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
     const float r2 = dx * dx + dy * dy + dz * dz;
     if (r2 <= h2 && (fluid_i || pj.w > 0.0f)) out[o++] = orig[j] - base;
-  }, s);
-}
-
-__global__ void k_e_export_items(const uint32_t* __restrict__ orig, uint32_t base, uint32_t n,
-                                 uint32_t* __restrict__ out) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = orig[base + i] - base;
+  });
 }
 
 }  // namespace

@@ -32,7 +32,7 @@ struct Tuning {
   uint32_t block = 256;   // threads per block of the density/force passes (128 or 256)
   uint32_t tile = 256;    // slots per tile (a multiple of 128, at least one block)
   uint32_t waves = 0;     // 0: one block per tile; k > 0: persistent, k x the occupancy limit
-  uint32_t density = 0;   // density kernel without provider walls: 0 per-particle walk, 1 grouped segments
+  uint32_t density = 0;   // accepted and reported for older callers; both values run the one density kernel
 };
 
 struct SceneInfo {
@@ -180,10 +180,9 @@ class Engine {
   void* bpos_ = nullptr;
   uint16_t* nbr_ = nullptr;  // neighbour lists: 16-bit plane-relative entries, list position major
   uint32_t* nbr_n_ = nullptr;
-  uint32_t* halves_ = nullptr;  // 4 words per 32 slots: upper-half masks along x, y, z
-  uint32_t* xorder_ = nullptr;  // density order of the provider-wall variant at doubled bins (lower x halves first)
-  uint32_t* order_ = nullptr;   // grouped density pass: slots of each chunk ordered by octant
-  void* segs_ = nullptr;        // grouped density pass: segments (first position, count | scene << 4)
+  uint32_t* words_ = nullptr;   // candidate-filter words of the sorted slots (sub_word): 3 x wstride_
+  uint32_t wstride_ = 0;
+  uint32_t* order_ = nullptr;   // density pass at doubled bins: slots of each chunk ordered by octant
   float4* blocal_ = nullptr;         // body-frame lattice per boundary slot (reference order), lazily
   BodyPoseDev* poses_d_ = nullptr;   // poses of one scene's bodies (staged per call)
   uint32_t poses_cap_ = 0;
@@ -260,7 +259,6 @@ class Engine {
   bool use_graph_ = true;
   Tuning tuning_;
   int grid_density_ = 0, grid_force_ = 0, grid_bforce_ = 0;
-  int grid_seg_ = 148;  // persistent grid of the grouped density pass (SMs x resident blocks)
   // graph of one tick
   cudaGraphExec_t graph_ = nullptr;
   uint32_t graph_epoch_ = 0;

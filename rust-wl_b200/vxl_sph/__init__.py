@@ -713,7 +713,7 @@ class Batch:
         return items, start, bins, info
 
     def set_tuning(self, block: int, tile: int, waves: int = 0, density: int | None = None):
-        """Launch shape; density 0 (per-particle walk) or 1 (grouped segments), None keeps it."""
+        """Launch shape; density 0 or 1 (one kernel since: the value is kept and reported), None keeps it."""
         t = Tuning()
         t.hdr = header(Tuning)
         if density is None:
