@@ -222,7 +222,7 @@ void Engine::free_all() {
   snap_stream_ = nullptr;
   if (rb_d_) cudaFree(rb_d_);
   rb_d_ = nullptr;
-  void* wd[] = {prov_d_,      wplanes_d_,    pflag_,        pnsum_,        plist_,   pblk_,
+  void* wd[] = {prov_d_,      wplanes_d_,    pflag_,        pnsum_,        ppos_,         plist_,   pblk_,
                 ct_ent_d_[0], ct_ent_d_[1],  ct_ids_d_[0],  ct_ids_d_[1],  ct_start_d_[0],
                 ct_start_d_[1], ct_pl_d_[0], ct_pl_d_[1]};
   for (void* p : wd)
@@ -234,7 +234,7 @@ void Engine::free_all() {
     ct_ent_d_[k] = ct_ids_d_[k] = ct_start_d_[k] = nullptr;
     ct_pl_d_[k] = nullptr;
   }
-  pnsum_ = nullptr;
+  pnsum_ = ppos_ = nullptr;
   if (blocal_) cudaFree(blocal_);
   if (poses_d_) cudaFree(poses_d_);
   blocal_ = nullptr;
@@ -918,6 +918,7 @@ vxl_status Engine::stage_walls() {
   if (walls_any_ && !pflag_) {
     vxl_status s = dalloc(&pflag_, slot_cap_);
     if (s == VXL_OK) s = dalloc((float4**)&pnsum_, slot_cap_);
+    if (s == VXL_OK) s = dalloc((float4**)&ppos_, slot_cap_);
     if (s == VXL_OK) s = dalloc(&plist_, slot_cap_);
     if (s == VXL_OK) s = dalloc(&pblk_, slot_cap_ / kPushedChunk + 2);
     if (s != VXL_OK) return s;
@@ -1503,9 +1504,11 @@ void Engine::enqueue_substep(bool with_reactions) {
                           (float4*)pos_[0], (float4*)vel_[0], sc_d_, tiles_d_, ntiles_, ctl_d_, prov_d_, wplanes_d_,
                           orig_, pflag_, (float4*)pnsum_, ctab(1)));
     LAUNCH(KID_WALLS, k_e_pushed_count<<<nblk, kThreads, 0, st>>>(pflag_, nref, ctl_d_, pblk_));
-    LAUNCH(KID_WALLS, k_e_pushed_emit<<<nblk, kThreads, 0, st>>>(pflag_, nref, pblk_, ctl_d_, plist_));
-    LAUNCH(KID_WALLS, k_e_separate_check<<<148 * 2, kThreads, 0, st>>>((const float4*)pos_[0], sc_d_, plist_,
-                                                                          (const float4*)pnsum_, slot_of_, ctl_d_));
+    LAUNCH(KID_WALLS, k_e_pushed_emit<<<nblk, kThreads, 0, st>>>(pflag_, nref, pblk_, ctl_d_, plist_,
+                                                                 (const float4*)pos_[0], (const float4*)pnsum_, slot_of_,
+                                                                 (float4*)ppos_));
+    LAUNCH(KID_WALLS, k_e_separate_check<<<148 * 4, kCheckTile, 0, st>>>(sc_d_, plist_, (const float4*)pnsum_,
+                                                                           (const float4*)ppos_, ctl_d_));
     LAUNCH(KID_WALLS, k_e_separate<<<1, 1024, 0, st>>>((float4*)pos_[0], sc_d_, S, plist_, (const float4*)pnsum_,
                                                          slot_of_, ctl_d_));
     LAUNCH(KID_WALLS, k_e_wall_rebox<<<key_blocks, kThreads, 0, st>>>((const float4*)pos_[0], sc_d_, tiles_d_,

@@ -205,6 +205,7 @@ class Engine {
   void* pnsum_ = nullptr;       // float4 per reference index: normal sum, scene
   uint32_t* plist_ = nullptr;   // pushed reference indices, ascending
   uint32_t* pblk_ = nullptr;    // pushed count per chunk
+  void* ppos_ = nullptr;        // float4 per pushed particle: projected position, scene
   std::vector<uint32_t> prov_first_st_, prov_count_st_;  // per scene, as staged on the device
   bool walls_any_ = false;      // some scene has providers (selects the walls kernels)
   vxl_status stage_walls();
