@@ -1267,6 +1267,9 @@ vxl_status Engine::stage_spans() {
       if (ge - gs > kReactExactSpan) ch.push_back(LongSpan{idx, gs, ge, 0u});  // a block of its own
     }
   const uint32_t ns = (uint32_t)sp.size(), nc = (uint32_t)ch.size();
+  // the tick graph copies the tables from the pinned mirrors: it stays valid for new contents
+  // of the same buffers and counts (a moving body's torque origin, every tick)
+  bool stale = ns != nspans_ || nc != nlongs_;
   if (!spans_h_ || ns > spans_cap_ || nc > longs_cap_) {
     void* d[] = {spans_d_, longs_d_, breact_d_};
     for (void* p : d)
@@ -1286,6 +1289,7 @@ vxl_status Engine::stage_spans() {
     CU(cudaMallocHost((void**)&breact_h_, cap * 6 * sizeof(float)));
     spans_cap_ = cap;
     longs_cap_ = ccap;
+    stale = true;
   }
   if (ns) std::memcpy(spans_h_, sp.data(), ns * sizeof(SpanDev));
   if (nc) std::memcpy(longs_h_, ch.data(), nc * sizeof(LongSpan));
@@ -1294,7 +1298,7 @@ vxl_status Engine::stage_spans() {
   spans_dirty_ = false;
   rb_dirty_ = true;              // the bodies' span indices follow the staging
   rb_have_reaction_ = false;     // reactions are indexed by the old staging
-  if (graph_) {
+  if (graph_ && stale) {
     cudaGraphExecDestroy(graph_);
     graph_ = nullptr;
   }
