@@ -28,7 +28,7 @@ thread_local std::string g_last_error;
   } while (0)
 
 constexpr int kThreads = 256;
-constexpr uint32_t kBoundaryTile = 128;  // boundary particles per tile of the reaction pass
+constexpr uint32_t kBoundaryTile = 128;  // boundary particles per tile of the reaction pass (= its block)
 inline uint32_t blocks_for(uint64_t n, int t = kThreads) { return (uint32_t)((n + t - 1) / t); }
 
 enum KernelId : int {
@@ -170,6 +170,7 @@ vxl_status Engine::alloc_all() {
   A(dalloc(&nbr_n_, n));
   wstride_ = (uint32_t)((n + 32 + 3) & ~size_t(3));  // the walk reads whole 16-byte groups, up to 32 words past the end
   A(dalloc(&words_, 3ull * wstride_));
+  A(dalloc(&bwet_, n / 32 + 4ull * scene_cap_ + 4));  // kBoundaryTile / 32 words per boundary tile
   A(dalloc(&stage_, 8 * n));
   A(dalloc(&counts_, cell_cap_ + 1));
   A(dalloc(&wet_, cell_cap_ + 1));
@@ -203,7 +204,7 @@ void Engine::free_all() {
   if (graph_) cudaGraphExecDestroy(graph_);
   graph_ = nullptr;
   void* d[] = {pos_[0], pos_[1], vel_[0], vel_[1], orig_, slot_of_, cellrank_, items_, rc_, press_, acc_, xsph_,
-               bforce_, bpos_, nbr_, nbr_n_, words_, order_, stage_, counts_, wet_, start_, partial_, sc_d_, tiles_d_, ctl_d_, spans_d_,
+               bforce_, bpos_, nbr_, nbr_n_, words_, bwet_, order_, stage_, counts_, wet_, start_, partial_, sc_d_, tiles_d_, ctl_d_, spans_d_,
                longs_d_, breact_d_};
   for (void* p : d)
     if (p) cudaFree(p);
@@ -1251,7 +1252,8 @@ vxl_status Engine::stage_spans() {
   std::vector<SpanDev> sp;
   std::vector<LongSpan> ch;
   span_scene_.clear();
-  for (uint32_t q = 0; q < scenes_.size() && q < spans_local_.size(); ++q)
+  uint32_t bword = 0;  // the scene's first word of the wet mask: a boundary tile is kBoundaryTile / 32 words
+  for (uint32_t q = 0; q < scenes_.size() && q < spans_local_.size(); ++q) {
     for (const vxl_sph_span& s : spans_local_[q]) {
       const uint32_t gs = scenes_[q].base + s.start, ge = scenes_[q].base + s.end;
       const uint32_t idx = (uint32_t)sp.size();
@@ -1262,10 +1264,13 @@ vxl_status Engine::stage_spans() {
             rigid = rb_off_[q] + b;
             break;
           }
-      sp.push_back(SpanDev{s.body, s.origin[0], s.origin[1], s.origin[2], gs, ge, rigid});
+      sp.push_back(SpanDev{s.body, s.origin[0], s.origin[1], s.origin[2], gs, ge, rigid, scenes_[q].base + scenes_[q].nf,
+                           bword});
       span_scene_.push_back(q);
       if (ge - gs > kReactExactSpan) ch.push_back(LongSpan{idx, gs, ge, 0u});  // a block of its own
     }
+    bword += (scenes_[q].nb + kBoundaryTile - 1) / kBoundaryTile * (kBoundaryTile / 32);
+  }
   const uint32_t ns = (uint32_t)sp.size(), nc = (uint32_t)ch.size();
   // the tick graph copies the tables from the pinned mirrors: it stays valid for new contents
   // of the same buffers and counts (a moving body's torque origin, every tick)
@@ -1472,7 +1477,7 @@ void Engine::enqueue_substep(bool with_reactions) {
       LAUNCH_ON(KID_BFORCE, side_,
                 k_e_bforce<<<gb, 128, 0, side_>>>(p1, v1, (const float2*)rc_, start_, orig_, nbr_, nbr_n_, nbr_cap_,
                                                   stride, sc_d_, slot_of_, tiles_d_ + ntiles_, nbtiles_, ctl_d_,
-                                                  (float4*)bforce_));
+                                                  (float4*)bforce_, bwet_));
     cudaEventRecord(ev_join_, side_);
     side_pending_ = true;
     if (react) {
@@ -1481,10 +1486,11 @@ void Engine::enqueue_substep(bool with_reactions) {
       if (nlongs_)  // the long spans (tank walls), a block each
         LAUNCH_ON(KID_REACT_LONG, react_,
                   k_react_long<<<nlongs_, kReactThreads, 0, react_>>>((const float4*)bforce_, (const float4*)bpos_,
-                                                                       spans_d_, longs_d_, rb_d_, ctl_d_, breact_d_));
+                                                                       bwet_, spans_d_, longs_d_, rb_d_, ctl_d_,
+                                                                       breact_d_));
       LAUNCH_ON(KID_REACT_SPANS, react_,
                 k_react_spans<<<(nspans_ + kReactSpanWarps - 1) / kReactSpanWarps, 32 * kReactSpanWarps, 0, react_>>>(
-                    (const float4*)bforce_, (const float4*)bpos_, spans_d_, rb_d_, ctl_d_, breact_d_, nspans_));
+                    (const float4*)bforce_, (const float4*)bpos_, bwet_, spans_d_, rb_d_, ctl_d_, breact_d_, nspans_));
       cudaEventRecord(ev_rjoin_, react_);
       react_pending_ = true;
     }

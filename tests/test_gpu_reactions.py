@@ -1,10 +1,53 @@
-"""Wall separation where its check's tiles can go wrong (B200), against the oracle."""
+"""Span reactions and wall separation where their kernels can go wrong (B200).
+
+The compacted span sums against the sequential float32 loop over the recorded reactions; the
+tiled separation check against the oracle.
+"""
 import numpy as np
 import pytest
 
-from test_gpu_parity import F32, _custom, compare_state, pair
+from test_gpu_parity import F32, _custom, assert_bits, compare_state, pair
 
 pytestmark = pytest.mark.gpu
+
+
+def _sequential(bf, bpos, origin, start, end):
+    f = np.zeros(6, F32)
+    with np.errstate(all="ignore"):
+        for k in range(start, end):
+            r = (bpos[k] - origin).astype(F32)
+            v = bf[k]
+            t = (r[1] * v[2] - r[2] * v[1], r[2] * v[0] - r[0] * v[2], r[0] * v[1] - r[1] * v[0])
+            f = (f + np.array([v[0], v[1], v[2], *t], F32)).astype(F32)
+    return f
+
+
+@pytest.mark.parametrize("origin", [(0.1, 0.2, -0.3), (3e18, 0.0, 0.0), (np.inf, 1.0, 0.0)])
+def test_span_sums_equal_the_sequential_loop(vxl, origin):
+    """Spans of every alignment to the mask's words, empty, one, a warp, a chunk, past the length that takes a
+    block, wet in places only; and torque origins with which a dry particle's term is not zero."""
+    from vxl_sph import scenes
+    s = 0.02
+    b = scenes.body_particles([scenes.Body(0, (0.75, 0.03, 0.75), (0.75, -0.05, 0.75))], s, 2 * s, 1, 1000.0)
+    nb = b[0].shape[0]
+    assert nb > 11000
+    rng = np.random.default_rng(2)
+    fluid = scenes.jitter(scenes.fluid_block((0.3, -0.02, 0.4), (30, 4, 9), s), s, 4, 0.2)
+    fluid = np.concatenate([fluid, rng.uniform((0.0, -0.02, 0.0), (1.5, 0.0, 1.5), (60, 3))]).astype(F32)
+    cuts = [(0, 0), (5, 5), (0, 1), (31, 32), (31, 33), (7, 39), (64, 96), (1, 1025), (100, 8292), (3, 8196), (0, nb),
+            (17, nb - 5), (nb - 1, nb)]
+    spec = _custom(vxl, fluid, h=2 * s, spacing=s, boundary=(b[0], b[1], b[2], [(k, origin, i, j) for k, (i, j) in enumerate(cuts)]),
+                   substeps=1)
+    g = vxl.Scene(spec.params, spec.pos, spec.vel, spec.pmass, spec.n_fluid)
+    g.set_record(True)
+    got = g.step_tick(1.0 / 600.0, spec.spans)
+    bf = g.read_fields()[4]
+    assert 0 < np.count_nonzero(np.any(bf != 0, axis=1)) < nb // 2
+    for (i, j), (_, force, torque) in zip(cuts, got):
+        want, have = _sequential(bf, b[0], np.array(origin, F32), i, j), np.concatenate([force, torque])
+        nan = np.isnan(want)  # the NaN's payload is the machine's own
+        assert np.array_equal(nan, np.isnan(have)), (i, j, want, have)
+        assert_bits(have[~nan], want[~nan], f"span {i}:{j}")
 
 
 @pytest.mark.parametrize("n,close", [(2, (0, 1)), (130, (3, 129)), (128, (126, 127)), (300, (5, 290)), (300, None)])
