@@ -105,6 +105,46 @@ __device__ __forceinline__ uint32_t sub_word(int bx, int by, int bz) {
   return (uint32_t)(bx & 255) | ((uint32_t)(by & 255) << 8) | ((uint32_t)(bz & 255) << 16) | (norm << 24);
 }
 
+// IEEE quotients by a shared reciprocal. An IEEE single division costs about 36 issue slots
+// on sm_100a (3.5 results per clock and SM), and a neighbour pair of the force pass has five, by
+// three different denominators. With y = RN(1 / b), q = RN(a y) and the residual r = a - b q
+// exact in an FMA, RN(q + r y) is the correctly rounded a / b (P. Markstein, Computation of
+// elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990; also
+// Muller et al., Handbook of Floating-Point Arithmetic, division by Newton-Raphson), so a
+// denominator's reciprocal is formed once and each quotient by it takes three instructions. One
+// Newton step from an approximation within 1 ulp (rcp.approx) rounds 1 / b correctly unless
+// b's significand is all ones. That case and operands whose quotient or residual could leave
+// the normal range are the caller's to keep out (scene_safe, pair_safe).
+__device__ __forceinline__ float recip_rn(float b) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+  return __fmaf_rn(y, __fmaf_rn(-b, y, 1.0f), y);
+}
+
+__device__ __forceinline__ float quot_rn(float a, float b, float y) {
+  const float q = a * y;
+  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+
+// Scene constants with which pair_safe keeps every quotient of a pair normal: r2 + h001 lies
+// in [2^-27, 2^21], a distance no smaller than 1e-9 in [2^-30, 2^10], and alpha_c scales by
+// at most 2^10 either way.
+__device__ __forceinline__ bool scene_safe(float h, float alpha_c) {
+  return h >= 0x1p-10f && h <= 0x1p10f && (alpha_c == 0.0f || (alpha_c >= 0x1p-10f && alpha_c <= 0x1p10f));
+}
+
+// The pair's numerators are 0 or in [2^-40, 2^40] (sum, the density sum, and mj are positive),
+// and no denominator's significand is all ones. NaN and infinity fail.
+__device__ __forceinline__ bool pair_safe(float sum, float mj, float coef, float vdh, float c, float denom, float dmu) {
+  constexpr uint32_t kLo = 0x2b800000u, kHi = 0x53800000u, kFrac = 0x7fffffu;  // 2^-40, 2^40
+  const uint32_t s = __float_as_uint(sum), m = __float_as_uint(mj), p = __float_as_uint(fabsf(coef)),
+                 v = __float_as_uint(vdh), a = __float_as_uint(c);
+  const uint32_t hi = max(max(max(s, m), max(p, v)), a);
+  const uint32_t lo = min(min(min(s, m), min(p - 1u, v - 1u)), a - 1u);  // 0 - 1 passes
+  const uint32_t frac = min(min(~s & kFrac, ~__float_as_uint(denom) & kFrac), ~__float_as_uint(dmu) & kFrac);
+  return hi <= kHi && lo >= kLo && frac != 0u;
+}
+
 // Tait EOS with the free-surface clamp: crates/vxl-phys-fluid/src/fluid_force.rs:11-29.
 __device__ __forceinline__ float tait(const SphConst& k, float rho) {
   float q = rho / k.rho0;

@@ -33,14 +33,15 @@
 #include "sph_device.cuh"
 
 // Resident threads per SM the density and force passes are compiled for (register
-// budget = 65536 / this). Density at 768 / 1024 / 1280: 0.352 / 0.291 / 0.288 ms on the 1M dam
+// budget = 65536 / this). Force at 1024 / 1280 / 1536: 0.279 / 0.310 / 0.436 ms on the 1M dam
+// break, 2.5 / 2.7 / 3.8 ms on the 10M one (1024 does not spill). Density at 768 / 1024 / 1280: 0.352 / 0.291 / 0.288 ms on the 1M dam
 // break, 5.0 / 4.2 / 4.1 ms on the 10M one with queues of 12 windows (below), and 1280 has no
 // room for longer ones.
 #ifndef VXL_DENSITY_THREADS_PER_SM
 #define VXL_DENSITY_THREADS_PER_SM 1024
 #endif
 #ifndef VXL_FORCE_THREADS_PER_SM
-#define VXL_FORCE_THREADS_PER_SM 1280
+#define VXL_FORCE_THREADS_PER_SM 1024
 #endif
 
 
@@ -1284,6 +1285,7 @@ __global__ void __launch_bounds__(kBlock, VXL_FORCE_THREADS_PER_SM / kBlock) k_e
     SceneDev& S = sc[td.scene];
     const SphConst& k = S.k;
     const float dt = S.dt, vmax = S.vmax, vmax2 = S.vmax2;
+    const bool safe = scene_safe(k.h, k.alpha_c);
     for (uint32_t b0 = 0; b0 < td.count; b0 += kBlock) {
       const uint32_t i = b0 + threadIdx.x;
       const bool valid = i < td.count;
@@ -1310,28 +1312,34 @@ __global__ void __launch_bounds__(kBlock, VXL_FORCE_THREADS_PER_SM / kBlock) k_e
             const float mj = fabsf(pj.w);
             const float r = sqrtf(r2);
             const float tt = h - r;
-            const float coef = mj * (ks * tt * tt) * (ci2 + cj2);
+            const float sp = ks * tt * tt;
+            const float coef = mj * sp * (ci2 + cj2);
             const float denom = fmaxf(r, 1e-9f);
-            const float q = coef / denom;
+            const float vx = vi.x - vj.x, vy = vi.y - vj.y, vz = vi.z - vj.z;
+            const float vdn = -(vx * dx + vy * dy + vz * dz);
+            const bool take = vdn > 0.0f;  // artificial viscosity only when approaching
+            const float vdh = take ? vdn * h : 0.0f;
+            const float dmu = r2 + h001, sum = rho_i + rho_j;
+            const float t2 = h2 - r2;
+            const float w = k6 * t2 * t2 * t2;
+            // the viscosity is computed for every pair and selected, so the warp does not
+            // diverge around it (the sums are the same)
+            const float ysum = recip_rn(sum), yden = recip_rn(denom);
+            const float mu = quot_rn(vdh, dmu, recip_rn(dmu));
+            const float c = mj * quot_rn(alpha_c * mu, 0.5f * sum, 2.0f * ysum) * sp;
+            float q = quot_rn(coef, denom, yden), q2 = quot_rn(c, denom, yden);
+            float f = quot_rn(mj * 2.0f, sum, ysum) * w;
+            if (!(safe && pair_safe(sum, mj, coef, vdh, c, denom, dmu))) {
+              q = coef / denom;
+              q2 = mj * (alpha_c * (vdn * h / dmu) / (0.5f * sum)) * sp / denom;
+              f = mj * 2.0f / sum * w;
+            }
             ax = ax + dx * q;
             ay = ay + dy * q;
             az = az + dz * q;
-            const float vx = vi.x - vj.x, vy = vi.y - vj.y, vz = vi.z - vj.z;
-            const float vdn = -(vx * dx + vy * dy + vz * dz);
-            {
-              // artificial viscosity only when approaching (vdn > 0): computed for every pair and
-              // selected, so the warp does not diverge around it (the sums are the same)
-              const float mu = vdn * h / (r2 + h001);
-              const float c = mj * (alpha_c * mu / (0.5f * (rho_i + rho_j))) * (ks * tt * tt);
-              const float q2 = c / denom;
-              const bool take = vdn > 0.0f;
-              ax = take ? ax + dx * q2 : ax;
-              ay = take ? ay + dy * q2 : ay;
-              az = take ? az + dz * q2 : az;
-            }
-            const float t2 = h2 - r2;
-            const float w = k6 * t2 * t2 * t2;
-            const float f = mj * 2.0f / (rho_i + rho_j) * w;
+            ax = take ? ax + dx * q2 : ax;
+            ay = take ? ay + dy * q2 : ay;
+            az = take ? az + dz * q2 : az;
             xx = xx + (vj.x - vi.x) * f;
             xy = xy + (vj.y - vi.y) * f;
             xz = xz + (vj.z - vi.z) * f;
@@ -1677,21 +1685,25 @@ __global__ void k_e_wall_rebox(const float4* __restrict__ pos, SceneDev* __restr
 // Pair term of the boundary reaction for fluid i on boundary j, from i's side of the
 // reference loop (crates/vxl-phys-fluid/src/fluid_force.rs:182-207): returns
 // q = m_i (coef + cv) / denom, with d = p_i - p_j; the caller applies bforce -= d * q.
-__device__ __forceinline__ float bforce_pair(const SphConst& k, float r2, float dx, float dy, float dz,
+__device__ __forceinline__ float bforce_pair(const SphConst& k, bool safe, float r2, float dx, float dy, float dz,
                                              float rho_i, float ci2, float mi, float4 vi, float rho_j, float cj2,
                                              float mj, float4 vj) {
   const float r = sqrtf(r2);
   const float t = k.h - r;
-  const float coef = mj * (k.ks * t * t) * (ci2 + cj2);
+  const float sp = k.ks * t * t;
+  const float coef = mj * sp * (ci2 + cj2);
   const float denom = fmaxf(r, 1e-9f);
-  float cv = 0.0f;
   const float vx = vi.x - vj.x, vy = vi.y - vj.y, vz = vi.z - vj.z;
   const float vdn = -(vx * dx + vy * dy + vz * dz);
-  if (vdn > 0.0f) {
-    const float mu = vdn * k.h / (r2 + k.h001);
-    cv = mj * (k.alpha_c * mu / (0.5f * (rho_i + rho_j))) * (k.ks * t * t);
-  }
-  return mi * (coef + cv) / denom;
+  const float vdh = vdn > 0.0f ? vdn * k.h : 0.0f;
+  const float dmu = r2 + k.h001, sum = rho_i + rho_j;
+  const float mu = quot_rn(vdh, dmu, recip_rn(dmu));
+  const float cv = mj * quot_rn(k.alpha_c * mu, 0.5f * sum, 2.0f * recip_rn(sum)) * sp;
+  const float num = mi * (coef + (vdn > 0.0f ? cv : 0.0f));
+  if (safe && pair_safe(sum, mj, num, vdh, cv, denom, dmu)) return quot_rn(num, denom, recip_rn(denom));
+  float ce = 0.0f;
+  if (vdn > 0.0f) ce = mj * (k.alpha_c * (vdn * k.h / dmu) / (0.5f * sum)) * sp;
+  return mi * (coef + ce) / denom;
 }
 
 // Reaction on each boundary particle j: the reference accumulates bforce[j] -= F_ij over
@@ -1715,6 +1727,7 @@ __global__ void __launch_bounds__(128) k_e_bforce(
     const GridBox g = S.g;
     const uint32_t* cst = start + S.cell_off;
     const float h2 = k.h2;
+    const bool safe = scene_safe(k.h, k.alpha_c);
     // a tile is at most one particle per thread (kBoundaryTile)
     const uint32_t i = threadIdx.x;
     bool wet = false;
@@ -1768,7 +1781,7 @@ __global__ void __launch_bounds__(128) k_e_bforce(
         const float dx = p.x - pj.x, dy = p.y - pj.y, dz = p.z - pj.z;
         const float r2 = dx * dx + dy * dy + dz * dz;
         const float2 rci = rc[ii];
-        const float q = bforce_pair(k, r2, dx, dy, dz, rci.x, rci.y, p.w, vel[ii], rcj.x, rcj.y, mj, vj);
+        const float q = bforce_pair(k, safe, r2, dx, dy, dz, rci.x, rci.y, p.w, vel[ii], rcj.x, rcj.y, mj, vj);
         bx = bx - dx * q;
         by = by - dy * q;
         bz = bz - dz * q;

@@ -1,12 +1,12 @@
-"""Span reactions and wall separation where their kernels can go wrong (B200).
+"""Span reactions, wall separation and pair quotients where their kernels can go wrong (B200).
 
 The compacted span sums against the sequential float32 loop over the recorded reactions; the
-tiled separation check against the oracle.
+tiled separation check and the force pass's shared-reciprocal quotients against the oracle.
 """
 import numpy as np
 import pytest
 
-from test_gpu_parity import F32, _custom, assert_bits, compare_state, pair
+from test_gpu_parity import F32, _custom, _run_both, assert_bits, compare_state, pair
 
 pytestmark = pytest.mark.gpu
 
@@ -68,3 +68,22 @@ def test_separation_check_over_tiles(vxl, oracle_mod, n, close):
         g.substep(1.0 / 240.0)
         o.substep(1.0 / 240.0)
         compare_state(g, o, f"{n} pushed, close {close}")
+
+
+@pytest.mark.parametrize("h,over", [(0.1, {}), (0.1, dict(tensile_instability_suppression=False)), (3e-4, {}), (2e-3, {}),
+                                    (900.0, {}), (3000.0, {}), (0.1, dict(artificial_viscosity=0.0)),
+                                    (0.1, dict(artificial_viscosity=3e3)), (0.1, dict(rest_density=1e-15)),
+                                    (0.1, dict(rest_density=1e12))])
+def test_pair_quotients_over_scales(vxl, oracle_mod, h, over):
+    """Smoothing lengths, viscosities and densities inside and outside the shared-reciprocal range, pressures of
+    both signs, pairs at rest, slow (1e-20) and fast, coincident pairs: forces and reactions bit for bit."""
+    from vxl_sph import scenes
+    s = 0.5 * h
+    rng = np.random.default_rng(9)
+    pos = scenes.jitter(scenes.fluid_block((0.0, 0.0, 0.0), (6, 5, 6), s), s, 3, 0.3)
+    pos[7] = pos[6]
+    vel = np.zeros_like(pos)
+    vel[:60] = rng.normal(size=(60, 3))
+    vel[60:120] = rng.normal(size=(60, 3)) * 1e-20
+    b = scenes.body_particles([scenes.Body(0, (3 * s, s, 3 * s), (3 * s, -1.2 * s, 3 * s))], s, h, 1, over.get("rest_density", 1000.0))
+    _run_both(vxl, oracle_mod, _custom(vxl, pos, vel=vel, h=h, spacing=s, boundary=b, **over), substeps=2)
