@@ -14,7 +14,6 @@ namespace vxl {
 
 constexpr uint32_t kGridDimMax = 1u << 14;   // crates/vxl-phys-core/src/grid.rs:8
 constexpr uint32_t kErrGridLoop = 1u << 0;    // grid-box doubling loop did not settle
-constexpr uint32_t kErrCanonLarge = 1u << 2;  // a cell above the shared-memory sort size (info)
 
 // Grid box of one substep: crates/vxl-phys-core/src/grid.rs:34-50 (min, bin, dims)
 // plus inv = 1 / bin (crates/vxl-phys-fluid/src/grid.rs:50).

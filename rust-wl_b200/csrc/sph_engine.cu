@@ -1432,9 +1432,10 @@ void Engine::enqueue_substep(bool with_reactions) {
   LAUNCH(KID_SCAN_PARTIAL, k_e_scan_partial<<<148 * 4, kScanThreads, 0, st>>>(counts_, ctl_d_, partial_, start_));
   LAUNCH(KID_SCAN_FINAL, k_e_scan_final<<<148 * 4, kScanThreads, 0, st>>>(counts_, ctl_d_, partial_, start_));
   LAUNCH(KID_PLACE, k_e_place<<<key_blocks, kThreads, 0, st>>>((const uint2*)cellrank_, start_, orig_, tiles_d_,
-                                                               ntiles_, ctl_d_, (uint2*)items_));
-  LAUNCH(KID_CANON, k_e_canon<<<148 * 8, 256, 0, st>>>((const uint2*)items_, start_, ctl_d_, p0, v0, (float4*)pos_[1],
-                                                       (float4*)vel_[1], orig_, slot_of_));
+                                                               ntiles_, ctl_d_, (uint2*)items_, order_));
+  LAUNCH(KID_CANON, k_e_canon<<<std::max<uint32_t>(blocks_for(used_), 1), 256, 0, st>>>(
+                        (const uint2*)items_, order_, start_, (uint32_t)used_, ctl_d_, p0, v0, (float4*)pos_[1],
+                        (float4*)vel_[1], orig_, slot_of_));
   // the candidate-filter words, and at doubled bins the density pass's thread order
   LAUNCH(KID_GROUPS, k_e_groups<<<key_blocks, kGroupChunk, 0, st>>>(p1, sc_d_, tiles_d_, ntiles_, ctl_d_, order_, words_,
                                                                     wstride_));

@@ -167,8 +167,6 @@ namespace {
 
 constexpr int kScanTile = 2048;
 constexpr int kScanThreads = 256;
-constexpr int kCanonSmem = 1024;
-constexpr int kCanonWindow = kCanonSmem / 2;  // window path: keys + segment table in one warp's buffer
 constexpr int kBGatherCap = 64;
 // Density walk: windows queued per thread. h-sized bins need 9 or 10 (a row each), 2h bins
 // about 20. 12 / 14 / 18 / 22 on the 10M dam break: 4.20 / 4.03 / 3.81 / 3.90 ms (shorter queues are
@@ -596,152 +594,52 @@ __global__ void k_e_scan_final(uint32_t* __restrict__ counts, const EngineCtl* _
   }
 }
 
-// Place each slot's (reference index, old slot) at start[cell] + rank (tiles).
+// Place each slot's (reference index, old slot) and its cell at start[cell] + rank (tiles).
 __global__ void k_e_place(const uint2* __restrict__ cellrank, const uint32_t* __restrict__ start,
                           const uint32_t* __restrict__ orig, const TileDev* __restrict__ tiles, uint32_t ntiles,
-                          const EngineCtl* __restrict__ ctl, uint2* __restrict__ items) {
+                          const EngineCtl* __restrict__ ctl, uint2* __restrict__ items, uint32_t* __restrict__ icell) {
   if (ctl->err & kErrCellCap) return;
   for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const TileDev td = tiles[t];
     for (uint32_t i = threadIdx.x; i < td.count; i += blockDim.x) {
       const uint32_t s = td.first + i;
       const uint2 cr = cellrank[s];
-      items[start[cr.x] + cr.y] = make_uint2(orig[s], s);
+      const uint32_t e = start[cr.x] + cr.y;
+      items[e] = make_uint2(orig[s], s);
+      icell[e] = cr.x;
     }
   }
 }
 
-// Per cell: order the placed entries by reference index (grid.rs:56-62) and gather
-// position/velocity into the sorted buffer. A warp scans 32 consecutive cells at a time
-// and handles each non-empty one cooperatively; rank = entries with a smaller index.
-__device__ __forceinline__ void canon_cell(uint32_t b, uint32_t n, int lane, uint32_t* skeys, EngineCtl* ctl,
-                                           const uint2* __restrict__ items, const float4* __restrict__ pos_in,
-                                           const float4* __restrict__ vel_in, float4* __restrict__ pos_out,
-                                           float4* __restrict__ vel_out, uint32_t* __restrict__ orig,
-                                           uint32_t* __restrict__ slot_of) {
-  if (n <= 32) {
-    uint2 it = make_uint2(0xffffffffu, 0u);
-    if ((uint32_t)lane < n) it = items[b + lane];
-    uint32_t rank = 0;
-    for (uint32_t j = 0; j < n; ++j) {
-      const uint32_t kj = __shfl_sync(0xffffffffu, it.x, j);
-      rank += (kj < it.x) ? 1u : 0u;
-    }
-    if ((uint32_t)lane < n) {
-      const uint32_t dst = b + rank;
-      pos_out[dst] = pos_in[it.y];
-      vel_out[dst] = vel_in[it.y];
-      orig[dst] = it.x;
-      slot_of[it.x] = dst;
-    }
-  } else if (n <= (uint32_t)kCanonSmem / 2) {
-    // keys and source slots both staged, so the cell's entries are read from memory once
-    uint32_t* sslot = skeys + kCanonSmem / 2;
-    for (uint32_t e = lane; e < n; e += 32) {
-      const uint2 it = items[b + e];
-      skeys[e] = it.x;
-      sslot[e] = it.y;
-    }
-    __syncwarp();
-    for (uint32_t e = lane; e < n; e += 32) {
-      const uint32_t key = skeys[e], src = sslot[e];
-      uint32_t rank = 0;
-      for (uint32_t j = 0; j < n; ++j) rank += (skeys[j] < key) ? 1u : 0u;
-      const uint32_t dst = b + rank;
-      pos_out[dst] = pos_in[src];
-      vel_out[dst] = vel_in[src];
-      orig[dst] = key;
-      slot_of[key] = dst;
-    }
-    __syncwarp();
-  } else if (n <= (uint32_t)kCanonSmem) {
-    for (uint32_t e = lane; e < n; e += 32) skeys[e] = items[b + e].x;
-    __syncwarp();
-    for (uint32_t e = lane; e < n; e += 32) {
-      const uint2 it = items[b + e];
-      uint32_t rank = 0;
-      for (uint32_t j = 0; j < n; ++j) rank += (skeys[j] < it.x) ? 1u : 0u;
-      const uint32_t dst = b + rank;
-      pos_out[dst] = pos_in[it.y];
-      vel_out[dst] = vel_in[it.y];
-      orig[dst] = it.x;
-      slot_of[it.x] = dst;
-    }
-    __syncwarp();
-  } else {
-    if (lane == 0) atomicOr(&ctl->err, kErrCanonLarge);
-    for (uint32_t e = lane; e < n; e += 32) {
-      const uint2 it = items[b + e];
-      uint32_t rank = 0;
-      for (uint32_t j = 0; j < n; ++j) rank += (items[b + j].x < it.x) ? 1u : 0u;
-      const uint32_t dst = b + rank;
-      pos_out[dst] = pos_in[it.y];
-      vel_out[dst] = vel_in[it.y];
-      orig[dst] = it.x;
-      slot_of[it.x] = dst;
-    }
+// Order the placed entries of each cell by reference index (grid.rs:56-62) and gather
+// position and velocity into the sorted buffer. A thread per entry, which ranks it against
+// its cell's entries (the lanes of a cell read the same ones) while its gathers are in
+// flight: the work spreads evenly whatever the cells hold. With a warp per 32 cells a
+// pool's few crowded rows of cells were left to a few hundred warps: 1.4M pool at doubled bins 185 -> 54
+// us, 10M dam break 501 -> 258, 1M 62 -> 25, 16k 20 -> 7.5.
+__global__ void __launch_bounds__(256) k_e_canon(const uint2* __restrict__ items, const uint32_t* __restrict__ icell,
+                                                 const uint32_t* __restrict__ start, uint32_t n,
+                                                 const EngineCtl* __restrict__ ctl, const float4* __restrict__ pos_in,
+                                                 const float4* __restrict__ vel_in, float4* __restrict__ pos_out,
+                                                 float4* __restrict__ vel_out, uint32_t* __restrict__ orig,
+                                                 uint32_t* __restrict__ slot_of) {
+  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n || (ctl->err & kErrCellCap)) return;
+  const uint2 it = items[e];
+  const uint32_t c = icell[e];
+  const float4 p = pos_in[it.y], v = vel_in[it.y];
+  const uint32_t b = start[c], end = start[c + 1];
+  uint32_t dst = b;
+  uint32_t j = b;
+  for (; j + 4 <= end; j += 4) {
+    const uint32_t k0 = items[j].x, k1 = items[j + 1].x, k2 = items[j + 2].x, k3 = items[j + 3].x;
+    dst += (k0 < it.x ? 1u : 0u) + (k1 < it.x ? 1u : 0u) + (k2 < it.x ? 1u : 0u) + (k3 < it.x ? 1u : 0u);
   }
-}
-
-__global__ void k_e_canon(const uint2* __restrict__ items, const uint32_t* __restrict__ start, EngineCtl* ctl,
-                          const float4* __restrict__ pos_in, const float4* __restrict__ vel_in,
-                          float4* __restrict__ pos_out, float4* __restrict__ vel_out, uint32_t* __restrict__ orig,
-                          uint32_t* __restrict__ slot_of) {
-  __shared__ uint32_t skeys[8][kCanonSmem];
-  if (ctl->err & kErrCellCap) return;
-  const uint32_t total = ctl->cells;
-  const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5;
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32u; base < total; base += warps * 32u) {
-    const uint32_t c = base + lane;
-    uint32_t b = 0, n = 0;
-    if (c < total) {
-      b = start[c];
-      n = start[c + 1] - b;
-    }
-    // Window path: the entries of these 32 cells are contiguous; when they are few and every
-    // cell is small, rank and gather them 32 at a time across cell boundaries, with the
-    // keys and a per-entry (cell start, cell size) table in shared memory.
-    const uint32_t wb = __shfl_sync(0xffffffffu, b, 0);
-    uint32_t we = c < total ? b + n : 0u;
-    uint32_t maxn = n;
-    for (int off = 16; off > 0; off >>= 1) {
-      we = max(we, __shfl_xor_sync(0xffffffffu, we, off));
-      maxn = max(maxn, __shfl_xor_sync(0xffffffffu, maxn, off));
-    }
-    if (maxn <= 32 && we - wb <= (uint32_t)kCanonWindow) {
-      uint32_t* wkeys = skeys[wib];
-      uint32_t* wseg = skeys[wib] + kCanonWindow;
-      const uint32_t rel = b - wb;
-      for (uint32_t q = 0; q < n; ++q) wseg[rel + q] = (rel << 6) | n;  // n <= 32 < 64
-      const uint32_t T = we - wb;
-      for (uint32_t e = lane; e < T; e += 32) wkeys[e] = items[wb + e].x;
-      __syncwarp();
-      for (uint32_t e = lane; e < T; e += 32) {
-        const uint2 it = items[wb + e];
-        const uint32_t seg = wseg[e];
-        const uint32_t s0 = seg >> 6, sn = seg & 63u;
-        uint32_t rank = 0;
-        for (uint32_t j = 0; j < sn; ++j) rank += (wkeys[s0 + j] < it.x) ? 1u : 0u;
-        const uint32_t dst = wb + s0 + rank;
-        pos_out[dst] = pos_in[it.y];
-        vel_out[dst] = vel_in[it.y];
-        orig[dst] = it.x;
-        slot_of[it.x] = dst;
-      }
-      __syncwarp();
-      continue;
-    }
-    uint32_t mask = __ballot_sync(0xffffffffu, n > 0);
-    while (mask) {
-      const int l = __ffs(mask) - 1;
-      mask &= mask - 1;
-      const uint32_t cb = __shfl_sync(0xffffffffu, b, l);
-      const uint32_t cn = __shfl_sync(0xffffffffu, n, l);
-      canon_cell(cb, cn, lane, skeys[wib], ctl, items, pos_in, vel_in, pos_out, vel_out, orig, slot_of);
-    }
-  }
+  for (; j < end; ++j) dst += items[j].x < it.x ? 1u : 0u;
+  pos_out[dst] = p;
+  vel_out[dst] = v;
+  orig[dst] = it.x;
+  slot_of[it.x] = dst;
 }
 
 // Squared gaps from a particle at p in cell c to the faces of that cell, per axis (0 where p

@@ -183,7 +183,8 @@ class Engine {
   uint32_t* words_ = nullptr;   // candidate-filter words of the sorted slots (sub_word): 3 x wstride_
   uint32_t wstride_ = 0;
   uint32_t* bwet_ = nullptr;    // boundary particles with a reaction: a bit each, 4 words per boundary tile
-  uint32_t* order_ = nullptr;   // density pass at doubled bins: slots of each chunk ordered by octant
+  uint32_t* order_ = nullptr;   // density pass at doubled bins: slots of each chunk ordered by octant (before
+                                // k_e_groups: the cell of each placed entry)
   float4* blocal_ = nullptr;         // body-frame lattice per boundary slot (reference order), lazily
   BodyPoseDev* poses_d_ = nullptr;   // poses of one scene's bodies (staged per call)
   uint32_t poses_cap_ = 0;
