@@ -29,6 +29,20 @@ thread_local std::string g_last_error;
 
 constexpr int kThreads = 256;
 constexpr uint32_t kBoundaryTile = 128;  // boundary particles per tile of the reaction pass (= its block)
+static_assert(kBoundaryTile == 4 * kTeams, "k_e_bforce_team: four blocks per boundary tile");
+// Lanes per particle of a pass over a load of n: with few particles a pass is as long as one
+// particle's chain, which more lanes shorten; with many it is bound by instructions, of which
+// they cost up to 2.4 times as many. For density and force the load is the fluid particles and a
+// quarter of the boundary's (many of those are dry). Density with 8 / 4 / 1 lanes: load 11k 20 / 23 / 36 us, 18k
+// 27 / 27 / 37, 28k 32 / 30 / 38, 39k 39 / 38 / 37, 47k (fluid only) 36 / 35 / 29; force: 11k 16 / 17 / 30, 18k
+// 22 / 19 / 31, 39k 30 / 27 / 30 (but its boundary forces, beside it, 22 -> 30), 47k 35 / 29 / 26
+// (fluid only); boundary forces by boundary
+// particles: 11k 17 / 19 / 25, 17k 23 / 22 / 26, 22k 32 / 29 / 22.
+struct TeamLimits {
+  uint64_t eight, four;
+};
+constexpr TeamLimits kTeamDensity{18000, 34000}, kTeamForce{12000, 36000}, kTeamBforce{12000, 20000};
+inline uint32_t team_lanes(uint64_t n, const TeamLimits& t) { return n <= t.eight ? 8u : (n <= t.four ? 4u : 1u); }
 inline uint32_t blocks_for(uint64_t n, int t = kThreads) { return (uint32_t)((n + t - 1) / t); }
 
 enum KernelId : int {
@@ -1418,6 +1432,7 @@ void Engine::enqueue_substep(bool with_reactions) {
   const uint32_t key_blocks = std::min<uint32_t>(std::max<uint32_t>(ntiles_, 1), 148 * 8);
   uint64_t nb_total = 0;
   for (auto& s : scenes_) nb_total += s.nb;
+  const uint64_t load = used_ - nb_total + nb_total / 4;  // of the density and force passes (team_lanes)
   const float4* p0 = (const float4*)pos_[0];
   const float4* v0 = (const float4*)vel_[0];
   const float4* p1 = (const float4*)pos_[1];
@@ -1442,6 +1457,7 @@ void Engine::enqueue_substep(bool with_reactions) {
   const uint32_t stride = (uint32_t)slot_cap_;
   const bool rec = record_;
   const uint32_t per_tile = std::max<uint32_t>(ntiles_, 1);
+  const uint32_t subs = (tuning_.tile + kTeams - 1) / kTeams;  // blocks per tile of the small-scene kernels
   const uint32_t gd = grid_density_ ? (uint32_t)grid_density_ : per_tile;
   const uint32_t gf = grid_force_ ? (uint32_t)grid_force_ : per_tile;
   const uint32_t gb = grid_bforce_ ? (uint32_t)grid_bforce_ : std::max<uint32_t>(nbtiles_, 1);
@@ -1454,6 +1470,11 @@ void Engine::enqueue_substep(bool with_reactions) {
       LAUNCH(KID_DENSITY, k_e_density<256, true><<<gd, 256, 0, st>>>(
                               p1, start_, sc_d_, tiles_d_, ntiles_, ctl_d_, words_, wstride_, (float2*)rc_, press_, nbr_, nbr_n_,
                               nbr_cap_, stride, wet_, order_, prov_d_, wplanes_d_, orig_, ctab(0)));
+  } else if (const uint32_t T = team_lanes(load, kTeamDensity); T > 1) {
+    auto kernel = T == 8 ? k_e_density_team<8> : k_e_density_team<4>;
+    LAUNCH(KID_DENSITY, kernel<<<per_tile * subs, kTeams * T, 0, st>>>(
+                            p1, start_, sc_d_, tiles_d_, subs, ctl_d_, words_, wstride_, (float2*)rc_, press_, nbr_,
+                            nbr_n_, nbr_cap_, stride, wet_));
   } else if (tuning_.block == 128) {
     LAUNCH(KID_DENSITY, k_e_density<128><<<gd, 128, 0, st>>>(p1, start_, sc_d_, tiles_d_, ntiles_, ctl_d_, words_, wstride_,
                                                              (float2*)rc_, press_, nbr_, nbr_n_, nbr_cap_, stride, wet_,
@@ -1474,7 +1495,13 @@ void Engine::enqueue_substep(bool with_reactions) {
       cudaStreamWaitEvent(side_, ev_rjoin_, 0);
       react_pending_ = false;
     }
-    if (bforce)
+    if (const uint32_t T = team_lanes(nb_total, kTeamBforce); bforce && T > 1) {
+      auto kernel = T == 8 ? k_e_bforce_team<8> : k_e_bforce_team<4>;
+      LAUNCH_ON(KID_BFORCE, side_,
+                kernel<<<nbtiles_ * (kBoundaryTile / kTeams), kTeams * T, 0, side_>>>(
+                    p1, v1, (const float2*)rc_, start_, orig_, nbr_, nbr_n_, nbr_cap_, stride, sc_d_, slot_of_,
+                    tiles_d_ + ntiles_, ctl_d_, (float4*)bforce_, bwet_));
+    } else if (bforce)
       LAUNCH_ON(KID_BFORCE, side_,
                 k_e_bforce<<<gb, 128, 0, side_>>>(p1, v1, (const float2*)rc_, start_, orig_, nbr_, nbr_n_, nbr_cap_,
                                                   stride, sc_d_, slot_of_, tiles_d_ + ntiles_, nbtiles_, ctl_d_,
@@ -1496,7 +1523,13 @@ void Engine::enqueue_substep(bool with_reactions) {
       react_pending_ = true;
     }
   }
-  if (tuning_.block == 128)
+  if (const uint32_t T = team_lanes(load, kTeamForce); T > 1) {
+    auto kernel = T == 8 ? k_e_force_team<8> : k_e_force_team<4>;
+    LAUNCH(KID_FORCE, kernel<<<per_tile * subs, kTeams * T, 0, st>>>(
+                          p1, v1, (const float2*)rc_, start_, nbr_, nbr_n_, nbr_cap_, stride, sc_d_, tiles_d_, subs,
+                          ctl_d_, (float4*)pos_[0], (float4*)vel_[0], rec ? (float4*)acc_ : nullptr,
+                          rec ? (float4*)xsph_ : nullptr));
+  } else if (tuning_.block == 128)
     LAUNCH(KID_FORCE, k_e_force<128><<<gf, 128, 0, st>>>(
                           p1, v1, (const float2*)rc_, start_, nbr_, nbr_n_, nbr_cap_, stride, sc_d_, tiles_d_,
                           ntiles_, ctl_d_, (float4*)pos_[0], (float4*)vel_[0], rec ? (float4*)acc_ : nullptr,

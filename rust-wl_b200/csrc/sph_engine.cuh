@@ -1163,6 +1163,65 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
   }
 }
 
+// Terms of one neighbour pair of the force pass (fluid_force.rs:165-214): the pressure and
+// viscosity scales of d = pi - pj, whether the viscosity applies (approaching pairs only), and the XSPH
+// scale of vj - vi.
+struct PairTerms {
+  float q, q2, f;
+  bool take;
+};
+
+__device__ __forceinline__ PairTerms force_pair(const SphConst& k, bool safe, float dx, float dy, float dz, float r2,
+                                                float rho_i, float ci2, const float4& vi, float rho_j, float cj2,
+                                                float mj, const float4& vj) {
+  const float r = sqrtf(r2);
+  const float tt = k.h - r;
+  const float sp = k.ks * tt * tt;
+  const float coef = mj * sp * (ci2 + cj2);
+  const float denom = fmaxf(r, 1e-9f);
+  const float vx = vi.x - vj.x, vy = vi.y - vj.y, vz = vi.z - vj.z;
+  const float vdn = -(vx * dx + vy * dy + vz * dz);
+  PairTerms o;
+  o.take = vdn > 0.0f;
+  const float vdh = o.take ? vdn * k.h : 0.0f;
+  const float dmu = r2 + k.h001, sum = rho_i + rho_j;
+  const float t2 = k.h2 - r2;
+  const float w = k.k6 * t2 * t2 * t2;
+  // the viscosity is computed for every pair and selected, so the warp does not diverge
+  // around it (the sums are the same)
+  const float ysum = recip_rn(sum), yden = recip_rn(denom);
+  const float mu = quot_rn(vdh, dmu, recip_rn(dmu));
+  const float c = mj * quot_rn(k.alpha_c * mu, 0.5f * sum, 2.0f * ysum) * sp;
+  o.q = quot_rn(coef, denom, yden);
+  o.q2 = quot_rn(c, denom, yden);
+  o.f = quot_rn(mj * 2.0f, sum, ysum) * w;
+  if (!(safe && pair_safe(sum, mj, coef, vdh, c, denom, dmu))) {
+    o.q = coef / denom;
+    o.q2 = mj * (k.alpha_c * (vdn * k.h / dmu) / (0.5f * sum)) * sp / denom;
+    o.f = mj * 2.0f / sum * w;
+  }
+  return o;
+}
+
+// Semi-implicit Euler with the CFL clamp (fluid_step.rs:112-123).
+__device__ __forceinline__ void integrate_slot(const SphConst& k, float dt, float vmax, float vmax2, const float4& pi,
+                                               const float4& vi, float ax, float ay, float az, float xx, float xy,
+                                               float xz, float4& p, float4& v) {
+  const float eps = k.eps;
+  float ux = vi.x + ax * dt + xx * eps;
+  float uy = vi.y + ay * dt + xy * eps;
+  float uz = vi.z + az * dt + xz * eps;
+  const float s2 = ux * ux + uy * uy + uz * uz;
+  if (s2 > vmax2) {
+    const float scl = vmax / sqrtf(s2);
+    ux = ux * scl;
+    uy = uy * scl;
+    uz = uz * scl;
+  }
+  p = make_float4(pi.x + ux * dt, pi.y + uy * dt, pi.z + uz * dt, pi.w);
+  v = make_float4(ux, uy, uz, 0.0f);
+}
+
 // Force (gravity + spiky pressure + Monaghan viscosity + XSPH, fluid_force.rs:165-214)
 // fused with integration (semi-implicit Euler + CFL clamp, fluid_step.rs:112-123) for
 // fluid slots; boundary slots are copied unchanged (kinematic within the tick).
@@ -1200,47 +1259,22 @@ __global__ void __launch_bounds__(kBlock, VXL_FORCE_THREADS_PER_SM / kBlock) k_e
         } else {
           const float2 rci = rc[s];
           const float rho_i = rci.x, ci2 = rci.y;
-          const float h = k.h, h2 = k.h2, ks = k.ks, k6 = k.k6, alpha_c = k.alpha_c, h001 = k.h001;
+          const float h = k.h, h2 = k.h2;
           float ax = k.gx, ay = k.gy, az = k.gz;
           float xx = 0.0f, xy = 0.0f, xz = 0.0f;
           auto pair = [&](uint32_t j, const float4& pj, float dx, float dy, float dz, float r2) {
             const float2 rcj = rc[j];
             const float4 vj = vel[j];
-            const float rho_j = rcj.x, cj2 = rcj.y;
-            const float mj = fabsf(pj.w);
-            const float r = sqrtf(r2);
-            const float tt = h - r;
-            const float sp = ks * tt * tt;
-            const float coef = mj * sp * (ci2 + cj2);
-            const float denom = fmaxf(r, 1e-9f);
-            const float vx = vi.x - vj.x, vy = vi.y - vj.y, vz = vi.z - vj.z;
-            const float vdn = -(vx * dx + vy * dy + vz * dz);
-            const bool take = vdn > 0.0f;  // artificial viscosity only when approaching
-            const float vdh = take ? vdn * h : 0.0f;
-            const float dmu = r2 + h001, sum = rho_i + rho_j;
-            const float t2 = h2 - r2;
-            const float w = k6 * t2 * t2 * t2;
-            // the viscosity is computed for every pair and selected, so the warp does not
-            // diverge around it (the sums are the same)
-            const float ysum = recip_rn(sum), yden = recip_rn(denom);
-            const float mu = quot_rn(vdh, dmu, recip_rn(dmu));
-            const float c = mj * quot_rn(alpha_c * mu, 0.5f * sum, 2.0f * ysum) * sp;
-            float q = quot_rn(coef, denom, yden), q2 = quot_rn(c, denom, yden);
-            float f = quot_rn(mj * 2.0f, sum, ysum) * w;
-            if (!(safe && pair_safe(sum, mj, coef, vdh, c, denom, dmu))) {
-              q = coef / denom;
-              q2 = mj * (alpha_c * (vdn * h / dmu) / (0.5f * sum)) * sp / denom;
-              f = mj * 2.0f / sum * w;
-            }
-            ax = ax + dx * q;
-            ay = ay + dy * q;
-            az = az + dz * q;
-            ax = take ? ax + dx * q2 : ax;
-            ay = take ? ay + dy * q2 : ay;
-            az = take ? az + dz * q2 : az;
-            xx = xx + (vj.x - vi.x) * f;
-            xy = xy + (vj.y - vi.y) * f;
-            xz = xz + (vj.z - vi.z) * f;
+            const PairTerms o = force_pair(k, safe, dx, dy, dz, r2, rho_i, ci2, vi, rcj.x, rcj.y, fabsf(pj.w), vj);
+            ax = ax + dx * o.q;
+            ay = ay + dy * o.q;
+            az = az + dz * o.q;
+            ax = o.take ? ax + dx * o.q2 : ax;
+            ay = o.take ? ay + dy * o.q2 : ay;
+            az = o.take ? az + dz * o.q2 : az;
+            xx = xx + (vj.x - vi.x) * o.f;
+            xy = xy + (vj.y - vi.y) * o.f;
+            xz = xz + (vj.z - vi.z) * o.f;
           };
           const uint32_t cnt = nbr_n[s];
           const GridBox g = S.g;
@@ -1276,28 +1310,304 @@ __global__ void __launch_bounds__(kBlock, VXL_FORCE_THREADS_PER_SM / kBlock) k_e
             acc_out[s] = make_float4(ax, ay, az, 0.0f);
             xsph_out[s] = make_float4(xx, xy, xz, 0.0f);
           }
-          const float eps = k.eps;
-          float ux = vi.x + ax * dt + xx * eps;
-          float uy = vi.y + ay * dt + xy * eps;
-          float uz = vi.z + az * dt + xz * eps;
-          const float s2 = ux * ux + uy * uy + uz * uz;
-          if (s2 > vmax2) {
-            const float scl = vmax / sqrtf(s2);
-            ux = ux * scl;
-            uy = uy * scl;
-            uz = uz * scl;
-          }
-          nx = pi.x + ux * dt;
-          ny = pi.y + uy * dt;
-          nz = pi.z + uz * dt;
-          pos_out[s] = make_float4(nx, ny, nz, pi.w);
-          vel_out[s] = make_float4(ux, uy, uz, 0.0f);
+          float4 p, v;
+          integrate_slot(k, dt, vmax, vmax2, pi, vi, ax, ay, az, xx, xy, xz, p, v);
+          nx = p.x;
+          ny = p.y;
+          nz = p.z;
+          pos_out[s] = p;
+          vel_out[s] = v;
         }
       }
       // scenes with provider walls take their fluid AABB after the projection pass
       if (S.prov_count == 0u) block_bbox_accumulate(S.fbox, nx, ny, nz, valid && fluid_i);
     }
   }
+}
+
+// ---------------------------------------------------------------- small scenes: several lanes per particle
+//
+// With few particles on the GPU the passes are bound by the length of one particle's chain
+// (rows, candidates, pairs one after another, each a gather and a few dozen dependent
+// instructions), not by the number of instructions. The team kernels give a particle T lanes
+// (8 or 4): they test its candidates and form its pairs' terms T at a time and put the terms in shared memory, from which one lane per component adds them in the walk's order,
+// so every sum is the one-lane kernels' sum, bit for bit. Terms that are not taken are
+// stored as the neutral element of the addition (-0: x + -0 = x for every x). 2.7k particles,
+// per substep: density 34 -> 16 us, force 26 -> 12, boundary forces 16 -> 11; 33k: 36 -> 26, 30 -> 19,
+// 26 -> 22. Where the lines lie: team_lanes.
+constexpr uint32_t kTeams = 32;     // particles per block
+constexpr uint32_t kTeamList = 64;  // candidates held per particle (pitch + T: the teams of a warp on different banks)
+
+template <uint32_t T>
+__global__ void __launch_bounds__(kTeams * T) k_e_density_team(
+    const float4* __restrict__ pos, const uint32_t* __restrict__ start, const SceneDev* __restrict__ sc,
+    const TileDev* __restrict__ tiles, uint32_t subs, const EngineCtl* __restrict__ ctl,
+    const uint32_t* __restrict__ words, uint32_t wstride, float2* __restrict__ rc, float* __restrict__ press_out,
+    uint16_t* __restrict__ nbr, uint32_t* __restrict__ nbr_n, uint32_t cap, uint32_t stride,
+    const uint32_t* __restrict__ wet) {
+  if (ctl->err & kErrCellCap) return;
+  constexpr uint32_t kMask = (1u << T) - 1u;
+  __shared__ uint32_t s_list[kTeams][kTeamList + T];
+  __shared__ __align__(16) float s_fluid[kTeams][kTeamList + T], s_bound[kTeams][kTeamList + T];
+  const TileDev td = tiles[blockIdx.x / subs];
+  const uint32_t first = blockIdx.x % subs * kTeams;  // this block's particles within the tile
+  if (first >= td.count) return;
+  const uint32_t team = threadIdx.x / T, l = threadIdx.x % T, shift = threadIdx.x & (32u - T);
+  const bool valid = first + team < td.count;
+  const uint32_t s = td.first + (valid ? first + team : 0u);
+  const SceneDev& S = sc[td.scene];
+  const GridBox g = S.g;
+  const SphConst& k = S.k;
+  const uint32_t* cst = start + S.cell_off;
+  const float h2 = k.h2, k6 = k.k6;
+  const float4 pi = pos[s];
+  const bool fluid_i = pi.w > 0.0f;
+  uint32_t cx, cy, cz;
+  bin_of(g, pi.x, pi.y, pi.z, cx, cy, cz);
+  const ListPlanes lp = list_planes(g, cst, cx, cy, cz);
+  bool active = valid;
+  if (!fluid_i) {  // a boundary particle with no fluid in its 27 cells has nothing to sum
+    const uint32_t* wc = wet + S.cell_off;
+    const uint32_t epoch = ctl->epoch;
+    active = false;
+    for (uint32_t r = l; r < 9; r += T) {
+      const int z = (int)cz + (int)(r / 3) - 1, y = (int)cy + (int)(r % 3) - 1;
+      if (z < 0 || z >= (int)g.nz || y < 0 || y >= (int)g.ny) continue;
+      const uint32_t c = ((uint32_t)z * g.ny + (uint32_t)y) * g.nx + cx;
+      active |= wc[c] == epoch || (cx > 0 && wc[c - 1] == epoch) || (cx + 1 < g.nx && wc[c + 1] == epoch);
+    }
+  }
+  active = ((__ballot_sync(0xffffffffu, active) >> shift) & kMask) != 0u && valid;
+  // the particle's rows, row r in lane r mod T (and the ninth in every lane), all loads in flight together
+  const CellGaps w = cell_gaps(g, pi.x, pi.y, pi.z, cx, cy, cz, k.h);
+  uint32_t ja[8 / T], jb[8 / T], ja8 = 0, jb8 = 0;
+#pragma unroll
+  for (uint32_t v = 0; v < 8 / T; ++v) {
+    const int r = (int)(l + v * T);
+    if (!active || !cell_row(g, cst, w, cx, cy, cz, r % 3 - 1, r / 3 - 1, ja[v], jb[v])) ja[v] = jb[v] = 0;
+  }
+  if (!active || !cell_row(g, cst, w, cx, cy, cz, 1, 1, ja8, jb8)) ja8 = jb8 = 0;
+  const int ax = axis_sub(g.minx, pi.x, g.inv, cx) - 32, ay = axis_sub(g.miny, pi.y, g.inv, cy) - 32,
+            az = axis_sub(g.minz, pi.z, g.inv, cz) - 32;
+  const uint32_t* wd = words + (size_t)(cx % 3) * wstride;
+  const uint32_t below = (1u << l) - 1u;
+  float sum = l == 0 && fluid_i ? k.w0 : 0.0f;  // lane 0: fluid terms, lane 1: boundary terms
+  uint32_t cnt = 0, bad = 0, n = 0;              // recorded neighbours, candidates held
+  auto drain = [&]() {
+    __syncwarp();
+    const uint32_t most = __reduce_max_sync(0xffffffffu, n);
+    for (uint32_t q = l; q - l < most; q += T) {  // whole rounds: the same trips in every lane
+      const bool on = q < n;
+      const uint32_t j = on ? s_list[team][q] : s;
+      const float4 pj = pos[j];
+      const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+      const float r2 = dx * dx + dy * dy + dz * dz;
+      const float tt = h2 - r2;
+      const float wv = k6 * tt * tt * tt;
+      const bool near = on && r2 <= h2, fj = pj.w > 0.0f;
+      s_fluid[team][q] = near && fj ? (fluid_i ? wv : pj.w * wv) : -0.0f;
+      s_bound[team][q] = near && fluid_i && !fj ? (-pj.w) * wv : -0.0f;
+      const bool rec = near && (fj || fluid_i);
+      const uint32_t taken = (__ballot_sync(0xffffffffu, rec) >> shift) & kMask;
+      if (rec) {
+        const uint32_t at = cnt + (uint32_t)__popc(taken & below);
+        const uint32_t pl = (j >= lp.b1 ? 1u : 0u) + (j >= lp.b2 ? 1u : 0u);
+        const uint32_t off = j - (pl == 0u ? lp.b0 : (pl == 1u ? lp.b1 : lp.b2));
+        bad |= off > kListOffMask ? 1u : 0u;
+        if (at < cap) nbr[(size_t)at * stride + s] = (unsigned short)((pl << kListOffBits) + off);
+      }
+      cnt += (uint32_t)__popc(taken);
+    }
+    __syncwarp();
+    if (l < 2) {
+      const float* t = l == 0 ? s_fluid[team] : s_bound[team];
+      for (uint32_t q = 0; q < most; q += 4) {  // entries past n hold the neutral element
+        const float4 a = *reinterpret_cast<const float4*>(t + q);
+        sum = sum + a.x;
+        sum = sum + a.y;
+        sum = sum + a.z;
+        sum = sum + a.w;
+      }
+    }
+    __syncwarp();
+    n = 0;
+  };
+#pragma unroll 1
+  for (uint32_t r = 0; r < 9; ++r) {
+    uint32_t j0 = ja8, j1 = jb8;
+#pragma unroll
+    for (uint32_t v = 0; v < 8 / T; ++v) {
+      const uint32_t a0 = __shfl_sync(0xffffffffu, ja[v], (int)(r % T), T);
+      const uint32_t a1 = __shfl_sync(0xffffffffu, jb[v], (int)(r % T), T);
+      if (r / T == v) {
+        j0 = a0;
+        j1 = a1;
+      }
+    }
+    const int my = (int)kSubUnits * ((int)(r % 3) - 1) - ay, mz = (int)kSubUnits * ((int)(r / 3) - 1) - az;
+    const int M = (int)((uint32_t)(-ax & 255) | ((uint32_t)(my & 255) << 8) | ((uint32_t)(mz & 255) << 16) |
+                        (kSubNorm << 24));
+    const int over = -(((int)g.reach_q - (ax * ax + my * my + mz * mz)) >> 1) - 1;  // kept: word . M + over < 0
+    for (uint32_t base = j0 & ~3u; __any_sync(0xffffffffu, base < j1); base += 4 * T) {
+      const uint32_t o = base + 4 * l;  // this lane's four slots
+      uint32_t m = 0;
+      if (o < j1) {
+        const int4 v = *reinterpret_cast<const int4*>(wd + o);
+        m = ((uint32_t)__dp4a(v.x, M, over) >> 31) | ((uint32_t)__dp4a(v.y, M, over) >> 31 << 1) |
+            ((uint32_t)__dp4a(v.z, M, over) >> 31 << 2) | ((uint32_t)__dp4a(v.w, M, over) >> 31 << 3);
+        if (o < j0) m &= 15u << (j0 - o);
+        if (j1 - o < 4u) m &= (1u << (j1 - o)) - 1u;
+        if (s - o < 4u) m &= ~(1u << (s - o));
+      }
+      uint32_t incl = (uint32_t)__popc(m);
+#pragma unroll
+      for (int d = 1; d < (int)T; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d, T);
+        if ((int)l >= d) incl += y;
+      }
+      const uint32_t total = __shfl_sync(0xffffffffu, incl, T - 1, T);
+      if (__any_sync(0xffffffffu, n + total > kTeamList)) drain();
+      uint32_t at = n + incl - (uint32_t)__popc(m);
+#pragma unroll
+      for (uint32_t t = 0; t < 4; ++t)
+        if ((m >> t) & 1u) s_list[team][at++] = o + t;
+      n += total;
+    }
+  }
+  drain();
+  const float sf = __shfl_sync(0xffffffffu, sum, 0, T), sb = __shfl_sync(0xffffffffu, sum, 1, T);
+  const bool any_bad = ((__ballot_sync(0xffffffffu, bad != 0u) >> shift) & kMask) != 0u;
+  if (l == 0 && valid) {
+    nbr_n[s] = cnt | (any_bad ? kListBad : 0u);
+    const float rho = fluid_i ? (k.mass * sf + sb) : ((-pi.w) * k.w0 + sf);
+    const float p = tait(k, rho);
+    rc[s] = make_float2(rho, p / (rho * rho));
+    if (press_out) press_out[s] = p;
+  }
+}
+
+template <uint32_t T>
+__global__ void __launch_bounds__(kTeams * T) k_e_force_team(
+    const float4* __restrict__ pos, const float4* __restrict__ vel, const float2* __restrict__ rc,
+    const uint32_t* __restrict__ start, const uint16_t* __restrict__ nbr, const uint32_t* __restrict__ nbr_n,
+    uint32_t cap, uint32_t stride, SceneDev* __restrict__ sc, const TileDev* __restrict__ tiles, uint32_t subs,
+    const EngineCtl* __restrict__ ctl, float4* __restrict__ pos_out, float4* __restrict__ vel_out,
+    float4* __restrict__ acc_out, float4* __restrict__ xsph_out) {
+  if (ctl->err & kErrCellCap) return;
+  // a team's terms: pressure xyz, viscosity xyz, XSPH xyz of T pairs (9 T words a team: the
+  // teams of a warp fall on different banks)
+  __shared__ __align__(16) float s_term[kTeams][9][T];
+  const TileDev td = tiles[blockIdx.x / subs];
+  const uint32_t first = blockIdx.x % subs * kTeams;
+  if (first >= td.count) return;
+  const uint32_t team = threadIdx.x / T, l = threadIdx.x % T;
+  const bool valid = first + team < td.count;
+  const uint32_t s = td.first + (valid ? first + team : 0u);
+  SceneDev& S = sc[td.scene];
+  const SphConst& k = S.k;
+  const GridBox g = S.g;
+  const uint32_t* cst = start + S.cell_off;
+  const bool safe = scene_safe(k.h, k.alpha_c);
+  const float4 pi = pos[s], vi = vel[s];
+  const float2 rci = rc[s];
+  const bool fluid_i = valid && pi.w > 0.0f;
+  if (valid && !fluid_i && l == 0) {
+    pos_out[s] = pi;
+    vel_out[s] = vi;
+  }
+  const uint32_t cnt = fluid_i ? nbr_n[s] : 0u;
+  const bool listed = cnt <= cap;
+  uint32_t cx, cy, cz;
+  bin_of(g, pi.x, pi.y, pi.z, cx, cy, cz);
+  // lane a < 3: acceleration and XSPH component a
+  float acc = l == 0 ? k.gx : (l == 1 ? k.gy : k.gz), xs = 0.0f;
+  auto round = [&](bool on, const float4& pj, const float4& vj, const float2& rcj) {
+    const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+    const PairTerms o = force_pair(k, safe, dx, dy, dz, dx * dx + dy * dy + dz * dz, rci.x, rci.y, vi, rcj.x, rcj.y,
+                                   fabsf(pj.w), vj);
+    const bool visc = on && o.take;
+    s_term[team][0][l] = on ? dx * o.q : -0.0f;
+    s_term[team][1][l] = on ? dy * o.q : -0.0f;
+    s_term[team][2][l] = on ? dz * o.q : -0.0f;
+    s_term[team][3][l] = visc ? dx * o.q2 : -0.0f;
+    s_term[team][4][l] = visc ? dy * o.q2 : -0.0f;
+    s_term[team][5][l] = visc ? dz * o.q2 : -0.0f;
+    s_term[team][6][l] = on ? (vj.x - vi.x) * o.f : -0.0f;
+    s_term[team][7][l] = on ? (vj.y - vi.y) * o.f : -0.0f;
+    s_term[team][8][l] = on ? (vj.z - vi.z) * o.f : -0.0f;
+    __syncwarp();
+    if (l < 3) {
+#pragma unroll
+      for (uint32_t q = 0; q < T; q += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(&s_term[team][l][q]),
+                     b = *reinterpret_cast<const float4*>(&s_term[team][l + 3][q]),
+                     c = *reinterpret_cast<const float4*>(&s_term[team][l + 6][q]);
+        acc = acc + a.x;
+        acc = acc + b.x;
+        acc = acc + a.y;
+        acc = acc + b.y;
+        acc = acc + a.z;
+        acc = acc + b.z;
+        acc = acc + a.w;
+        acc = acc + b.w;
+        xs = xs + c.x;
+        xs = xs + c.y;
+        xs = xs + c.z;
+        xs = xs + c.w;
+      }
+    }
+    __syncwarp();
+  };
+  {  // the recorded list, T neighbours a round, the next round's loaded beside the current one's terms
+    const uint32_t n = listed ? cnt : 0u;
+    const uint32_t most = __reduce_max_sync(0xffffffffu, n);
+    const ListPlanes lp = list_planes(g, cst, cx, cy, cz);
+    uint32_t j = l < n ? list_decode(lp, nbr[(size_t)l * stride + s]) : s;
+    float4 pj = pos[j], vj = vel[j];
+    float2 rcj = rc[j];
+    uint32_t jn = l + T < n ? list_decode(lp, nbr[(size_t)(l + T) * stride + s]) : s;
+    for (uint32_t q = l; q - l < most; q += T) {
+      const float4 pc = pj, vc = vj;
+      const float2 rcc = rcj;
+      pj = pos[jn];
+      vj = vel[jn];
+      rcj = rc[jn];
+      jn = q + 2 * T < n ? list_decode(lp, nbr[(size_t)(q + 2 * T) * stride + s]) : s;
+      round(q < n, pc, vc, rcc);
+    }
+  }
+  if (__any_sync(0xffffffffu, !listed)) {  // longer or unusable lists: the cells again, T slots at a time
+    const CellGaps w = cell_gaps(g, pi.x, pi.y, pi.z, cx, cy, cz, k.h);
+#pragma unroll 1
+    for (int r = 0; r < 9; ++r) {
+      uint32_t j0 = 0, j1 = 0;
+      if (listed || !cell_row(g, cst, w, cx, cy, cz, r % 3 - 1, r / 3 - 1, j0, j1)) j0 = j1 = 0;
+      const uint32_t most = __reduce_max_sync(0xffffffffu, j1 - j0);
+      for (uint32_t q = 0; q < most; q += T) {
+        const uint32_t j = j0 + q + l;
+        const bool in = j < j1 && j != s;
+        const float4 pj = in ? pos[j] : pi;
+        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+        const bool on = in && dx * dx + dy * dy + dz * dz <= k.h2;
+        if (__any_sync(0xffffffffu, on)) round(on, pj, on ? vel[j] : vi, on ? rc[j] : rci);
+      }
+    }
+  }
+  const float ax = __shfl_sync(0xffffffffu, acc, 0, T), ay = __shfl_sync(0xffffffffu, acc, 1, T),
+              az = __shfl_sync(0xffffffffu, acc, 2, T), xx = __shfl_sync(0xffffffffu, xs, 0, T),
+              xy = __shfl_sync(0xffffffffu, xs, 1, T), xz = __shfl_sync(0xffffffffu, xs, 2, T);
+  float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f), v;
+  if (fluid_i && l == 0) {
+    if (acc_out) {
+      acc_out[s] = make_float4(ax, ay, az, 0.0f);
+      xsph_out[s] = make_float4(xx, xy, xz, 0.0f);
+    }
+    integrate_slot(k, S.dt, S.vmax, S.vmax2, pi, vi, ax, ay, az, xx, xy, xz, p, v);
+    pos_out[s] = p;
+    vel_out[s] = v;
+  }
+  // scenes with provider walls take their fluid AABB after the projection pass
+  if (S.prov_count == 0u) block_bbox_accumulate(S.fbox, p.x, p.y, p.z, fluid_i && l == 0);
 }
 
 // ---------------------------------------------------------------- provider walls after integration
@@ -1604,6 +1914,13 @@ __device__ __forceinline__ float bforce_pair(const SphConst& k, bool safe, float
   return mi * (coef + ce) / denom;
 }
 
+// Whether a boundary particle's terms count in its span's sums: without force it adds only
+// zeros, unless its arm is not a small finite number.
+__device__ __forceinline__ bool bforce_wet(float bx, float by, float bz, const float4& p) {
+  const bool arm = fabsf(p.x) < kReactArm && fabsf(p.y) < kReactArm && fabsf(p.z) < kReactArm;  // false for NaN
+  return !(bx == 0.0f && by == 0.0f && bz == 0.0f) || !arm;
+}
+
 // Reaction on each boundary particle j: the reference accumulates bforce[j] -= F_ij over
 // fluid i in ascending reference index (the outer loop of force_pass_serial). Here the
 // boundary particle takes its fluid neighbours (recorded by the density pass, or found by
@@ -1712,14 +2029,169 @@ __global__ void __launch_bounds__(128) k_e_bforce(
         }
       }
       bforce[o] = make_float4(bx, by, bz, 0.0f);
-      // a particle without force adds only zeros to its span's sums, unless its arm is not finite
-      wet = !(bx == 0.0f && by == 0.0f && bz == 0.0f) ||
-            !(fmaxf(fmaxf(fabsf(pj.x), fabsf(pj.y)), fabsf(pj.z)) < kReactArm) || pj.x != pj.x || pj.y != pj.y ||
-            pj.z != pj.z;
+      wet = bforce_wet(bx, by, bz, pj);
     }
     const uint32_t wm = __ballot_sync(0xffffffffu, wet);
     if ((threadIdx.x & 31) == 0) bwet[4 * t + (threadIdx.x >> 5)] = wm;
   }
+}
+
+// The same with T lanes per boundary particle (see the small-scene kernels above): the
+// neighbours' reference indices are ranked against one another in shared memory instead of
+// inserted one by one, and the pairs' terms formed T at a time and subtracted in order by a lane per
+// component (x - 0 = x: the neutral term). A block is 32 consecutive boundary particles, a
+// word of the wet mask.
+template <uint32_t T>
+__global__ void __launch_bounds__(kTeams * T) k_e_bforce_team(
+    const float4* __restrict__ pos, const float4* __restrict__ vel, const float2* __restrict__ rc,
+    const uint32_t* __restrict__ start, const uint32_t* __restrict__ orig, const uint16_t* __restrict__ nbr,
+    const uint32_t* __restrict__ nbr_n, uint32_t cap, uint32_t stride, const SceneDev* __restrict__ sc,
+    const uint32_t* __restrict__ slot_of, const TileDev* __restrict__ btiles, EngineCtl* ctl,
+    float4* __restrict__ bforce, uint32_t* __restrict__ bwet) {
+  if (ctl->err & kErrCellCap) return;
+  static_assert(kBGatherCap <= (int)kTeamList, "a team's list holds the gathered neighbours");
+  constexpr uint32_t kMask = (1u << T) - 1u;
+  __shared__ uint32_t s_key[kTeams][kTeamList + T], s_slot[kTeams][kTeamList + T], s_sorted[kTeams][kTeamList + T];
+  __shared__ __align__(16) float s_term[kTeams][3][T];
+  __shared__ uint32_t s_wet;
+  const uint32_t t = blockIdx.x / 4, first = blockIdx.x % 4 * kTeams;  // a boundary tile is 128 particles
+  const TileDev td = btiles[t];
+  const uint32_t team = threadIdx.x / T, l = threadIdx.x % T, shift = threadIdx.x & (32u - T);
+  if (threadIdx.x == 0) s_wet = 0u;
+  __syncthreads();
+  const bool valid = first + team < td.count;
+  const SceneDev& S = sc[td.scene];
+  const SphConst& k = S.k;
+  const GridBox g = S.g;
+  const uint32_t* cst = start + S.cell_off;
+  const bool safe = scene_safe(k.h, k.alpha_c);
+  const uint32_t o = td.first + (valid ? first + team : 0u);
+  const uint32_t s = slot_of[o];
+  const float4 pj = pos[s], vj = vel[s];
+  const float2 rcj = rc[s];
+  const float mj = -pj.w;
+  uint32_t cx, cy, cz;
+  bin_of(g, pj.x, pj.y, pj.z, cx, cy, cz);
+  const uint32_t cnt = valid ? nbr_n[s] : 0u;
+  const bool listed = cnt <= cap;
+  uint32_t n = listed ? cnt : 0u;
+  bool overflow = false;
+  if (listed) {
+    const ListPlanes lp = list_planes(g, cst, cx, cy, cz);
+    for (uint32_t q = l; q < n; q += T) {
+      const uint32_t ii = list_decode(lp, nbr[(size_t)q * stride + s]);
+      s_slot[team][q] = ii;
+      s_key[team][q] = orig[ii];
+    }
+  }
+  const CellGaps w = cell_gaps(g, pj.x, pj.y, pj.z, cx, cy, cz, k.h);
+  if (__any_sync(0xffffffffu, !listed)) {  // longer or unusable lists: the cells again, T slots at a time
+#pragma unroll 1
+    for (int r = 0; r < 9; ++r) {
+      uint32_t j0 = 0, j1 = 0;
+      if (listed || !cell_row(g, cst, w, cx, cy, cz, r % 3 - 1, r / 3 - 1, j0, j1)) j0 = j1 = 0;
+      const uint32_t most = __reduce_max_sync(0xffffffffu, j1 - j0);
+      for (uint32_t q = 0; q < most; q += T) {
+        const uint32_t ii = j0 + q + l;
+        bool on = false;
+        if (ii < j1) {
+          const float4 p = pos[ii];
+          const float dx = p.x - pj.x, dy = p.y - pj.y, dz = p.z - pj.z;
+          on = p.w > 0.0f && dx * dx + dy * dy + dz * dz <= k.h2;
+        }
+        const uint32_t taken = (__ballot_sync(0xffffffffu, on) >> shift) & kMask;
+        const uint32_t at = n + (uint32_t)__popc(taken & ((1u << l) - 1u));
+        if (on && at < (uint32_t)kBGatherCap) {
+          s_slot[team][at] = ii;
+          s_key[team][at] = orig[ii];
+        }
+        n += (uint32_t)__popc(taken);
+      }
+    }
+    overflow = n > (uint32_t)kBGatherCap;
+    if (overflow) n = 0;
+  }
+  __syncwarp();
+  for (uint32_t q = l; q < n; q += T) {
+    const uint32_t key = s_key[team][q];
+    uint32_t rank = 0;
+    for (uint32_t m = 0; m < n; ++m) rank += s_key[team][m] < key ? 1u : 0u;
+    s_sorted[team][rank] = s_slot[team][q];
+  }
+  __syncwarp();
+  float b = 0.0f;  // lane a < 3: component a
+  auto pair_q = [&](uint32_t ii, float& dx, float& dy, float& dz) {
+    const float4 p = pos[ii];
+    dx = p.x - pj.x;
+    dy = p.y - pj.y;
+    dz = p.z - pj.z;
+    const float2 rci = rc[ii];
+    return bforce_pair(k, safe, dx * dx + dy * dy + dz * dz, dx, dy, dz, rci.x, rci.y, p.w, vel[ii], rcj.x, rcj.y, mj, vj);
+  };
+  const uint32_t most = __reduce_max_sync(0xffffffffu, n);
+  for (uint32_t q = l; q - l < most; q += T) {
+    float dx = 0.0f, dy = 0.0f, dz = 0.0f, qq = 0.0f;
+    if (q < n) qq = pair_q(s_sorted[team][q], dx, dy, dz);
+    s_term[team][0][l] = q < n ? dx * qq : 0.0f;
+    s_term[team][1][l] = q < n ? dy * qq : 0.0f;
+    s_term[team][2][l] = q < n ? dz * qq : 0.0f;
+    __syncwarp();
+    if (l < 3) {
+#pragma unroll
+      for (uint32_t c = 0; c < T; c += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(&s_term[team][l][c]);
+        b = b - x.x;
+        b = b - x.y;
+        b = b - x.z;
+        b = b - x.w;
+      }
+    }
+    __syncwarp();
+  }
+  if (__any_sync(0xffffffffu, overflow)) {
+    // more fluid neighbours than the list holds: in ascending reference index by repeated
+    // minimum search, the team's lanes over the candidates; counted in ctl->slow_gathers
+    if (overflow && l == 0) atomicAdd(&ctl->slow_gathers, 1u);
+    uint32_t last = 0;
+    bool begun = false, more = overflow;
+    while (__any_sync(0xffffffffu, more)) {
+      unsigned long long best = ~0ull;  // reference index, slot
+      if (more) {
+#pragma unroll 1
+        for (int r = 0; r < 9; ++r) {
+          uint32_t j0, j1;
+          if (!cell_row(g, cst, w, cx, cy, cz, r % 3 - 1, r / 3 - 1, j0, j1)) continue;
+          for (uint32_t ii = j0 + l; ii < j1; ii += T) {
+            const float4 p = pos[ii];
+            if (!(p.w > 0.0f)) continue;
+            const uint32_t oi = orig[ii];
+            if (begun && oi <= last) continue;
+            const float dx = p.x - pj.x, dy = p.y - pj.y, dz = p.z - pj.z;
+            if (!(dx * dx + dy * dy + dz * dz <= k.h2)) continue;
+            best = min(best, ((unsigned long long)oi << 32) | ii);
+          }
+        }
+      }
+#pragma unroll
+      for (int d = 1; d < (int)T; d <<= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, d, T));
+      more = more && best != ~0ull;
+      if (more) {
+        float dx, dy, dz;
+        const float qq = pair_q((uint32_t)best, dx, dy, dz);
+        b = b - (l == 0 ? dx : (l == 1 ? dy : dz)) * qq;
+        last = (uint32_t)(best >> 32);
+        begun = true;
+      }
+    }
+  }
+  const float bx = __shfl_sync(0xffffffffu, b, 0, T), by = __shfl_sync(0xffffffffu, b, 1, T),
+              bz = __shfl_sync(0xffffffffu, b, 2, T);
+  if (valid && l == 0) {
+    bforce[o] = make_float4(bx, by, bz, 0.0f);
+    if (bforce_wet(bx, by, bz, pj)) atomicOr(&s_wet, 1u << team);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) bwet[blockIdx.x] = s_wet;
 }
 
 // Per-span force and torque about the body origin (fluid_boundary.rs:10-28), added to

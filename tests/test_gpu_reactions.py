@@ -87,3 +87,53 @@ def test_pair_quotients_over_scales(vxl, oracle_mod, h, over):
     vel[60:120] = rng.normal(size=(60, 3)) * 1e-20
     b = scenes.body_particles([scenes.Body(0, (3 * s, s, 3 * s), (3 * s, -1.2 * s, 3 * s))], s, h, 1, over.get("rest_density", 1000.0))
     _run_both(vxl, oracle_mod, _custom(vxl, pos, vel=vel, h=h, spacing=s, boundary=b, **over), substeps=2)
+
+
+def _edge_scenes(vxl):
+    from vxl_sph import scenes
+    rng = np.random.default_rng(17)
+    s = 0.025
+    plate = scenes.body_particles([scenes.Body(0, (0.2, 0.05, 0.2), (0.125, -0.05, 0.125))], s, 4 * s, 1, 1000.0)
+    walled = scenes.small_dam(n=(9, 8, 7), spacing=0.05, tank=(0.7, 0.6, 0.5), seed=8)
+    return [_custom(vxl, rng.uniform(0.0, 0.08, (230, 3)).astype(F32), h=0.1),  # one crowded cell
+            _custom(vxl, scenes.jitter(scenes.fluid_block((0, 0, 0), (9, 8, 9), s), s, 5), h=3 * s, spacing=s),  # > 64 neighbours
+            _custom(vxl, scenes.fluid_block((0.0, 0.0, 0.0), (10, 8, 10), s), h=4 * s, spacing=s, boundary=plate),  # reactions too
+            _custom(vxl, rng.uniform(0.0, 0.9, (701, 3)).astype(F32), h=0.1, max_bins=100),  # doubled bins
+            walled]
+
+
+@pytest.mark.parametrize("filler", [19000, 30000, 50000])
+def test_scenes_step_the_same_beside_a_filler(vxl, filler):
+    """The lanes per particle follow the whole batch's size: edge scenes alone (eight lanes) and beside a block that
+    brings the passes to four lanes and to one, bitwise, with their reactions."""
+    from vxl_sph import scenes
+    specs = _edge_scenes(vxl)
+    alone = vxl.Batch(specs)
+    n = int(round(filler ** (1 / 3)))
+    big = _custom(vxl, scenes.jitter(scenes.fluid_block((0, 0, 0), (n, n, n), 0.05), 0.05, 6))
+    both = vxl.Batch(specs + [big])
+    for t in range(2):
+        ra, rb = alone.step_tick(1.0 / 60.0), both.step_tick(1.0 / 60.0)
+        assert len(ra) == len(rb) >= 6
+        for (b1, f1, t1), (b2, f2, t2) in zip(ra, rb):
+            assert b1 == b2 and f1.tobytes() == f2.tobytes() and t1.tobytes() == t2.tobytes(), (t, b1)
+        for q in range(len(specs)):
+            for x, y in zip(alone.read_state(q), both.read_state(q)):
+                assert x.tobytes() == y.tobytes(), (t, q)
+
+
+@pytest.mark.parametrize("walls", [2600, 14000, 23000])
+def test_boundary_forces_over_lane_counts(vxl, walls):
+    """Boundary forces with eight, four and one lane per particle: the edge scenes' reactions beside a dry plate
+    of `walls` boundary particles."""
+    from vxl_sph import scenes
+    specs = [_edge_scenes(vxl)[k] for k in (2, 0)]  # (a handle of one scene takes its spans per call)
+    half = 0.02 * (walls / 2) ** 0.5 / 2
+    plate = scenes.body_particles([scenes.Body(0, (half, 0.02, half), (0.0, -0.5, 0.0))], 0.02, 0.04, 1, 1000.0)
+    assert 0.7 * walls < plate[0].shape[0] < 1.4 * walls
+    far = _custom(vxl, [[0.0, 0.5, 0.0]], h=0.04, spacing=0.02, boundary=plate)
+    alone, both = vxl.Batch(specs), vxl.Batch(specs + [far])
+    for t in range(2):
+        a, b = alone.step_tick(1.0 / 60.0)[0], both.step_tick(1.0 / 60.0)[0]
+        assert np.any(a[1] != 0)
+        assert a[1].tobytes() == b[1].tobytes() and a[2].tobytes() == b[2].tobytes(), t
