@@ -30,19 +30,29 @@ constexpr uint32_t kStaticMaxCells = 1u << 19;      // 524,288
 constexpr int kTile = 2048;
 constexpr int kTileThreads = 256;
 constexpr uint32_t kMaxTiles = (kStaticMaxCells + kTile - 1) / kTile;  // 256
-constexpr int kWideThreads = 512;                                          // block of ks_canon_wide
-constexpr uint32_t kWideRank = 2048;  // cells up to this size are ranked in shared memory
-constexpr uint32_t kWideSmemWords = (kStaticMaxParticles + 31) / 32 > kWideRank ? (kStaticMaxParticles + 31) / 32
-                                                                               : kWideRank;  // 64 KB
+constexpr uint32_t kBoxBlocks = 148 * 2;  // blocks of ks_box, each leaving one box
+constexpr int kBoxThreads = 256;
+constexpr int kWideThreads = 512;     // block of ks_canon_wide
+constexpr uint32_t kWideRank = 2048;  // cells up to this size are ranked entry against entry
+constexpr uint32_t kMaxWide = kStaticMaxParticles / (kWideRank + 1) + 1;  // larger cells there can be
+constexpr uint32_t kWideSmemWords = (kStaticMaxParticles + 31) / 32;      // 64 KB: a bit per particle
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 constexpr size_t kCountsOff = 0;
 constexpr size_t kRankOff = align256(kCountsOff + (size_t)(kStaticMaxCells + 1) * 4);
 constexpr size_t kTmpOff = align256(kRankOff + (size_t)kStaticMaxParticles * 8);
 constexpr size_t kPartialOff = align256(kTmpOff + (size_t)kStaticMaxParticles * 4);
-constexpr size_t kBoxOff = align256(kPartialOff + (size_t)kMaxTiles * 4);
-constexpr size_t kGridOff = align256(kBoxOff + 6 * 4);
-constexpr size_t kScratchBytes = align256(kGridOff + sizeof(GridBox));
+constexpr size_t kGridOff = align256(kPartialOff + (size_t)kMaxTiles * 4);
+constexpr size_t kCtlOff = align256(kGridOff + sizeof(GridBox));
+constexpr size_t kScratchBytes = align256(kCtlOff + sizeof(uint32_t) * (3 + kMaxWide));
+static_assert(kBoxBlocks * 6 <= kStaticMaxParticles, "the blocks' boxes use the placement's words");
+
+// Control words at kCtlOff: blocks done in ks_box and in ks_scan_partial (both 0 between
+// calls; the array starts zeroed), cells above kWideRank, and their indices.
+struct Ctl {
+  uint32_t box_done, scan_done, nwide;
+  uint32_t wide[kMaxWide];
+};
 
 // The working memory (about 8.4 MB). Host code must not pass this name to a kernel: on
 // the host it is only a stand-in; the device address comes from cudaGetSymbolAddress.
@@ -56,46 +66,75 @@ vxl_status fail(vxl_status s, const std::string& m) {
   return s;
 }
 
-__device__ __forceinline__ void box_reduce(uint32_t* acc, float x, float y, float z, bool valid) {
-  uint32_t mn[3], mx[3];
-  const float v[3] = {x, y, z};
+// Bounding box and grid, and the counts zeroed (the array keeps the previous call's
+// contents), in one launch: each block leaves the box of its particles, and whichever finishes
+// last (an atomic count; nothing waits) reduces the blocks' boxes and applies the grid rule.
+// Six global atomics per warp on one box took 13k turns per address at 430k particles.
+__global__ void __launch_bounds__(kBoxThreads) ks_box(const float* __restrict__ xyz, uint32_t n, float h,
+                                                      uint32_t max_bins, uint32_t* __restrict__ boxes, GridBox* g,
+                                                      uint32_t* __restrict__ counts, Ctl* ctl) {
+  __shared__ uint32_t s_box[6][kBoxThreads / 32];
+  __shared__ bool last;
+  const uint32_t step = gridDim.x * kBoxThreads;
+  for (uint32_t c = blockIdx.x * kBoxThreads + threadIdx.x; c <= max_bins; c += step) counts[c] = 0u;
+  uint32_t mn[3] = {~0u, ~0u, ~0u}, mx[3] = {0u, 0u, 0u};
+  for (uint32_t i = blockIdx.x * kBoxThreads + threadIdx.x; i < n; i += step)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float v = xyz[3 * i + a];
+      if (v == v) {  // NaN never wins
+        mn[a] = min(mn[a], f2o(v));
+        mx[a] = max(mx[a], f2o(v));
+      }
+    }
+  auto reduce = [&]() {  // over the block, into thread a < 6's s_box[a][0]
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const uint32_t lo = __reduce_min_sync(0xffffffffu, mn[a]), hi = __reduce_max_sync(0xffffffffu, mx[a]);
+      if (lane == 0) {
+        s_box[a][w] = lo;
+        s_box[3 + a][w] = hi;
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+      uint32_t v = s_box[threadIdx.x][0];
+      for (int k = 1; k < kBoxThreads / 32; ++k)
+        v = threadIdx.x < 3 ? min(v, s_box[threadIdx.x][k]) : max(v, s_box[threadIdx.x][k]);
+      s_box[threadIdx.x][0] = v;
+    }
+    __syncthreads();
+  };
+  reduce();
+  if (threadIdx.x < 6) boxes[6 * blockIdx.x + threadIdx.x] = s_box[threadIdx.x][0];
+  __threadfence();  // this block's box is visible before it counts itself done
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&ctl->box_done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const bool ok = valid && (v[a] == v[a]);
-    mn[a] = ok ? f2o(v[a]) : 0xffffffffu;
-    mx[a] = ok ? f2o(v[a]) : 0u;
+    mn[a] = ~0u;
+    mx[a] = 0u;
   }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      mn[a] = min(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], off));
-      mx[a] = max(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], off));
-    }
-  if ((threadIdx.x & 31) == 0)
+  for (uint32_t k = threadIdx.x; k < gridDim.x; k += kBoxThreads)
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      if (mn[a] != 0xffffffffu) atomicMin(&acc[a], mn[a]);
-      if (mx[a] != 0u) atomicMax(&acc[3 + a], mx[a]);
+      mn[a] = min(mn[a], __ldcg(boxes + 6 * k + a));  // written by other blocks: skip L1
+      mx[a] = max(mx[a], __ldcg(boxes + 6 * k + 3 + a));
     }
-}
-
-__global__ void ks_init(uint32_t* box) {
-  if (threadIdx.x < 3) box[threadIdx.x] = 0xffffffffu;
-  else if (threadIdx.x < 6) box[threadIdx.x] = 0u;
-}
-
-__global__ void ks_bbox(const float* __restrict__ xyz, uint32_t n, uint32_t* box) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool ok = i < n;
-  box_reduce(box, ok ? xyz[3 * i] : 0.f, ok ? xyz[3 * i + 1] : 0.f, ok ? xyz[3 * i + 2] : 0.f, ok);
-}
-
-__global__ void ks_gridbox(const uint32_t* box, float h, uint32_t max_bins, GridBox* g) {
-  if (threadIdx.x != 0) return;
-  GridBox gb;
-  grid_box(o2f(box[0]), o2f(box[1]), o2f(box[2]), o2f(box[3]), o2f(box[4]), o2f(box[5]), h, max_bins, gb);
-  *g = gb;
+  __syncthreads();
+  reduce();
+  if (threadIdx.x == 0) {
+    GridBox gb;
+    grid_box(o2f(s_box[0][0]), o2f(s_box[1][0]), o2f(s_box[2][0]), o2f(s_box[3][0]), o2f(s_box[4][0]), o2f(s_box[5][0]),
+             h, max_bins, gb);
+    *g = gb;
+    ctl->box_done = 0u;
+    ctl->nwide = 0u;
+  }
 }
 
 __global__ void ks_keys(const float* __restrict__ xyz, uint32_t n, const GridBox* __restrict__ gp,
@@ -115,43 +154,51 @@ __global__ void ks_keys(const float* __restrict__ xyz, uint32_t n, const GridBox
   cellrank[i] = make_uint2(c, base + __popc(peers & ((1u << lane) - 1u)));
 }
 
+// Per-tile sums of the counts, and in the block that finishes last their exclusive scan in
+// place and the total.
 __global__ void ks_scan_partial(const uint32_t* __restrict__ counts, const GridBox* __restrict__ gp,
-                                uint32_t* __restrict__ partial) {
-  const uint32_t total = gp->total, base = blockIdx.x * kTile;
+                                uint32_t* __restrict__ partial, uint32_t* __restrict__ start, Ctl* ctl) {
+  const uint32_t total = gp->total, base = blockIdx.x * kTile, ntiles = (total + kTile - 1) / kTile;
   if (base >= total) return;
   uint32_t sum = 0;
   for (uint32_t i = base + threadIdx.x; i < min(base + kTile, total); i += kTileThreads) sum += counts[i];
-  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  sum = __reduce_add_sync(0xffffffffu, sum);
   __shared__ uint32_t ws[kTileThreads / 32];
+  __shared__ bool last;
   if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = sum;
   __syncthreads();
   if (threadIdx.x == 0) {
     uint32_t t = 0;
     for (int w = 0; w < kTileThreads / 32; ++w) t += ws[w];
     partial[blockIdx.x] = t;
+    __threadfence();
+    last = atomicAdd(&ctl->scan_done, 1u) == ntiles - 1;
   }
-}
-
-__global__ void ks_scan_top(uint32_t* __restrict__ partial, const GridBox* __restrict__ gp,
-                            uint32_t* __restrict__ start) {
-  const uint32_t total = gp->total, ntiles = (total + kTile - 1) / kTile;
-  __shared__ uint32_t sh[kMaxTiles];
-  const uint32_t t = threadIdx.x;
-  const uint32_t v = t < ntiles ? partial[t] : 0u;
-  sh[t] = v;
   __syncthreads();
-  for (uint32_t off = 1; off < kMaxTiles; off <<= 1) {
-    const uint32_t add = t >= off ? sh[t - off] : 0u;
-    __syncthreads();
-    sh[t] += add;
-    __syncthreads();
+  if (!last) return;
+  __threadfence();
+  static_assert(kTileThreads >= (int)kMaxTiles, "a thread per tile");
+  const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const uint32_t v = t < ntiles ? __ldcg(partial + t) : 0u;
+  uint32_t incl = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+    if ((int)lane >= off) incl += y;
   }
-  if (t < ntiles) partial[t] = sh[t] - v;
-  if (t == kMaxTiles - 1) start[total] = sh[kMaxTiles - 1];
+  __syncthreads();
+  if (lane == 31) ws[w] = incl;
+  __syncthreads();
+  for (uint32_t k = 0; k < w; ++k) incl += ws[k];
+  if (t < ntiles) partial[t] = incl - v;
+  if (t == kTileThreads - 1) {
+    start[total] = incl;
+    ctl->scan_done = 0u;
+  }
 }
 
 __global__ void ks_scan_final(const uint32_t* __restrict__ counts, const GridBox* __restrict__ gp,
-                              const uint32_t* __restrict__ partial, uint32_t* __restrict__ start) {
+                              const uint32_t* __restrict__ partial, uint32_t* __restrict__ start, Ctl* ctl) {
   const uint32_t total = gp->total, base = blockIdx.x * kTile;
   if (base >= total) return;
   constexpr int kPer = kTile / kTileThreads;
@@ -178,6 +225,7 @@ __global__ void ks_scan_final(const uint32_t* __restrict__ counts, const GridBox
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
     if ((i0 + q) < total) start[i0 + q] = run;
+    if (v[q] > kWideRank) ctl->wide[atomicAdd(&ctl->nwide, 1u)] = i0 + q;  // any order: a block each
     run += v[q];
   }
 }
@@ -190,51 +238,39 @@ __global__ void ks_place(const uint2* __restrict__ cellrank, const uint32_t* __r
   tmp[start[cr.x] + cr.y] = i;
 }
 
-// One warp per cell of at most 32 entries: the placed indices of the cell, in ascending
-// order, into items (each lane ranks its entry against the others).
-__global__ void ks_canon(const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ start,
-                         const GridBox* __restrict__ gp, uint32_t* __restrict__ items) {
-  const uint32_t total = gp->total;
-  const int lane = threadIdx.x & 31;
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < total; c += warps) {
-    const uint32_t b = start[c], n = start[c + 1] - b;
-    if (n > 32) continue;  // ks_canon_wide
-    const uint32_t key = lane < (int)n ? tmp[b + lane] : 0xffffffffu;
-    uint32_t rank = 0;
-    for (uint32_t j = 0; j < n; ++j) rank += __shfl_sync(0xffffffffu, key, (int)j) < key ? 1u : 0u;
-    if (lane < (int)n) items[b + rank] = key;
+// The placed indices of each cell of at most kWideRank entries in ascending order, into
+// items: a thread per entry ranks it against its cell's entries (the lanes of a cell read the
+// same ones). A warp per cell, and a pass of blocks over all cells for those above 32 entries,
+// took most of a call's 182 us at 430k particles; it takes 79 now (62 -> 54 at 125: launches).
+__global__ void __launch_bounds__(256) ks_canon(const uint32_t* __restrict__ tmp, const uint2* __restrict__ cellrank,
+                                                const uint32_t* __restrict__ start, uint32_t n,
+                                                uint32_t* __restrict__ items) {
+  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const uint32_t key = tmp[e], c = cellrank[key].x;
+  const uint32_t b = start[c], end = start[c + 1];
+  if (end - b > kWideRank) return;  // ks_canon_wide
+  uint32_t dst = b, j = b;
+  for (; j + 4 <= end; j += 4) {
+    const uint32_t k0 = tmp[j], k1 = tmp[j + 1], k2 = tmp[j + 2], k3 = tmp[j + 3];
+    dst += (k0 < key ? 1u : 0u) + (k1 < key ? 1u : 0u) + (k2 < key ? 1u : 0u) + (k3 < key ? 1u : 0u);
   }
+  for (; j < end; ++j) dst += tmp[j] < key ? 1u : 0u;
+  items[dst] = key;
 }
 
-// Cells of more than 32 entries, one block per cell in turn. Up to kWideRank entries:
-// each thread ranks entries against the cell's keys in shared memory (m^2 / kWideThreads
-// shared reads per thread). More: the cell's indices are distinct values below n, so
-// they are set in a bitmap of n bits in shared memory and read back in ascending order
-// (n / 32 words scanned once, whatever the cell's size).
+// Cells above kWideRank entries, a block per cell in turn: the cell's indices are distinct
+// values below n, so they are set in a bitmap of n bits in shared memory and read back in
+// ascending order (n / 32 words scanned once, whatever the cell's size).
 __global__ void __launch_bounds__(kWideThreads) ks_canon_wide(const uint32_t* __restrict__ tmp,
                                                               const uint32_t* __restrict__ start,
-                                                              const GridBox* __restrict__ gp, uint32_t n,
+                                                              const Ctl* __restrict__ ctl, uint32_t n,
                                                               uint32_t* __restrict__ items) {
   extern __shared__ uint32_t sm[];  // kWideSmemWords
   __shared__ uint32_t s_warp[kWideThreads / 32];
-  const uint32_t total = gp->total;
   const uint32_t t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
-    const uint32_t b = start[c], m = start[c + 1] - b;
-    if (m <= 32) continue;
-    if (m <= kWideRank) {
-      for (uint32_t e = t; e < m; e += kWideThreads) sm[e] = tmp[b + e];
-      __syncthreads();
-      for (uint32_t e = t; e < m; e += kWideThreads) {
-        const uint32_t key = sm[e];
-        uint32_t rank = 0;
-        for (uint32_t j = 0; j < m; ++j) rank += sm[j] < key ? 1u : 0u;
-        items[b + rank] = key;
-      }
-      __syncthreads();
-      continue;
-    }
+  for (uint32_t q = blockIdx.x; q < ctl->nwide; q += gridDim.x) {
+    const uint32_t c = ctl->wide[q], b = start[c], m = start[c + 1] - b;
     const uint32_t words = (n + 31) / 32;
     for (uint32_t w = t; w < words; w += kWideThreads) sm[w] = 0;
     __syncthreads();
@@ -314,23 +350,17 @@ extern "C" vxl_status vxl_sph_build_grid_static(const float* d_pos_xyz, uint32_t
   uint2* cellrank = (uint2*)(base + kRankOff);
   uint32_t* tmp = (uint32_t*)(base + kTmpOff);
   uint32_t* partial = (uint32_t*)(base + kPartialOff);
-  uint32_t* box = (uint32_t*)(base + kBoxOff);
   GridBox* g = (GridBox*)(base + kGridOff);
+  Ctl* ctl = (Ctl*)(base + kCtlOff);
   const uint32_t nblk = (n + 255) / 256, tiles = (budget + kTile - 1) / kTile;
-  // the array keeps the previous call's contents: zero the counts and reset the box
-  cudaError_t e = cudaMemsetAsync(counts, 0, ((size_t)budget + 1) * 4, s);
-  if (e != cudaSuccess) return fail(VXL_CUDA_ERROR, std::string("grid build: ") + cudaGetErrorString(e));
-  ks_init<<<1, 32, 0, s>>>(box);
-  ks_bbox<<<nblk, 256, 0, s>>>(d_pos_xyz, n, box);
-  ks_gridbox<<<1, 32, 0, s>>>(box, h, budget, g);
+  ks_box<<<kBoxBlocks, kBoxThreads, 0, s>>>(d_pos_xyz, n, h, budget, tmp, g, counts, ctl);
   ks_keys<<<nblk, 256, 0, s>>>(d_pos_xyz, n, g, counts, cellrank);
-  ks_scan_partial<<<tiles, kTileThreads, 0, s>>>(counts, g, partial);
-  ks_scan_top<<<1, kMaxTiles, 0, s>>>(partial, g, d_start);
-  ks_scan_final<<<tiles, kTileThreads, 0, s>>>(counts, g, partial, d_start);
+  ks_scan_partial<<<tiles, kTileThreads, 0, s>>>(counts, g, partial, d_start, ctl);
+  ks_scan_final<<<tiles, kTileThreads, 0, s>>>(counts, g, partial, d_start, ctl);
   ks_place<<<nblk, 256, 0, s>>>(cellrank, d_start, n, tmp);
-  ks_canon<<<148 * 4, 256, 0, s>>>(tmp, d_start, g, d_items);
-  ks_canon_wide<<<148 * 2, kWideThreads, kWideSmemWords * sizeof(uint32_t), s>>>(tmp, d_start, g, n, d_items);
-  e = cudaGetLastError();
+  ks_canon<<<nblk, 256, 0, s>>>(tmp, cellrank, d_start, n, d_items);
+  ks_canon_wide<<<32, kWideThreads, kWideSmemWords * sizeof(uint32_t), s>>>(tmp, d_start, ctl, n, d_items);
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(VXL_CUDA_ERROR, std::string("grid build launch: ") + cudaGetErrorString(e));
   GridBox hg;
   e = cudaMemcpyAsync(&hg, g, sizeof(GridBox), cudaMemcpyDeviceToHost, s);

@@ -15,3 +15,36 @@ def test_cells_of_every_size_sort(vxl, oracle_mod, sizes):
     pos = np.concatenate([rng.uniform(0.01, 0.09, (n, 3)) + (0.2 * k, 0.0, 0.1 * (k % 2)) for k, n in enumerate(sizes)])
     pos = pos[rng.permutation(len(pos))].astype(F32)
     _run_both(vxl, oracle_mod, _custom(vxl, pos, h=0.1), substeps=3)
+
+
+def _static(vxl, pos, h, max_bins):
+    import ctypes as C
+    import torch
+    n = pos.shape[0]
+    d_pos = torch.from_numpy(np.ascontiguousarray(pos, F32)).cuda()
+    items = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    start = torch.full((max_bins + 1,), -1, dtype=torch.int32, device="cuda")
+    info = vxl.GridInfo()
+    info.hdr = vxl.header(vxl.GridInfo)
+    st = vxl.load().vxl_sph_build_grid_static(C.c_void_p(d_pos.data_ptr()), n, h, max_bins, C.c_void_p(items.data_ptr()),
+                                              C.c_void_p(start.data_ptr()), max_bins + 1, C.byref(info),
+                                              C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert st == vxl.OK
+    return items.cpu().numpy().view(np.uint32), start[: int(info.total) + 1].cpu().numpy().view(np.uint32), info
+
+
+@pytest.mark.parametrize("n,cells", [(1, 1), (31, 3), (257, 2), (2048, 1), (2049, 1), (4100, 2), (70000, 30), (100000, 20)])
+def test_static_grid_over_cell_sizes(vxl, oracle_mod, n, cells):
+    """The allocation-free table around the ranking limit (2,048 entries a cell; larger ones by bitmap), called
+    twice so that the second starts from the first's leftovers, against the oracle's table."""
+    rng = np.random.default_rng(n)
+    pos = rng.uniform(0.0, 0.09, (n, 3))
+    pos[:, 0] += 0.1 * rng.integers(0, cells, n)
+    pos[0] = 0.0
+    if n > 2:
+        pos[1] = np.nan  # never in the box; binned into the first cell
+    pos = pos.astype(F32)
+    ref_start, ref_items, _ = oracle_mod.rebuild_grid(pos, 0.1, 4096)
+    for _ in range(2):
+        items, start, info = _static(vxl, pos, 0.1, 4096)
+        assert np.array_equal(start, ref_start) and np.array_equal(items, ref_items), (n, cells)
