@@ -58,7 +58,7 @@ def algorithmic_bytes(kernel: str, nf: int, nb: int, cells: int) -> float | None
         "k_canon": 72.0 * nt,
         "k_density": 24.0 * nt,
         "k_force": 72.0 * nf + 40.0 * nb,
-        "k_scan_final": 8.0 * cells,
+        "k_scan": 8.0 * cells,
     }.get(kernel)
 
 

@@ -46,12 +46,12 @@ inline uint32_t team_lanes(uint64_t n, const TeamLimits& t) { return n <= t.eigh
 inline uint32_t blocks_for(uint64_t n, int t = kThreads) { return (uint32_t)((n + t - 1) / t); }
 
 enum KernelId : int {
-  KID_CELLOFF, KID_KEYS, KID_SCAN_PARTIAL, KID_SCAN_FINAL, KID_PLACE, KID_CANON,
+  KID_CELLOFF, KID_KEYS, KID_SCAN, KID_PLACE, KID_CANON,
   KID_DENSITY, KID_FORCE, KID_BFORCE, KID_REACT_LONG, KID_REACT_SPANS, KID_SCALE, KID_WALLS,
   KID_GROUPS, KID_COUNT
 };
 const char* const kKernelNames[KID_COUNT] = {
-    "k_celloff", "k_keys", "k_scan_partial", "k_scan_final", "k_place", "k_canon",
+    "k_celloff", "k_keys", "k_scan", "k_place", "k_canon",
     "k_density", "k_force", "k_bforce", "k_react_long", "k_react_spans", "k_scale", "k_walls",
     "k_groups"};
 
@@ -190,7 +190,7 @@ vxl_status Engine::alloc_all() {
   A(dalloc(&wet_, cell_cap_ + 1));
   A(dalloc(&order_, slot_cap_));
   A(dalloc(&start_, cell_cap_ + 1));
-  A(dalloc(&partial_, cell_cap_ / kScanTile + 2));
+  A(dalloc(&scan_, cell_cap_ / kScanTile + 2));
   A(dalloc(&sc_d_, scene_cap_));
   tiles_cap_ = (uint32_t)(n / 64 + 2ull * scene_cap_ + 2);  // particle tiles (>= 128 slots) + boundary tiles
   A(dalloc(&tiles_d_, tiles_cap_));
@@ -203,6 +203,7 @@ vxl_status Engine::alloc_all() {
   CU(cudaMemsetAsync(counts_, 0, (cell_cap_ + 1) * 4, stream_));
   CU(cudaMemsetAsync(wet_, 0, (cell_cap_ + 1) * 4, stream_));
   CU(cudaMemsetAsync(start_, 0, (cell_cap_ + 1) * 4, stream_));
+  CU(cudaMemsetAsync(scan_, 0, (cell_cap_ / kScanTile + 2) * sizeof(*scan_), stream_));
   CU(cudaMemsetAsync(ctl_d_, 0, sizeof(EngineCtl), stream_));
   CU(cudaMemsetAsync(sc_d_, 0, scene_cap_ * sizeof(SceneDev), stream_));
   CU(cudaMemsetAsync(acc_, 0, n * 16, stream_));
@@ -218,7 +219,7 @@ void Engine::free_all() {
   if (graph_) cudaGraphExecDestroy(graph_);
   graph_ = nullptr;
   void* d[] = {pos_[0], pos_[1], vel_[0], vel_[1], orig_, slot_of_, cellrank_, items_, rc_, press_, acc_, xsph_,
-               bforce_, bpos_, nbr_, nbr_n_, words_, bwet_, order_, stage_, counts_, wet_, start_, partial_, sc_d_, tiles_d_, ctl_d_, spans_d_,
+               bforce_, bpos_, nbr_, nbr_n_, words_, bwet_, order_, stage_, counts_, wet_, start_, scan_, sc_d_, tiles_d_, ctl_d_, spans_d_,
                longs_d_, breact_d_};
   for (void* p : d)
     if (p) cudaFree(p);
@@ -365,15 +366,10 @@ vxl_status Engine::push_scene_records(const std::vector<float>& dt) {
 }
 
 vxl_status Engine::recompute_scene_boxes(uint32_t q) {
-  static const uint32_t init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
   const SceneInfo& si = scenes_[q];
   const uint32_t n = si.nf + si.nb;
-  CU(cudaMemcpyAsync(sc_d_[q].fbox, init, sizeof(init), cudaMemcpyHostToDevice, stream_));
-  CU(cudaMemcpyAsync(sc_d_[q].bbox, init, sizeof(init), cudaMemcpyHostToDevice, stream_));
-  if (n) {
-    k_e_bbox<<<blocks_for(n), kThreads, 0, stream_>>>((const float4*)pos_[0], si.base, n, 1, sc_d_[q].fbox);
-    k_e_bbox<<<blocks_for(n), kThreads, 0, stream_>>>((const float4*)pos_[0], si.base, n, 0, sc_d_[q].bbox);
-  }
+  k_e_box_empty<<<1, 32, 0, stream_>>>(sc_d_ + q, 1, 1);
+  if (n) k_e_bbox<<<blocks_for(n), kThreads, 0, stream_>>>((const float4*)pos_[0], si.base, n, sc_d_ + q);
   CU(cudaGetLastError());
   CU(cudaStreamSynchronize(stream_));
   return VXL_OK;
@@ -538,10 +534,9 @@ vxl_status Engine::upload_boundary(uint32_t q, const float* pos, const float* ve
   if (nb == 0) return VXL_OK;
   if (!pos || !vel) return set_error(VXL_NULL_POINTER, "pos/vel is NULL");
   CU(cudaSetDevice(device_));
-  static const uint32_t init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
   CU(cudaMemcpyAsync(stage_, pos, nb * 12, cudaMemcpyHostToDevice, stream_));
   CU(cudaMemcpyAsync(stage_ + 3 * nb, vel, nb * 12, cudaMemcpyHostToDevice, stream_));
-  CU(cudaMemcpyAsync(sc_d_[q].bbox, init, sizeof(init), cudaMemcpyHostToDevice, stream_));
+  k_e_box_empty<<<1, 32, 0, stream_>>>(sc_d_ + q, 0, 1);
   k_e_upload_boundary<<<blocks_for(nb), kThreads, 0, stream_>>>(stage_, stage_ + 3 * nb, (float4*)pos_[0],
                                                                  (float4*)vel_[0], slot_of_, (float4*)bpos_,
                                                                  sc_d_[q].bbox, si.base, si.nf, si.nb);
@@ -686,11 +681,10 @@ vxl_status Engine::step_coupled_async(float dt_tick, uint32_t rigid_substeps, co
                                                            dt, rigid_substeps, max_linear, max_angular);
   CU(cudaGetLastError());
   // 2. boundary segments from the new poses
-  static const uint32_t init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
   for (uint32_t q = 0; q < scenes_.size(); ++q) {
     if (q >= rigid_.size() || rigid_[q].empty() || scenes_[q].nb == 0) continue;
     const SceneInfo& si = scenes_[q];
-    CU(cudaMemcpyAsync(sc_d_[q].bbox, init, sizeof(init), cudaMemcpyHostToDevice, stream_));
+    k_e_box_empty<<<1, 32, 0, stream_>>>(sc_d_ + q, 0, 1);
     k_e_body_rebuild<<<blocks_for(si.nb), kThreads, 0, stream_>>>(blocal_, rb_d_ + rb_off_[q], (float4*)pos_[0],
                                                                    (float4*)vel_[0], slot_of_, (float4*)bpos_,
                                                                    sc_d_[q].bbox, si.base, si.nf, si.nb);
@@ -999,9 +993,8 @@ vxl_status Engine::set_body_poses(uint32_t q, const vxl_sph_body_pose* poses, ui
     h[b] = BodyPoseDev{p.pos[0], p.pos[1], p.pos[2], p.rot[0], p.rot[1], p.rot[2], p.rot[3],
                        p.linvel[0], p.linvel[1], p.linvel[2], p.angvel[0], p.angvel[1], p.angvel[2]};
   }
-  static const uint32_t init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
   CU(cudaMemcpyAsync(poses_d_, h.data(), nbodies * sizeof(BodyPoseDev), cudaMemcpyHostToDevice, stream_));
-  CU(cudaMemcpyAsync(sc_d_[q].bbox, init, sizeof(init), cudaMemcpyHostToDevice, stream_));
+  k_e_box_empty<<<1, 32, 0, stream_>>>(sc_d_ + q, 0, 1);
   k_e_body_rebuild<<<blocks_for(si.nb), kThreads, 0, stream_>>>(blocal_, poses_d_, (float4*)pos_[0],
                                                                  (float4*)vel_[0], slot_of_, (float4*)bpos_,
                                                                  sc_d_[q].bbox, si.base, si.nf, si.nb);
@@ -1441,11 +1434,10 @@ void Engine::enqueue_substep(bool with_reactions) {
   // grids, cell table, sorted buffer, permutation, lists, work counters): join it first.
   // Its reaction sums read only bforce / bpos and go on beside this substep.
   join_side_only();
-  LAUNCH(KID_CELLOFF, k_e_celloff<<<1, 1024, 0, st>>>(sc_d_, S, ctl_d_, (uint32_t)cell_cap_));
+  LAUNCH(KID_CELLOFF, k_e_celloff<<<1, S <= 32 ? 32 : kCelloffThreads, 0, st>>>(sc_d_, S, ctl_d_, (uint32_t)cell_cap_));
   LAUNCH(KID_KEYS, k_e_keys<<<key_blocks, kThreads, 0, st>>>(p0, sc_d_, tiles_d_, ntiles_, ctl_d_, counts_,
                                                              (uint2*)cellrank_, wet_));
-  LAUNCH(KID_SCAN_PARTIAL, k_e_scan_partial<<<148 * 4, kScanThreads, 0, st>>>(counts_, ctl_d_, partial_, start_));
-  LAUNCH(KID_SCAN_FINAL, k_e_scan_final<<<148 * 4, kScanThreads, 0, st>>>(counts_, ctl_d_, partial_, start_));
+  LAUNCH(KID_SCAN, k_e_scan<<<148 * 4, kScanThreads, 0, st>>>(counts_, ctl_d_, scan_, start_));
   LAUNCH(KID_PLACE, k_e_place<<<key_blocks, kThreads, 0, st>>>((const uint2*)cellrank_, start_, orig_, tiles_d_,
                                                                ntiles_, ctl_d_, (uint2*)items_, order_));
   LAUNCH(KID_CANON, k_e_canon<<<std::max<uint32_t>(blocks_for(used_), 1), 256, 0, st>>>(
@@ -1645,6 +1637,7 @@ vxl_status Engine::finish() {
   prof_collect();
   if (ctl_h_->err & kErrGridLoop) return set_error(VXL_DEVICE_FAULT_FLAG, "grid box doubling loop did not settle");
   if (ctl_h_->err & kErrCellCap) {
+    const bool wait = (ctl_h_->err & kErrScanWait) != 0u;
     ctl_h_->err = 0;
     cudaMemsetAsync(&ctl_d_->err, 0, 4, stream_);
     // the skipped substeps left the state as it was but emptied the fluid AABB
@@ -1655,7 +1648,8 @@ vxl_status Engine::finish() {
     }
     cudaStreamSynchronize(stream_);
     return set_error(VXL_DEVICE_FAULT_FLAG,
-                     "the scenes' cells exceed the engine's cell capacity; the tick was skipped, state unchanged");
+                     wait ? "a wait of the cell scan ran out; the rest of the tick was skipped"
+                          : "the scenes' cells exceed the engine's cell capacity; the tick was skipped, state unchanged");
   }
   return VXL_OK;
 }

@@ -48,6 +48,7 @@
 namespace vxl {
 
 constexpr uint32_t kErrCellCap = 1u << 3;  // the scenes' cells exceed the cell capacity
+constexpr uint32_t kErrScanWait = 1u << 4;  // the scan's wait ran out (with kErrCellCap: the substep is skipped)
 
 // Per-scene device record (one per scene of the engine). The fields up to `g` are
 // written by the host (constants, substep dt, slot range); the rest by the kernels.
@@ -317,17 +318,20 @@ __global__ void k_e_upload_boundary(const float* __restrict__ pin, const float* 
   block_bbox_accumulate(bbox_acc, x, y, z, valid);
 }
 
-// AABB of one scene's fluid (pos.w > 0) or boundary (pos.w < 0) slots into acc.
-__global__ void k_e_bbox(const float4* __restrict__ pos, uint32_t base, uint32_t n, int want_fluid,
-                         uint32_t* __restrict__ acc) {
+// AABBs of one scene's fluid (pos.w > 0) and boundary (pos.w < 0) slots into its (emptied)
+// accumulators.
+__global__ void k_e_bbox(const float4* __restrict__ pos, uint32_t base, uint32_t n, SceneDev* __restrict__ S) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   float4 p = make_float4(0, 0, 0, 0);
-  bool valid = false;
-  if (i < n) {
-    p = pos[base + i];
-    valid = want_fluid ? (p.w > 0.0f) : (p.w < 0.0f);
-  }
-  block_bbox_accumulate(acc, p.x, p.y, p.z, valid);
+  if (i < n) p = pos[base + i];
+  if (__syncthreads_or(p.w > 0.0f)) block_bbox_accumulate(S->fbox, p.x, p.y, p.z, p.w > 0.0f);
+  if (__syncthreads_or(p.w < 0.0f)) block_bbox_accumulate(S->bbox, p.x, p.y, p.z, p.w < 0.0f);
+}
+
+__global__ void k_e_box_empty(SceneDev* __restrict__ S, int fluid, int boundary) {
+  const uint32_t a = threadIdx.x;
+  if (a < 6 && fluid) S->fbox[a] = a < 3 ? 0xffffffffu : 0u;
+  if (a < 6 && boundary) S->bbox[a] = a < 3 ? 0xffffffffu : 0u;
 }
 
 // Move whole scenes to new bases (the served form's repack): slot ranges are copied into
@@ -412,14 +416,16 @@ __global__ void k_e_slot_of(const uint32_t* __restrict__ orig, uint32_t* __restr
 // exclusive scan of the scenes' cell counts;
 // flags the substep when the total exceeds the cell capacity (every later kernel then
 // returns without touching memory).
-__global__ void k_e_celloff(SceneDev* __restrict__ sc, uint32_t nscenes, EngineCtl* ctl, uint32_t cell_cap) {
-  __shared__ uint32_t sh[1024];
-  __shared__ unsigned long long carry;
-  if (threadIdx.x == 0) carry = 0;
-  if (threadIdx.x < kWorkSlots) ctl->work[threadIdx.x] = 0;  // persistent-pass counters of this substep
+// A warp for up to 32 scenes, kCelloffThreads threads for more.
+constexpr uint32_t kCelloffThreads = 1024;
+__global__ void __launch_bounds__(kCelloffThreads) k_e_celloff(SceneDev* __restrict__ sc, uint32_t nscenes,
+                                                               EngineCtl* ctl, uint32_t cell_cap) {
+  __shared__ uint32_t ws[32];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  unsigned long long carry = 0;  // the same in every thread
+  if (threadIdx.x < kWorkSlots) ctl->work[threadIdx.x] = 0;  // work counters of this substep
   if (threadIdx.x == 0) ctl->epoch = ctl->epoch + 1u;
-  __syncthreads();
-  for (uint32_t b0 = 0; b0 < nscenes; b0 += 1024) {
+  for (uint32_t b0 = 0; b0 < nscenes; b0 += blockDim.x) {
     const uint32_t q = b0 + threadIdx.x;
     uint32_t v = 0;
     if (q < nscenes) {
@@ -442,18 +448,23 @@ __global__ void k_e_celloff(SceneDev* __restrict__ sc, uint32_t nscenes, EngineC
       }
       v = g.total;
     }
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (uint32_t off = 1; off < 1024; off <<= 1) {
-      const uint32_t add = threadIdx.x >= off ? sh[threadIdx.x - off] : 0u;
-      __syncthreads();
-      sh[threadIdx.x] += add;
-      __syncthreads();
+    // exclusive scan of the scenes' cells (at most 2^21 each: a block's sum fits 32 bits)
+    uint32_t incl = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+      if ((int)lane >= off) incl += y;
     }
-    const unsigned long long ex = carry + (unsigned long long)(sh[threadIdx.x] - v);
-    if (q < nscenes) sc[q].cell_off = ex > 0xffffffffull ? 0xffffffffu : (uint32_t)ex;
+    if (lane == 31) ws[w] = incl;
     __syncthreads();
-    if (threadIdx.x == 1023) carry += sh[1023];
+    uint32_t before = 0, total = 0;
+    for (uint32_t k = 0; k < warps; ++k) {
+      if (k < w) before += ws[k];
+      total += ws[k];
+    }
+    const unsigned long long ex = carry + before + (incl - v);
+    if (q < nscenes) sc[q].cell_off = ex > 0xffffffffull ? 0xffffffffu : (uint32_t)ex;
+    carry += total;
     __syncthreads();
   }
   if (threadIdx.x == 0) {
@@ -501,68 +512,32 @@ __global__ void k_e_keys(const float4* __restrict__ pos, const SceneDev* __restr
   }
 }
 
-// Phases 1-2 of the scan: per-tile sums of the counts (tiles of kScanTile cells,
-// grid-stride), then, in whichever block finishes last (an atomic count of finished blocks;
-// nothing waits), the exclusive scan of the tile sums in place and the total into
-// start[cells].
-__global__ void k_e_scan_partial(const uint32_t* __restrict__ counts, EngineCtl* ctl,
-                                 uint32_t* __restrict__ partial, uint32_t* __restrict__ start) {
+// Exclusive scan of the counts into start, in one pass; the counts are zeroed for the next
+// substep. Blocks draw tiles of kScanTile cells in order from an atomic counter; a tile's block publishes
+// the tile's sum, then looks back over its predecessors, 32 at a time, adding sums until it meets
+// one whose whole prefix is known, and publishes its own. A published word is (epoch, kind,
+// value) in 64 bits, so words of earlier substeps read as unpublished. Every tile looked at
+// was drawn earlier by a block that publishes without waiting, so the wait ends; it has a limit
+// all the same, after which the substep is flagged like a cell overflow (the later
+// kernels touch nothing). In two launches (tile sums, then tiles) the scan took 8 us of a
+// small scene's substep; SCAN_FIGURES.
+constexpr uint32_t kScanSum = 1u, kScanPrefix = 2u;
+constexpr uint32_t kScanWait = 1u << 22;
+__global__ void __launch_bounds__(kScanThreads) k_e_scan(uint32_t* __restrict__ counts, EngineCtl* ctl,
+                                                         unsigned long long* state, uint32_t* __restrict__ start) {
   if (ctl->err & kErrCellCap) return;
   const uint32_t total = ctl->cells;
-  __shared__ uint32_t ws[kScanThreads / 32];
-  for (uint32_t tile = blockIdx.x; (size_t)tile * kScanTile < total; tile += gridDim.x) {
-    const uint32_t base = tile * kScanTile;
-    uint32_t sum = 0;
-    for (uint32_t i = base + threadIdx.x; i < min(base + kScanTile, total); i += kScanThreads) sum += counts[i];
-    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      uint32_t t = 0;
-      for (int w = 0; w < kScanThreads / 32; ++w) t += ws[w];
-      partial[tile] = t;
-    }
-    __syncthreads();
-  }
-  __shared__ uint32_t last;
-  if (threadIdx.x == 0) {
-    __threadfence();  // this block's tile sums are visible before it counts itself done
-    last = atomicAdd(&ctl->work[kWorkScan], 1u) == gridDim.x - 1 ? 1u : 0u;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
   const uint32_t ntiles = (total + kScanTile - 1) / kScanTile;
-  __shared__ uint32_t sh[kScanThreads];
-  __shared__ uint32_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (uint32_t b0 = 0; b0 < ntiles; b0 += kScanThreads) {
-    const uint32_t t = b0 + threadIdx.x;
-    const uint32_t v = t < ntiles ? __ldcg(partial + t) : 0u;  // written by other blocks: skip L1
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (uint32_t off = 1; off < kScanThreads; off <<= 1) {
-      const uint32_t add = threadIdx.x >= off ? sh[threadIdx.x - off] : 0u;
-      __syncthreads();
-      sh[threadIdx.x] += add;
-      __syncthreads();
-    }
-    if (t < ntiles) partial[t] = carry + sh[threadIdx.x] - v;
-    __syncthreads();
-    if (threadIdx.x == kScanThreads - 1) carry += sh[kScanThreads - 1];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) start[total] = carry;
-}
-// Phase 3: per-tile exclusive scan + tile offset -> start; zero counts for the next substep.
-__global__ void k_e_scan_final(uint32_t* __restrict__ counts, const EngineCtl* __restrict__ ctl,
-                               const uint32_t* __restrict__ partial, uint32_t* __restrict__ start) {
-  if (ctl->err & kErrCellCap) return;
-  const uint32_t total = ctl->cells;
+  const uint32_t tag = ctl->epoch << 2;  // upper half of this substep's words: tag | kind
   constexpr int kPer = kScanTile / kScanThreads;
-  __shared__ uint32_t ws[kScanThreads / 32];
-  for (uint32_t tile = blockIdx.x; (size_t)tile * kScanTile < total; tile += gridDim.x) {
+  __shared__ uint32_t ws[kScanThreads / 32], s_prefix;
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  volatile unsigned long long* vs = state;
+  if (total == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) start[0] = 0u;
+    return;
+  }
+  for (uint32_t tile = next_tile(&ctl->work[kWorkScan]); tile < ntiles; tile = next_tile(&ctl->work[kWorkScan])) {
     const uint32_t i0 = tile * kScanTile + threadIdx.x * kPer;
     uint32_t v[kPer], local = 0;
 #pragma unroll
@@ -571,17 +546,52 @@ __global__ void k_e_scan_final(uint32_t* __restrict__ counts, const EngineCtl* _
       local += v[q];
     }
     uint32_t incl = local;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
       const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += y;
+      if ((int)lane >= off) incl += y;
     }
-    if (lane == 31) ws[wid] = incl;
+    if (lane == 31) ws[w] = incl;
     __syncthreads();
-    uint32_t woff = 0;
-    for (int w = 0; w < wid; ++w) woff += ws[w];
-    uint32_t run = partial[tile] + woff + incl - local;
+    uint32_t before = 0, sum = 0;
+    for (uint32_t k = 0; k < kScanThreads / 32; ++k) {
+      if (k < w) before += ws[k];
+      sum += ws[k];
+    }
+    if (w == 0) {
+      if (lane == 0)
+        vs[tile] = ((unsigned long long)(tag | (tile == 0 ? kScanPrefix : kScanSum)) << 32) | sum;
+      uint32_t prefix = 0;
+      for (uint32_t at = tile; at > 0;) {  // look back over tiles at - 32 .. at - 1, lane 0 the nearest
+        const bool in = lane < at;
+        uint32_t kind = in ? 0u : kScanPrefix, val = 0;  // before the first tile: a known prefix of 0
+        for (uint32_t tries = 0; !__all_sync(0xffffffffu, kind != 0u); ++tries) {
+          if (kind == 0u) {
+            const unsigned long long word = vs[at - 1 - lane];
+            if ((uint32_t)(word >> 34) == tag >> 2) {
+              kind = (uint32_t)(word >> 32) & 3u;
+              val = (uint32_t)word;
+            }
+          }
+          if (tries == kScanWait) {
+            if (kind == 0u) {
+              atomicOr(&ctl->err, kErrCellCap | kErrScanWait);
+              kind = kScanPrefix;
+            }
+          }
+        }
+        const uint32_t known = __ballot_sync(0xffffffffu, kind == kScanPrefix);
+        const uint32_t last = known ? (uint32_t)__ffs(known) - 1u : 31u;  // add up to the nearest known prefix
+        prefix += __reduce_add_sync(0xffffffffu, lane <= last ? val : 0u);
+        at = known ? 0u : at - 32u;
+      }
+      if (lane == 0) {
+        if (tile) vs[tile] = ((unsigned long long)(tag | kScanPrefix) << 32) | (prefix + sum);
+        s_prefix = prefix;
+      }
+    }
+    __syncthreads();
+    uint32_t run = s_prefix + before + incl - local;
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
       if ((i0 + q) < total) {
@@ -590,7 +600,7 @@ __global__ void k_e_scan_final(uint32_t* __restrict__ counts, const EngineCtl* _
       }
       run += v[q];
     }
-    __syncthreads();
+    if (tile == ntiles - 1 && threadIdx.x == kScanThreads - 1) start[total] = run;
   }
 }
 

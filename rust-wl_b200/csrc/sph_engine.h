@@ -236,7 +236,7 @@ class Engine {
   uint32_t* counts_ = nullptr;
   uint32_t* wet_ = nullptr;  // per cell: the substep epoch of the last substep it held fluid
   uint32_t* start_ = nullptr;
-  uint32_t* partial_ = nullptr;
+  unsigned long long* scan_ = nullptr;  // k_e_scan: a word per tile
   // scenes / tiles / control
   SceneDev* sc_d_ = nullptr;
   SceneDev* sc_h_ = nullptr;  // pinned mirror (pushed when dt or membership changes)
