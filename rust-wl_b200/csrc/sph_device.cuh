@@ -86,11 +86,12 @@ __device__ __forceinline__ uint32_t cell_slot(const GridBox& g, float x, float y
 // - 32, q.z - 64 dz - 32), and |b - A|^2 = 2 (|b|^2 / 2 - A.b) + |A|^2: with M = (-A, 45) as signed
 // bytes, one four-way byte dot product per candidate, word . M <= |b|^2 / 2 - A.b, decides
 // |b - A|^2 <= T conservatively. A slot the filter drops is farther than sqrt(T); one it keeps is
-// tested exactly. T = (64 h / bin + 2.5)^2: flooring two positions moves their difference by
-// less than 1 per axis (sqrt(3) in all), and the f32 rounding of (v - o) * inv by at most 0.19
-// per axis and particle at the largest grid (16,384 cells of 64). Positions outside the grid's
-// cells are clamped into the last one, which never moves two particles apart, so the filter
-// stays conservative there.
+// tested exactly. T = (64 h / bin + 1.75 + 4.2e-5 n)^2, n the longest axis in cells: flooring
+// two positions moves their difference by less than 1 per axis (sqrt(3) = 1.733 in all), and the
+// f32 rounding of (v - o) * inv (three roundings) by at most 64 n 3 2^-24 = 1.15e-5 n per axis
+// and particle (2 sqrt(3) times that in all); the rest covers the rounding of r2 and of T's own
+// terms. Positions outside the grid's cells are clamped into the last one, which never moves
+// two particles apart, so the filter stays conservative there.
 constexpr uint32_t kSubUnits = 64;
 constexpr uint32_t kSubNorm = 45;  // |b|^2 / 2 is kept in multiples of this
 
@@ -193,7 +194,7 @@ __device__ inline bool grid_box(float lox, float loy, float loz, float hix, floa
   g.ny = dims[1];
   g.nz = dims[2];
   g.total = dims[0] * dims[1] * dims[2];
-  const float reach = (float)kSubUnits * (h / bin) + 2.5f;  // at most 66.5: bin >= h
+  const float reach = (float)kSubUnits * (h / bin) + (1.75f + 4.2e-5f * (float)max(dims[0], max(dims[1], dims[2])));
   g.reach_q = (uint32_t)ceilf(reach * reach);
   return ok;
 }

@@ -30,7 +30,7 @@ def _kept(pos, i, j, h, lo, bin_, dims):
     assert norm.max() <= 127 and max(np.abs(x).max() for x in b) <= 128
     A = [q[0][i] - 32, q[1][i] - 64 * d[1] - 32, q[2][i] - 64 * d[2] - 32]
     assert all(np.abs(a[near]).max(initial=0) <= 127 for a in A)
-    reach = F32(64) * (F32(h) / F32(bin_)) + F32(2.5)
+    reach = F32(64) * (F32(h) / F32(bin_)) + (F32(1.75) + F32(4.2e-5) * F32(max(dims)))
     T = int(np.ceil(reach * reach))
     AA = A[0] ** 2 + A[1] ** 2 + A[2] ** 2
     over = -((T - AA) >> 1) - 1
