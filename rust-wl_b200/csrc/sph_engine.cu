@@ -1151,11 +1151,9 @@ vxl_status Engine::export_grid(uint32_t q, uint32_t* items, uint32_t* start, uin
   }
   if (start && start_cap < total + 1) return set_error(VXL_SIZE_MISMATCH, "start buffer smaller than cells + 1");
   if (!start && !(items && n) && !(bins && n)) return VXL_OK;
-  uint32_t* ref_start = nullptr;  // the table in the reference's cell order
-  if (cudaMalloc((void**)&ref_start, (total + 1) * 4) != cudaSuccess) {
-    cudaGetLastError();
-    return set_error(VXL_OUT_OF_MEMORY, "no device memory for the exported table");
-  }
+  if ((uint64_t)rec.cell_off + total > cell_cap_)
+    return set_error(VXL_NOT_READY, "no table: the last substep's cells exceeded the capacity and it was skipped");
+  uint32_t* ref_start = counts_;  // the table in the reference's cell order (the counts are zero between substeps)
   uint32_t* d_items = (uint32_t*)stage_;
   uint32_t* d_bins = d_items + n;
   const uint32_t blocks = blocks_for(total + 1);
@@ -1169,8 +1167,9 @@ vxl_status Engine::export_grid(uint32_t q, uint32_t* items, uint32_t* start, uin
     e = cudaMemcpyAsync(start, ref_start, (total + 1) * 4, cudaMemcpyDeviceToHost, stream_);
   if (e == cudaSuccess && items && n) e = cudaMemcpyAsync(items, d_items, (size_t)n * 4, cudaMemcpyDeviceToHost, stream_);
   if (e == cudaSuccess && bins && n) e = cudaMemcpyAsync(bins, d_bins, (size_t)n * 4, cudaMemcpyDeviceToHost, stream_);
+  const cudaError_t z = cudaMemsetAsync(counts_, 0, (total + 1) * 4, stream_);
+  if (e == cudaSuccess) e = z;
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
-  cudaFree(ref_start);
   if (e != cudaSuccess) return set_error(VXL_CUDA_ERROR, std::string("export: ") + cudaGetErrorString(e));
   return VXL_OK;
 }
