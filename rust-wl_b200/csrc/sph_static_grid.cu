@@ -47,8 +47,9 @@ constexpr size_t kCtlOff = align256(kGridOff + sizeof(GridBox));
 constexpr size_t kScratchBytes = align256(kCtlOff + sizeof(uint32_t) * (3 + kMaxWide));
 static_assert(kBoxBlocks * 6 <= kStaticMaxParticles, "the blocks' boxes use the placement's words");
 
-// Control words at kCtlOff: blocks done in ks_box and in ks_scan_partial (both 0 between
-// calls; the array starts zeroed), cells above kWideRank, and their indices.
+// Control words at kCtlOff: blocks done in ks_box and in ks_scan_partial, cells above
+// kWideRank, and their indices. The array starts zeroed; ks_keys, between their users, zeroes
+// the three counts, so that whatever a call left in them lasts no longer than the next.
 struct Ctl {
   uint32_t box_done, scan_done, nwide;
   uint32_t wide[kMaxWide];
@@ -132,14 +133,13 @@ __global__ void __launch_bounds__(kBoxThreads) ks_box(const float* __restrict__ 
     grid_box(o2f(s_box[0][0]), o2f(s_box[1][0]), o2f(s_box[2][0]), o2f(s_box[3][0]), o2f(s_box[4][0]), o2f(s_box[5][0]),
              h, max_bins, gb);
     *g = gb;
-    ctl->box_done = 0u;
-    ctl->nwide = 0u;
   }
 }
 
 __global__ void ks_keys(const float* __restrict__ xyz, uint32_t n, const GridBox* __restrict__ gp,
-                        uint32_t* __restrict__ counts, uint2* __restrict__ cellrank) {
+                        uint32_t* __restrict__ counts, uint2* __restrict__ cellrank, Ctl* ctl) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) ctl->box_done = ctl->scan_done = ctl->nwide = 0u;
   const bool valid = i < n;
   uint32_t c = 0xffffffffu;
   if (valid) c = cell_index(*gp, xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]);
@@ -191,10 +191,7 @@ __global__ void ks_scan_partial(const uint32_t* __restrict__ counts, const GridB
   __syncthreads();
   for (uint32_t k = 0; k < w; ++k) incl += ws[k];
   if (t < ntiles) partial[t] = incl - v;
-  if (t == kTileThreads - 1) {
-    start[total] = incl;
-    ctl->scan_done = 0u;
-  }
+  if (t == kTileThreads - 1) start[total] = incl;
 }
 
 __global__ void ks_scan_final(const uint32_t* __restrict__ counts, const GridBox* __restrict__ gp,
@@ -225,7 +222,10 @@ __global__ void ks_scan_final(const uint32_t* __restrict__ counts, const GridBox
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
     if ((i0 + q) < total) start[i0 + q] = run;
-    if (v[q] > kWideRank) ctl->wide[atomicAdd(&ctl->nwide, 1u)] = i0 + q;  // any order: a block each
+    if (v[q] > kWideRank) {
+      const uint32_t at = atomicAdd(&ctl->nwide, 1u);  // any order: a block each
+      if (at < kMaxWide) ctl->wide[at] = i0 + q;
+    }
     run += v[q];
   }
 }
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kWideThreads) ks_canon_wide(const uint32_t* __
   extern __shared__ uint32_t sm[];  // kWideSmemWords
   __shared__ uint32_t s_warp[kWideThreads / 32];
   const uint32_t t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  for (uint32_t q = blockIdx.x; q < ctl->nwide; q += gridDim.x) {
+  for (uint32_t q = blockIdx.x; q < min(ctl->nwide, kMaxWide); q += gridDim.x) {
     const uint32_t c = ctl->wide[q], b = start[c], m = start[c + 1] - b;
     const uint32_t words = (n + 31) / 32;
     for (uint32_t w = t; w < words; w += kWideThreads) sm[w] = 0;
@@ -354,7 +354,7 @@ extern "C" vxl_status vxl_sph_build_grid_static(const float* d_pos_xyz, uint32_t
   Ctl* ctl = (Ctl*)(base + kCtlOff);
   const uint32_t nblk = (n + 255) / 256, tiles = (budget + kTile - 1) / kTile;
   ks_box<<<kBoxBlocks, kBoxThreads, 0, s>>>(d_pos_xyz, n, h, budget, tmp, g, counts, ctl);
-  ks_keys<<<nblk, 256, 0, s>>>(d_pos_xyz, n, g, counts, cellrank);
+  ks_keys<<<nblk, 256, 0, s>>>(d_pos_xyz, n, g, counts, cellrank, ctl);
   ks_scan_partial<<<tiles, kTileThreads, 0, s>>>(counts, g, partial, d_start, ctl);
   ks_scan_final<<<tiles, kTileThreads, 0, s>>>(counts, g, partial, d_start, ctl);
   ks_place<<<nblk, 256, 0, s>>>(cellrank, d_start, n, tmp);
