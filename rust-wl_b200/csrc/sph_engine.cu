@@ -1542,8 +1542,8 @@ void Engine::enqueue_substep(bool with_reactions) {
     LAUNCH(KID_WALLS, k_e_pushed_emit<<<nblk, kThreads, 0, st>>>(pflag_, nref, pblk_, ctl_d_, plist_,
                                                                  (const float4*)pos_[0], (const float4*)pnsum_, slot_of_,
                                                                  (float4*)ppos_));
-    LAUNCH(KID_WALLS, k_e_separate_check<<<148 * 4, kCheckTile, 0, st>>>(sc_d_, plist_, (const float4*)pnsum_,
-                                                                           (const float4*)ppos_, ctl_d_));
+    LAUNCH(KID_WALLS, k_e_separate_check<<<dim3(kCheckCols, kCheckRows), kCheckTile, 0, st>>>(
+                          sc_d_, plist_, (const float4*)pnsum_, (const float4*)ppos_, ctl_d_));
     LAUNCH(KID_WALLS, k_e_separate<<<1, 1024, 0, st>>>((float4*)pos_[0], sc_d_, S, plist_, (const float4*)pnsum_,
                                                          slot_of_, ctl_d_));
     LAUNCH(KID_WALLS, k_e_wall_rebox<<<key_blocks, kThreads, 0, st>>>((const float4*)pos_[0], sc_d_, tiles_d_,

@@ -1776,12 +1776,18 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* __restrict__
 // separate_coincident (fluid_boundary.rs:103-128) moves a pushed particle only if some
 // earlier pushed particle of its scene lies closer than r_min = 0.2 h. If no pair is that
 // close at the projected positions, nothing moves (by induction over the sequential loop):
-// this pass decides whether the sequential pass must run. The P (P - 1) / 2 pairs go over
-// the GPU as pairs of tiles of kCheckTile pushed particles (gathered with their scene by
-// k_e_pushed_emit): a thread holds one particle of the later tile and tests it against the
-// earlier tile in shared memory. With one thread per particle and gathers through plist and
-// slot_of it was P dependent loads long (0.15 ms of a 65k-particle tank's 0.31 ms substep).
+// this pass decides whether the sequential pass must run. The pairs of a scene go over the GPU
+// as pairs of tiles of kCheckTile pushed particles (gathered with their scene by k_e_pushed_emit):
+// a thread holds one particle of the later tile (a row) and tests it against an earlier tile in
+// shared memory. blockIdx.y takes rows, up and down in turn so that long and short ones mix;
+// blockIdx.x takes tiles back from the row's own and stops at the first that ends in an earlier
+// scene: the list ascends by scene, so a batch of scenes costs the sum of their pairs, not the
+// pairs of all (wall kernels of a substep of 64 scenes with 2,048 pushed particles each: 91 us,
+// 1.33 ms with all pairs; of one scene 65 us either way). 4 or 16 columns are within 10% of 8. One
+// thread per particle and gathers through plist and slot_of was P dependent loads long (0.15 ms
+// of a 65k-particle tank's 0.31 ms substep).
 constexpr uint32_t kCheckTile = 128;
+constexpr uint32_t kCheckRows = 148, kCheckCols = 8;  // grid: (cols, rows), so that a few rows still spread over the SMs
 __global__ void __launch_bounds__(kCheckTile) k_e_separate_check(const SceneDev* __restrict__ sc,
                                                                  const uint32_t* __restrict__ plist,
                                                                  const float4* __restrict__ pnsum,
@@ -1790,26 +1796,36 @@ __global__ void __launch_bounds__(kCheckTile) k_e_separate_check(const SceneDev*
   if (ctl->err & kErrCellCap) return;
   __shared__ float4 tile[kCheckTile];
   __shared__ uint32_t found;
-  const uint32_t P = ctl->work[kWorkPushed];
-  const unsigned long long nt = (P + kCheckTile - 1) / kCheckTile, npairs = nt * (nt + 1) / 2;
-  unsigned long long row = 0, row0 = 0;  // pair k = row (row + 1) / 2 + col, col <= row
-  for (unsigned long long k = blockIdx.x; k < npairs; k += gridDim.x) {
-    while (row0 + row + 1 <= k) row0 += ++row;
-    const uint32_t a = (uint32_t)row * kCheckTile + threadIdx.x, b0 = (uint32_t)(k - row0) * kCheckTile;
-    __syncthreads();
-    if (b0 + threadIdx.x < P) tile[threadIdx.x] = ppos[b0 + threadIdx.x];
-    if (threadIdx.x == 0) found = *(volatile const uint32_t*)&ctl->work[kWorkTrigger];
-    __syncthreads();
-    if (found) return;
+  const uint32_t P = ctl->work[kWorkPushed], nt = (P + kCheckTile - 1) / kCheckTile;
+  for (uint32_t turn = 0; turn * kCheckRows < nt; ++turn) {
+    const uint32_t row = turn * kCheckRows + ((turn & 1u) ? kCheckRows - 1u - blockIdx.y : blockIdx.y);
+    if (row >= nt || blockIdx.x > row) continue;
+    const uint32_t a = row * kCheckTile + threadIdx.x;
+    const uint32_t earliest = __float_as_uint(ppos[row * kCheckTile].w);  // scene of the row's first particle
+    bool moves = false;
+    float4 pa = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float rm2 = 0.0f;
     if (a < P) {
       const float4 na = pnsum[plist[a]];
-      if (!(sqrtf(na.x * na.x + na.y * na.y + na.z * na.z) <= 1e-9f)) {  // else it never moves
-        const float4 pa = ppos[a];
+      moves = !(sqrtf(na.x * na.x + na.y * na.y + na.z * na.z) <= 1e-9f);
+      pa = ppos[a];
+      const float r_min = 0.2f * sc[__float_as_uint(pa.w)].k.h;
+      rm2 = r_min * r_min;
+    }
+    for (uint32_t back = blockIdx.x; back <= row; back += kCheckCols) {
+      const uint32_t b0 = (row - back) * kCheckTile;
+      __syncthreads();
+      if (b0 + threadIdx.x < P) tile[threadIdx.x] = ppos[b0 + threadIdx.x];
+      if (threadIdx.x == 0) found = *(volatile const uint32_t*)&ctl->work[kWorkTrigger];
+      __syncthreads();
+      if (found) return;
+      if (back && __float_as_uint(tile[kCheckTile - 1].w) < earliest) break;  // (a tile before the row's own is full)
+      if (moves) {
         const uint32_t q = __float_as_uint(pa.w);
-        const float r_min = 0.2f * sc[q].k.h;
-        const float rm2 = r_min * r_min;
         bool close = false;
-        for (uint32_t t = 0; t < min(kCheckTile, a - b0); ++t) {
+        const uint32_t n = back ? kCheckTile : threadIdx.x;  // of its own tile, the earlier ones
+#pragma unroll 8
+        for (uint32_t t = 0; t < n; ++t) {
           const float4 pb = tile[t];
           const float dx = pa.x - pb.x, dy = pa.y - pb.y, dz = pa.z - pb.z;
           close |= dx * dx + dy * dy + dz * dz < rm2 && __float_as_uint(pb.w) == q;

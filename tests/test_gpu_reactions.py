@@ -70,6 +70,56 @@ def test_separation_check_over_tiles(vxl, oracle_mod, n, close):
         compare_state(g, o, f"{n} pushed, close {close}")
 
 
+def _pushed_line(vxl, n, close=()):
+    """n particles on a line under the floor, two of them 1e-4 apart."""
+    pos = np.stack([0.05 * np.arange(n), np.full(n, -0.001), np.zeros(n)], 1).astype(F32)
+    if close:
+        pos[close[1]] = pos[close[0]] + np.array([0.0001, 0.0, 0.0], F32)
+    return _custom(vxl, pos, h=0.1, spacing=0.05)
+
+
+def _floored(vxl, specs):
+    from vxl_sph import scenes
+    b = vxl.Batch(specs)
+    for q in range(len(specs)):
+        b.set_providers([scenes.floor_provider()], q)
+    return b
+
+
+def test_separation_check_over_scenes(vxl):
+    """Scenes shorter and longer than the check's tiles side by side, at the same places, some with a close pair:
+    each as alone."""
+    specs = [_pushed_line(vxl, n, c) for n, c in ((1, ()), (130, (3, 129)), (5, ()), (127, ()), (300, (5, 290)), (2, (0, 1)),
+                                                  (256, ()), (700, (0, 699)), (1, ()))]
+    both = _floored(vxl, specs)
+    alone = [_floored(vxl, [s]) for s in specs]
+    for t in range(2):
+        both.substep(1.0 / 240.0)
+        for q, g in enumerate(alone):
+            g.substep(1.0 / 240.0)
+            for x, y in zip(both.read_state(q), g.read_state(0)):
+                assert x.tobytes() == y.tobytes(), (t, q)
+
+
+def test_separation_check_grows_with_the_scenes_not_their_square(vxl):
+    """Eight times the scenes (2,048 pushed particles each) take at most eight times the wall kernels' time; with
+    the pairs of all scenes tested it was 64 times the pairs."""
+    ms = []
+    for n in (8, 64):
+        line = _pushed_line(vxl, 2048)
+        b = _floored(vxl, [line] * n)
+        b.set_profile(True)
+        for _ in range(5):
+            for q in range(n):
+                b.write_state(q, line.pos, line.vel)
+            b.substep(1e-4)
+        total, launches = b.profile()["k_walls"]
+        assert launches > 0
+        ms.append(total / launches)
+        b.close()
+    assert ms[1] < 8 * ms[0], ms
+
+
 @pytest.mark.parametrize("h,over", [(0.1, {}), (0.1, dict(tensile_instability_suppression=False)), (3e-4, {}), (2e-3, {}),
                                     (900.0, {}), (3000.0, {}), (0.1, dict(artificial_viscosity=0.0)),
                                     (0.1, dict(artificial_viscosity=3e3)), (0.1, dict(rest_density=1e-15)),
