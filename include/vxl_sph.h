@@ -193,7 +193,9 @@ vxl_status vxl_sph_read_fields(vxl_sph_handle* h, float* dens, float* press, flo
 /* Neighbour table of the last substep (FluidSystem::neighbor_grid,
  * crates/vxl-phys-fluid/src/fluid_access.rs:125-133): items[n_total] = particle
  * index per cell-ordered slot, start[total+1], bins[n_total] = cell of each particle.
- * start_cap is the capacity of start in entries. Any array may be NULL. */
+ * start_cap is the capacity of start in entries. Any array may be NULL. After a skipped
+ * substep (vxl_sph_create_batch) there is no table until the next one that runs: info
+ * alone is filled, a call for an array returns VXL_NOT_READY. */
 vxl_status vxl_sph_export_grid(vxl_sph_handle* h, uint32_t* items, uint32_t* start, uint64_t start_cap,
                                uint32_t* bins, vxl_sph_grid_info* info);
 
@@ -207,7 +209,8 @@ vxl_status vxl_sph_export_grid(vxl_sph_handle* h, uint32_t* items, uint32_t* sta
  * entries NULL only offsets and *total are written (call once to size, once to fill);
  * entries_cap below the total is VXL_SIZE_MISMATCH. Lists longer than the recorded cap
  * are walked again from that substep's sorted positions, as the consumers do. Valid until
- * the next substep starts. */
+ * the next substep starts; a skipped one (vxl_sph_create_batch) leaves the offsets of the
+ * lists before it, and a call for the entries returns VXL_NOT_READY. */
 vxl_status vxl_sph_export_neighbors(vxl_sph_handle* h, uint64_t* offsets, uint64_t offsets_len, uint32_t* entries,
                                     uint64_t entries_cap, uint64_t* total);
 

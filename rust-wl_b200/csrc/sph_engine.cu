@@ -1151,8 +1151,7 @@ vxl_status Engine::export_grid(uint32_t q, uint32_t* items, uint32_t* start, uin
   }
   if (start && start_cap < total + 1) return set_error(VXL_SIZE_MISMATCH, "start buffer smaller than cells + 1");
   if (!start && !(items && n) && !(bins && n)) return VXL_OK;
-  if ((uint64_t)rec.cell_off + total > cell_cap_)
-    return set_error(VXL_NOT_READY, "no table: the last substep's cells exceeded the capacity and it was skipped");
+  if (last_skipped()) return set_error(VXL_NOT_READY, "no table: the last substep was skipped");
   uint32_t* ref_start = counts_;  // the table in the reference's cell order (the counts are zero between substeps)
   uint32_t* d_items = (uint32_t*)stage_;
   uint32_t* d_bins = d_items + n;
@@ -1200,6 +1199,7 @@ vxl_status Engine::export_neighbors(uint32_t q, uint64_t* offsets, uint64_t offs
   if (total) *total = acc;
   if (!entries || acc == 0) return VXL_OK;
   if (entries_cap < acc) return set_error(VXL_SIZE_MISMATCH, "entries buffer smaller than the list total");
+  if (last_skipped()) return set_error(VXL_NOT_READY, "no lists: the last substep was skipped");
   unsigned long long* off_d = nullptr;
   uint32_t* ent_d = nullptr;
   cudaError_t ce = cudaMalloc(&off_d, ((size_t)n + 1) * 8);
@@ -1604,6 +1604,7 @@ vxl_status Engine::step_tick_async(float dt_tick) {
     launches_last_tick_ = launches_counter_;
     CU(cudaGetLastError());
     ran_substep_ = true;
+    skipped_ = false;
     return VXL_OK;
   }
   if (!graph_ || graph_key_ != key || graph_epoch_ != membership_epoch_) {
@@ -1628,6 +1629,7 @@ vxl_status Engine::step_tick_async(float dt_tick) {
   CU(cudaGraphLaunch(graph_, stream_));
   prof_pending_ = prof_;
   ran_substep_ = true;
+  skipped_ = false;
   return VXL_OK;
 }
 
@@ -1638,6 +1640,7 @@ vxl_status Engine::finish() {
   if (ctl_h_->err & kErrCellCap) {
     const bool wait = (ctl_h_->err & kErrScanWait) != 0u;
     ctl_h_->err = 0;
+    skipped_ = true;
     cudaMemsetAsync(&ctl_d_->err, 0, 4, stream_);
     // the skipped substeps left the state as it was but emptied the fluid AABB
     // accumulators (reset by the grid-box pass): rebuild them from the state
@@ -1695,6 +1698,7 @@ vxl_status Engine::substep(const std::vector<float>& dt) {
   launches_last_tick_ = launches_counter_;
   CU(cudaGetLastError());
   ran_substep_ = true;
+  skipped_ = false;
   return finish();
 }
 
@@ -1786,6 +1790,8 @@ vxl_status Engine::autotune(float dt_tick, uint32_t trials, Tuning* best, float*
   if (best_ms) *best_ms = best_v;
   return VXL_OK;
 }
+
+bool Engine::last_skipped() const { return skipped_ || (ctl_h_->err & kErrCellCap) != 0u; }
 
 uint32_t Engine::cells_last() {
   EngineCtl c;

@@ -2624,7 +2624,6 @@ __global__ void k_e_export_table(const uint32_t* __restrict__ start, const uint3
   uint32_t at = ref_start[c];
   for (uint32_t q = start[e]; q < start[e + 1]; ++q) {
     const uint32_t o = orig[q] - S.base;
-    if (o >= S.count || at >= S.count) return;  // the table of a skipped substep is not this grid's
     if (items) items[at] = o;
     if (bins) bins[o] = c;
     ++at;

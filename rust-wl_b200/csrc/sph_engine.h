@@ -259,6 +259,8 @@ class Engine {
 
   bool record_ = false;
   bool ran_substep_ = false;
+  bool skipped_ = false;  // the last tick ended in a skipped substep: the scenes' grids are newer than table and lists
+  bool last_skipped() const;  // with the stream idle: a tick not yet waited for counts too
   bool use_graph_ = true;
   Tuning tuning_;
   int grid_density_ = 0, grid_force_ = 0, grid_bforce_ = 0;

@@ -9,6 +9,8 @@ boundaries; each finished request's state must equal the same scene stepped alon
 plain handle for the same number of ticks (the alone-vs-mix check), bit for bit,
 including when the budget forces requests to wait in the queue.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -169,6 +171,48 @@ def test_cell_capacity_overflow_is_reported_and_harmless(vxl):
             p, v = b.read_state(q)
             _assert_same(p, before[q][0], f"scene {q} pos")
             _assert_same(v, before[q][1], f"scene {q} vel")
+
+
+def test_no_table_after_a_skipped_substep(vxl):
+    """A substep that ran, then one skipped because another scene's cells outgrew the capacity: the tables and
+    lists of every scene are refused (its new grid would be read against the old table), before and after the
+    tick is waited for, until a substep runs again."""
+    specs = _specs()[:2]
+    b = vxl.Batch(specs, cell_capacity=60000)
+    wide = specs[1].pos.copy()
+    wide[:1000:7] += F32(3.0)  # some 38^3 cells
+    info = vxl.GridInfo()
+    for late in (False, True):
+        b.step_tick(DT_TICK)
+        table = b.export_grid(0)
+        b.write_state(1, wide, None)
+        b.step_tick_async(DT_TICK)
+        if late:
+            with pytest.raises(vxl.VxlError) as e:
+                b.sync()
+            assert e.value.status == vxl.DEVICE_FAULT_FLAG and "cell capacity" in str(e.value)
+        for q in (0, 1):
+            with pytest.raises(vxl.VxlError) as e:
+                b.export_grid(q)
+            assert e.value.status == vxl.NOT_READY
+            info.hdr = vxl.header(vxl.GridInfo)
+            assert b.lib.vxl_sph_export_grid_scene(b._h, q, None, None, 0, None, ctypes.byref(info)) == vxl.OK
+            assert info.total > 0
+        off, tot = np.empty(specs[0].n_total + 1, np.uint64), ctypes.c_uint64()
+        op = off.ctypes.data_as(ctypes.POINTER(ctypes.c_uint64))
+        ent = np.empty(1 << 20, np.uint32)
+        assert b.lib.vxl_sph_export_neighbors(b._h, op, off.size, None, 0, ctypes.byref(tot)) == vxl.OK
+        assert 0 < tot.value <= ent.size
+        st = b.lib.vxl_sph_export_neighbors(b._h, op, off.size, vxl._u32ptr(ent), ent.size, ctypes.byref(tot))
+        assert st == vxl.NOT_READY
+        if not late:
+            with pytest.raises(vxl.VxlError):
+                b.sync()
+        b.write_state(0, specs[0].pos, specs[0].vel)
+        b.write_state(1, specs[1].pos, specs[1].vel)
+    b.step_tick(DT_TICK)
+    for x, y in zip(table[:3], b.export_grid(0)[:3]):
+        assert np.array_equal(x, y)
 
 
 def test_served_request_that_never_fits_is_rejected(vxl):
