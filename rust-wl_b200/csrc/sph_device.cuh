@@ -23,7 +23,8 @@ struct GridBox {
   uint32_t nx, ny, nz;
   uint32_t total;
   uint32_t reach_q;  // candidate filter: the squared reach in cell units of 1/64 bin (sub_word below)
-  uint32_t pad[2];
+  uint32_t rows;     // neighbour-list entries by rows (list_by_rows)
+  uint32_t pad;
 };
 
 // Constants of one scene, computed on the host exactly as FluidSystem::new does
@@ -196,6 +197,7 @@ __device__ inline bool grid_box(float lox, float loy, float loz, float hix, floa
   g.total = dims[0] * dims[1] * dims[2];
   const float reach = (float)kSubUnits * (h / bin) + (1.75f + 4.2e-5f * (float)max(dims[0], max(dims[1], dims[2])));
   g.reach_q = (uint32_t)ceilf(reach * reach);
+  g.rows = 0;
   return ok;
 }
 

@@ -1433,7 +1433,10 @@ void Engine::enqueue_substep(bool with_reactions) {
   // grids, cell table, sorted buffer, permutation, lists, work counters): join it first.
   // Its reaction sums read only bforce / bpos and go on beside this substep.
   join_side_only();
-  LAUNCH(KID_CELLOFF, k_e_celloff<<<1, S <= 32 ? 32 : kCelloffThreads, 0, st>>>(sc_d_, S, ctl_d_, (uint32_t)cell_cap_));
+  static_assert(kTeamForce.four >= kTeamDensity.four, "rows: one lane in the force pass means one lane in the density pass");
+  const bool rows = team_lanes(load, kTeamForce) == 1;
+  LAUNCH(KID_CELLOFF, k_e_celloff<<<1, S <= 32 ? 32 : kCelloffThreads, 0, st>>>(sc_d_, S, ctl_d_, (uint32_t)cell_cap_,
+                                                                                                 rows));
   LAUNCH(KID_KEYS, k_e_keys<<<key_blocks, kThreads, 0, st>>>(p0, sc_d_, tiles_d_, ntiles_, ctl_d_, counts_,
                                                              (uint2*)cellrank_, wet_));
   LAUNCH(KID_SCAN, k_e_scan<<<148 * 4, kScanThreads, 0, st>>>(counts_, ctl_d_, scan_, start_));

@@ -20,7 +20,7 @@ import os
 import numpy as np
 import pytest
 
-from test_gpu_parity import F32, assert_bits, compare_grid, compare_state, f32_dt
+from test_gpu_parity import F32, _custom, assert_bits, compare_grid, compare_state, f32_dt
 
 pytestmark = pytest.mark.gpu
 
@@ -108,6 +108,83 @@ def test_neighbor_lists_longer_than_the_recorded_cap(vxl, oracle_mod, density):
     g, o = _lists_after(vxl, oracle_mod, spec, density=density)
     offs, _ = _compare_lists(g, o, "h = 3 s")
     assert np.diff(offs.astype(np.int64)).max() > 64
+
+
+def _channel(vxl, max_bins, plate=0.0):
+    """A channel of fluid 1,200 particles long in x (more than 36,000: one lane per particle), over a plate."""
+    from vxl_sph import scenes
+    s = 0.005
+    pos = scenes.jitter(scenes.fluid_block((0.0, 0.0, 0.0), (1200, 6, 6), s), s, 8, 0.2)
+    b = None
+    if plate:
+        b = scenes.body_particles([scenes.Body(0, (plate / 2, s, 0.03), (3.0, -1.5 * s, 0.015))], s, 2 * s, 1, 1000.0)
+    return _custom(vxl, pos, h=2 * s, spacing=s, max_bins=max_bins, boundary=b)
+
+
+@pytest.mark.parametrize("max_bins,plate,walls", [(3000, 0.0, False), (3000, 2.0, False), (3000, 5.5, False), (3000, 0.0, True),
+                                                  (200, 0.0, False), (20, 0.0, False)])
+def test_lists_of_a_scene_long_in_x(vxl, oracle_mod, max_bins, plate, walls):
+    """List entries by rows: at bins of 2h, with boundary reactions of few and of many boundary particles, with
+    provider walls, and at 8h and 32h, where three cells hold up to 1,728 and 6,912 particles (past the
+    12 bits, walked again)."""
+    from vxl_sph import scenes
+    spec = _channel(vxl, max_bins, plate)
+    assert plate < 5 or spec.n_boundary > 20000
+    g = vxl.Scene(spec.params, spec.pos, spec.vel, spec.pmass, spec.n_fluid)
+    o = oracle_mod.OracleSystem.from_scene(spec, threads=_threads())
+    if walls:
+        for x in (g, o):
+            x.set_providers([scenes.floor_provider(), scenes.box_obstacle((3.0, 0.0, 0.0), (0.5, 0.01, 0.01))])
+    dt = f32_dt(40)
+    g.set_record(True)
+    for _ in range(2):
+        g.substep(dt)
+        o.substep(dt)
+    bf = g.read_fields()[4]
+    if plate:
+        assert np.any(bf != 0)
+        assert_bits(bf, o.read_f32()["bforce"][spec.n_fluid:], "bforce")
+    compare_grid(g, o, "channel")
+    compare_state(g, o, "channel")
+    g.substep(dt)
+    _compare_lists(g, o, "channel")  # the oracle's from its positions, the next substep's
+
+
+def test_long_scene_beside_a_short_one(vxl):
+    """Entries by rows and by planes in one handle, each scene bitwise as alone."""
+    from vxl_sph import scenes
+    specs = [scenes.small_dam(n=(9, 8, 7), spacing=0.05, tank=(0.7, 0.6, 0.5), seed=8), _channel(vxl, 3000, 1.0),
+             _custom(vxl, scenes.jitter(scenes.fluid_block((0, 0, 0), (12, 10, 8), 0.05), 0.05, 11), max_bins=64)]
+    both = vxl.Batch(specs)
+    alone = [vxl.Batch([x]) for x in specs]
+    for t in range(2):
+        rb = both.step_tick(1.0 / 600.0)
+        ra = [r for g in alone for r in g.step_tick(1.0 / 600.0)]
+        for (b1, f1, t1), (b2, f2, t2) in zip(ra, rb):
+            assert b1 == b2 and f1.tobytes() == f2.tobytes() and t1.tobytes() == t2.tobytes(), (t, b1)
+        for q, g in enumerate(alone):
+            for x, y in zip(both.read_state(q), g.read_state(0)):
+                assert x.tobytes() == y.tobytes(), (t, q)
+
+
+def test_force_pass_of_a_long_scene_is_no_slower_along_x(vxl):
+    """The lists hold whichever way a scene is long: the force pass of a block 900 long in x takes at most twice
+    that of the same block along z (walked again for want of lists it took eight times as long)."""
+    from vxl_sph import scenes
+    ms = []
+    for dims in ((900, 30, 30), (30, 30, 900)):
+        s = 0.005
+        pos = scenes.jitter(scenes.fluid_block((0.0, 0.0, 0.0), dims, s), s, 1)
+        spec = _custom(vxl, pos, h=2 * s, spacing=s, max_bins=60000)
+        g = vxl.Scene(spec.params, spec.pos, spec.vel, spec.pmass, spec.n_fluid)
+        g.substep(1e-5)
+        g.set_profile(True)
+        for _ in range(5):
+            g.substep(1e-5)
+        total, n = g.profile()["k_force"]
+        ms.append(total / n)
+        g.close()
+    assert ms[0] < 2 * ms[1], ms
 
 
 def test_neighbor_lists_before_any_substep_is_not_ready(vxl):
