@@ -1869,6 +1869,11 @@ __global__ void __launch_bounds__(kCheckTile) k_e_separate_check(const SceneDev*
   for (uint32_t turn = 0; turn * kCheckRows < nt; ++turn) {
     const uint32_t row = turn * kCheckRows + ((turn & 1u) ? kCheckRows - 1u - blockIdx.y : blockIdx.y);
     if (row >= nt || blockIdx.x > row) continue;
+    auto load = [&](uint32_t back) {
+      const uint32_t b = (row - back) * kCheckTile + threadIdx.x;
+      return b < P ? ppos[b] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    };
+    float4 next = load(blockIdx.x);  // in flight beside the row's own loads, the following ones beside the tests
     const uint32_t a = row * kCheckTile + threadIdx.x;
     const uint32_t earliest = __float_as_uint(ppos[row * kCheckTile].w);  // scene of the row's first particle
     bool moves = false;
@@ -1884,11 +1889,12 @@ __global__ void __launch_bounds__(kCheckTile) k_e_separate_check(const SceneDev*
     for (uint32_t back = blockIdx.x; back <= row; back += kCheckCols) {
       const uint32_t b0 = (row - back) * kCheckTile;
       __syncthreads();
-      if (b0 + threadIdx.x < P) tile[threadIdx.x] = ppos[b0 + threadIdx.x];
+      tile[threadIdx.x] = next;
       if (threadIdx.x == 0) found = *(volatile const uint32_t*)&ctl->work[kWorkTrigger];
       __syncthreads();
       if (found) return;
       if (back && __float_as_uint(tile[kCheckTile - 1].w) < earliest) break;  // (a tile before the row's own is full)
+      if (back + kCheckCols <= row) next = load(back + kCheckCols);
       if (moves) {
         const uint32_t q = __float_as_uint(pa.w);
         bool close = false;
