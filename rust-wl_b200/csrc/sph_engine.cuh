@@ -1887,7 +1887,6 @@ __global__ void __launch_bounds__(kCheckTile) k_e_separate_check(const SceneDev*
       rm2 = r_min * r_min;
     }
     for (uint32_t back = blockIdx.x; back <= row; back += kCheckCols) {
-      const uint32_t b0 = (row - back) * kCheckTile;
       __syncthreads();
       tile[threadIdx.x] = next;
       if (threadIdx.x == 0) found = *(volatile const uint32_t*)&ctl->work[kWorkTrigger];
@@ -2664,55 +2663,84 @@ __device__ __forceinline__ uint32_t engine_cell(const GridBox& g, uint32_t c) {
   return (z * g.ny + y) * g.nx + x;
 }
 
-__global__ void k_e_export_counts(const uint32_t* __restrict__ start, const SceneDev* __restrict__ sc, uint32_t scene,
-                                  uint32_t* __restrict__ ref_start) {
-  const SceneDev& S = sc[scene];
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c > S.cells) return;
-  const uint32_t e = S.cell_off + (c < S.cells ? engine_cell(S.g, c) : 0u);
-  ref_start[c] = c < S.cells ? start[e + 1] - start[e] : 0u;
-}
+constexpr uint32_t kExportTile = 512;
+constexpr int kExportThreads = 256;
 
-// Exclusive scan in place, one block.
-__global__ void __launch_bounds__(1024) k_e_export_scan(uint32_t* __restrict__ v, uint32_t n) {
-  __shared__ uint32_t ws[32];
-  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint32_t carry = 0;
-  for (uint32_t b0 = 0; b0 < n; b0 += 1024) {
-    const uint32_t i = b0 + threadIdx.x;
-    const uint32_t x = i < n ? v[i] : 0u;
-    uint32_t incl = x;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
-      if ((int)lane >= off) incl += y;
-    }
-    __syncthreads();
-    if (lane == 31) ws[w] = incl;
-    __syncthreads();
-    uint32_t before = carry;
-    for (uint32_t k = 0; k < 32; ++k) {
-      if (k < w) before += ws[k];
-      carry += ws[k];
-    }
-    if (i < n) v[i] = before + incl - x;
+// Reference cells of one tile: their counts, and the tile's sum.
+__global__ void __launch_bounds__(kExportThreads) k_e_export_counts(const uint32_t* __restrict__ start,
+                                                                    const SceneDev* __restrict__ sc, uint32_t scene,
+                                                                    uint32_t* __restrict__ ref_start,
+                                                                    uint32_t* __restrict__ sums) {
+  __shared__ uint32_t sh[32];
+  const SceneDev& S = sc[scene];
+  uint32_t sum = 0;
+  for (uint32_t k = threadIdx.x; k < kExportTile; k += kExportThreads) {
+    const uint32_t c = blockIdx.x * kExportTile + k;
+    if (c > S.cells) break;
+    const uint32_t e = S.cell_off + (c < S.cells ? engine_cell(S.g, c) : 0u);
+    const uint32_t n = c < S.cells ? start[e + 1] - start[e] : 0u;
+    ref_start[c] = n;
+    sum += n;
   }
+  sum = block_sum(sum, sh);
+  if (threadIdx.x == 0) sums[blockIdx.x] = sum;
 }
 
-__global__ void k_e_export_table(const uint32_t* __restrict__ start, const uint32_t* __restrict__ orig,
-                                 const SceneDev* __restrict__ sc, uint32_t scene,
-                                 const uint32_t* __restrict__ ref_start, uint32_t* __restrict__ items,
-                                 uint32_t* __restrict__ bins) {
+// The tile's exclusive scan in place, from the sums of the tiles before it, and its cells'
+// particles. Tiles of 512 spread a small scene's cells over the SMs: 33k particles in 9k cells, a
+// call of 0.122 ms (0.144 with tiles of 2,048); 1.1M cells 0.60 ms, 1.86 when one block scanned them all.
+__global__ void __launch_bounds__(kExportThreads) k_e_export_table(const uint32_t* __restrict__ start,
+                                                                   const uint32_t* __restrict__ orig,
+                                                                   const SceneDev* __restrict__ sc, uint32_t scene,
+                                                                   uint32_t* __restrict__ ref_start,
+                                                                   const uint32_t* __restrict__ sums,
+                                                                   uint32_t* __restrict__ items, uint32_t* __restrict__ bins) {
+  constexpr uint32_t kPer = kExportTile / kExportThreads;
+  __shared__ uint32_t sh[32], s_at[kExportTile];
   const SceneDev& S = sc[scene];
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= S.cells) return;
-  const uint32_t e = S.cell_off + engine_cell(S.g, c);
-  uint32_t at = ref_start[c];
-  for (uint32_t q = start[e]; q < start[e + 1]; ++q) {
-    const uint32_t o = orig[q] - S.base;
-    if (items) items[at] = o;
-    if (bins) bins[o] = c;
-    ++at;
+  uint32_t part = 0;
+  for (uint32_t k = threadIdx.x; k < blockIdx.x; k += kExportThreads) part += sums[k];
+  uint32_t run = block_sum(part, sh);
+  const uint32_t c0 = blockIdx.x * kExportTile, last = min(kExportTile, S.cells + 1u - c0);  // cells of the tile, one past the last too
+  for (uint32_t k = threadIdx.x; k < last; k += kExportThreads) s_at[k] = ref_start[c0 + k];
+  __syncthreads();
+  uint32_t v[kPer], local = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < kPer; ++q) {
+    const uint32_t k = threadIdx.x * kPer + q;
+    v[q] = k < last ? s_at[k] : 0u;
+    local += v[q];
+  }
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t incl = local;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+    if ((int)lane >= off) incl += y;
+  }
+  if (lane == 31) sh[w] = incl;
+  __syncthreads();
+  for (uint32_t k = 0; k < w; ++k) run += sh[k];
+  run += incl - local;
+#pragma unroll
+  for (uint32_t q = 0; q < kPer; ++q) {
+    const uint32_t k = threadIdx.x * kPer + q;
+    if (k < last) s_at[k] = run;
+    run += v[q];
+  }
+  __syncthreads();
+  for (uint32_t k = threadIdx.x; k < last; k += kExportThreads) {
+    const uint32_t c = c0 + k;
+    uint32_t at = s_at[k];
+    ref_start[c] = at;
+    if (c == S.cells || (!items && !bins)) continue;
+    const uint32_t e = S.cell_off + engine_cell(S.g, c);
+    for (uint32_t q = start[e]; q < start[e + 1]; ++q) {
+      const uint32_t o = orig[q] - S.base;
+      if (items) items[at] = o;
+      if (bins) bins[o] = c;
+      ++at;
+    }
   }
 }
 
