@@ -255,8 +255,10 @@ vxl_status vxl_sph_profile_read(vxl_sph_handle* h, uint32_t k, const char** name
 /* Create a handle holding n scenes (descs[i] as for vxl_sph_create; all on `device`;
  * all must share `substeps` to be stepped by vxl_sph_step_tick). cell_capacity bounds
  * the sum of the scenes' cells per substep (0 = the sum of their max_bins, capped at
- * 2^28); a substep that would exceed it is skipped and reported as
- * VXL_DEVICE_FAULT_FLAG. */
+ * 2^28); a substep that would exceed it is skipped with the rest of its tick, and the
+ * tick reported as VXL_DEVICE_FAULT_FLAG: the state is the last substep's that ran (the
+ * tick's own start if it was its first). The same status, with another message, says that
+ * a bounded wait inside the substep ran out. */
 vxl_status vxl_sph_create_batch(const vxl_sph_desc* descs, uint32_t n, int32_t device, uint64_t cell_capacity,
                                 vxl_sph_handle** out);
 uint32_t vxl_sph_scene_count(vxl_sph_handle* h);

@@ -313,6 +313,12 @@ vxl_status vxl_sph_substep(vxl_sph_handle* h, float dt) {
   return h->e->substep(std::vector<float>(h->e->scenes().size(), dt));
 }
 
+int vxl_sph_internal_scan_wait(vxl_sph_handle* h, uint32_t looks) {
+  HANDLE_OR_FAIL(h);
+  h->e->set_scan_wait(looks);
+  return VXL_OK;
+}
+
 vxl_status vxl_sph_bounds(vxl_sph_handle* h, float lo[3], float hi[3]) {
   HANDLE_OR_FAIL(h);
   if (!lo || !hi) return set_error(VXL_NULL_POINTER, "NULL argument");

@@ -1438,7 +1438,7 @@ void Engine::enqueue_substep(bool with_reactions) {
                                                                                                  rows));
   LAUNCH(KID_KEYS, k_e_keys<<<key_blocks, kThreads, 0, st>>>(p0, sc_d_, tiles_d_, ntiles_, ctl_d_, counts_,
                                                              (uint2*)cellrank_, wet_));
-  LAUNCH(KID_SCAN, k_e_scan<<<148 * 4, kScanThreads, 0, st>>>(counts_, ctl_d_, scan_, start_));
+  LAUNCH(KID_SCAN, k_e_scan<<<148 * 4, kScanThreads, 0, st>>>(counts_, ctl_d_, scan_, start_, scan_wait_));
   LAUNCH(KID_PLACE, k_e_place<<<key_blocks, kThreads, 0, st>>>((const uint2*)cellrank_, start_, orig_, tiles_d_,
                                                                ntiles_, ctl_d_, (uint2*)items_, order_));
   LAUNCH(KID_CANON, k_e_canon<<<std::max<uint32_t>(blocks_for(used_), 1), 256, 0, st>>>(
@@ -1652,8 +1652,9 @@ vxl_status Engine::finish() {
     }
     cudaStreamSynchronize(stream_);
     return set_error(VXL_DEVICE_FAULT_FLAG,
-                     wait ? "a wait of the cell scan ran out; the rest of the tick was skipped"
-                          : "the scenes' cells exceed the engine's cell capacity; the tick was skipped, state unchanged");
+                     std::string(wait ? "a wait of the cell scan ran out"
+                                      : "the scenes' cells exceed the engine's cell capacity") +
+                         "; the substep and the rest of its tick were skipped, the state is the last substep's that ran");
   }
   return VXL_OK;
 }
@@ -1791,6 +1792,14 @@ vxl_status Engine::autotune(float dt_tick, uint32_t trials, Tuning* best, float*
   if (best) *best = best_t;
   if (best_ms) *best_ms = best_v;
   return VXL_OK;
+}
+
+void Engine::set_scan_wait(uint32_t looks) {
+  scan_wait_ = looks;
+  if (graph_) {  // the limit is an argument of the captured launches
+    cudaGraphExecDestroy(graph_);
+    graph_ = nullptr;
+  }
 }
 
 bool Engine::last_skipped() const { return skipped_ || (ctl_h_->err & kErrCellCap) != 0u; }

@@ -533,14 +533,15 @@ __global__ void k_e_keys(const float4* __restrict__ pos, const SceneDev* __restr
 // one whose whole prefix is known, and publishes its own. A published word is (epoch, kind,
 // value) in 64 bits, so words of earlier substeps read as unpublished. Every tile looked at
 // was drawn earlier by a block that publishes without waiting, so the wait ends; it has a limit
-// all the same, after which the substep is flagged like a cell overflow (the later
-// kernels touch nothing). In two launches (tile sums, then tiles) the scan took 8 us of a
+// all the same (`wait` looks at a group of predecessors), after which the substep is flagged like a
+// cell overflow: the block goes on with a prefix of its own making, so that every tile is drawn and its
+// counts zeroed, and the later kernels touch nothing. In two launches (tile sums, then tiles) the scan took 8 us of a
 // small scene's substep: with the cell offsets 17 us of a 33k-particle substep, 11 in one; at
 // 10M particles 20 us either way.
 constexpr uint32_t kScanSum = 1u, kScanPrefix = 2u;
-constexpr uint32_t kScanWait = 1u << 22;
 __global__ void __launch_bounds__(kScanThreads) k_e_scan(uint32_t* __restrict__ counts, EngineCtl* ctl,
-                                                         unsigned long long* state, uint32_t* __restrict__ start) {
+                                                         unsigned long long* state, uint32_t* __restrict__ start,
+                                                         uint32_t wait) {
   if (__syncthreads_or((ctl->err & kErrCellCap) != 0u)) return;  // a whole block: another may flag its wait meanwhile
   const uint32_t total = ctl->cells;
   const uint32_t ntiles = (total + kScanTile - 1) / kScanTile;
@@ -582,17 +583,16 @@ __global__ void __launch_bounds__(kScanThreads) k_e_scan(uint32_t* __restrict__ 
         const bool in = lane < at;
         uint32_t kind = in ? 0u : kScanPrefix, val = 0;  // before the first tile: a known prefix of 0
         for (uint32_t tries = 0; !__all_sync(0xffffffffu, kind != 0u); ++tries) {
-          if (kind == 0u) {
+          if (tries == wait) {
+            if (kind == 0u) {
+              atomicOr(&ctl->err, kErrCellCap | kErrScanWait);
+              kind = kScanPrefix;
+            }
+          } else if (kind == 0u) {
             const unsigned long long word = vs[at - 1 - lane];
             if ((uint32_t)(word >> 34) == tag >> 2) {
               kind = (uint32_t)(word >> 32) & 3u;
               val = (uint32_t)word;
-            }
-          }
-          if (tries == kScanWait) {
-            if (kind == 0u) {
-              atomicOr(&ctl->err, kErrCellCap | kErrScanWait);
-              kind = kScanPrefix;
             }
           }
         }

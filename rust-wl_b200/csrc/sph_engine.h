@@ -114,6 +114,7 @@ class Engine {
   void set_record(bool on) { record_ = on; }
   bool record() const { return record_; }
   void set_use_graph(bool on) { use_graph_ = on; }
+  void set_scan_wait(uint32_t looks);
   void set_tuning(const Tuning& t);
   const Tuning& tuning() const { return tuning_; }
   vxl_status set_profile(bool on);
@@ -261,6 +262,7 @@ class Engine {
   bool record_ = false;
   bool ran_substep_ = false;
   bool skipped_ = false;  // the last tick ended in a skipped substep: the scenes' grids are newer than table and lists
+  uint32_t scan_wait_ = 1u << 22;  // k_e_scan: looks at a group of predecessors before it gives up
   bool last_skipped() const;  // with the stream idle: a tick not yet waited for counts too
   bool use_graph_ = true;
   Tuning tuning_;

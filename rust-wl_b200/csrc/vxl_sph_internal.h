@@ -26,6 +26,11 @@ inline float vxl_o2f_host(uint32_t o) {
   return f;
 }
 
+// Limit of the cell scan's wait (Engine::set_scan_wait): not part of the public header, so that a
+// test can make the wait run out. 0: a tile gives up before its first look.
+struct vxl_sph_handle;
+extern "C" int vxl_sph_internal_scan_wait(vxl_sph_handle* h, uint32_t looks);
+
 // The thread-local message returned by vxl_sph_last_error() (defined in sph_engine.cu).
 void vxl_set_last_error(const char* msg);
 const char* vxl_get_last_error();

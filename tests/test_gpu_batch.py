@@ -215,6 +215,42 @@ def test_no_table_after_a_skipped_substep(vxl):
         assert np.array_equal(x, y)
 
 
+@pytest.mark.parametrize("form", ["tick", "substep"])
+def test_a_scan_wait_that_runs_out_is_reported_and_harmless(vxl, form):
+    """The cell scan's wait limit set to no look at all, on a grid of several tiles: the substep and the rest of the
+    tick are skipped and reported, the state stays, and with the limit back the handle steps like a new one."""
+    from vxl_sph import scenes
+    spec = scenes.small_dam(n=(8, 8, 8), spacing=0.02, tank=(1.0, 0.6, 0.6), seed=4)
+    g, ref = (vxl.Scene(spec.params, spec.pos, spec.vel, spec.pmass, spec.n_fluid) for _ in range(2))
+    lib = vxl.load()
+    lib.vxl_sph_internal_scan_wait.argtypes = [ctypes.c_void_p, ctypes.c_uint32]
+
+    def step(x):
+        return x.step_tick(DT_TICK, spec.spans) if form == "tick" else x.substep(DT_TICK / 4)
+
+    before = g.read_state()
+    for _ in range(2):
+        assert lib.vxl_sph_internal_scan_wait(g._h, 0) == vxl.OK
+        with pytest.raises(vxl.VxlError) as e:
+            step(g)
+        assert e.value.status == vxl.DEVICE_FAULT_FLAG and "wait" in str(e.value)
+        for a, b in zip(g.read_state(), before):
+            _assert_same(a, b, "state after the skipped substep")
+        with pytest.raises(vxl.VxlError) as e:
+            g.export_grid()
+        assert e.value.status == vxl.NOT_READY
+        assert lib.vxl_sph_internal_scan_wait(g._h, 1 << 22) == vxl.OK
+        got, want = step(g), step(ref)
+        assert g.export_grid()[3].total > 3 * 2048
+        for x, y in zip(got or [], want or []):
+            assert x[1].tobytes() == y[1].tobytes() and x[2].tobytes() == y[2].tobytes()
+        for x, y in zip(g.export_grid()[:3], ref.export_grid()[:3]):
+            assert np.array_equal(x, y)
+        before = g.read_state()
+        for a, b in zip(before, ref.read_state()):
+            _assert_same(a, b, "state after the wait's limit is back")
+
+
 def test_served_request_that_never_fits_is_rejected(vxl):
     from vxl_sph import scenes
     srv = vxl.Server(budget_bytes=64 << 20)
