@@ -280,7 +280,10 @@ vxl_status vxl_sph_reactions_all(vxl_sph_handle* h, vxl_sph_reaction* out, uint3
 /* Launch shape of the particle passes: threads per block (128 or 256), slots per tile
  * (a multiple of 128, at least one block) and the scheduling: waves = 0 runs one block
  * per tile, waves = k > 0 runs k x the occupancy limit of persistent blocks that draw
- * tiles from a counter. density once chose between two density kernels with the same
+ * tiles from a counter. Handles of up to about 34,000 particles (fluid and a quarter of
+ * the boundary; without provider walls) run kernels with several lanes per particle, whose
+ * shape follows tile alone; block and waves take effect when the handle outgrows them.
+ * density once chose between two density kernels with the same
  * results; both values are accepted and reported back, and run the one walk there is
  * now. Default {256, 256, 0, WALK}. */
 #define VXL_SPH_DENSITY_WALK 0u
@@ -296,7 +299,8 @@ typedef struct vxl_sph_tuning {
 vxl_status vxl_sph_set_tuning(vxl_sph_handle* h, const vxl_sph_tuning* t);
 vxl_status vxl_sph_get_tuning(vxl_sph_handle* h, vxl_sph_tuning* t);
 /* Autotuner: times every candidate shape on the handle's own scenes (`trials` substeps
- * each, from a snapshot of the state that is restored afterwards) and keeps the fastest.
+ * each, from a snapshot of the state that is restored afterwards) and keeps the fastest;
+ * where only tile has an effect (above) it tries the tiles and leaves block and waves.
  * Results are identical for every shape; only the time differs. */
 vxl_status vxl_sph_autotune(vxl_sph_handle* h, float dt_tick, uint32_t trials, vxl_sph_tuning* best);
 

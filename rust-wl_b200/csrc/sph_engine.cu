@@ -1417,13 +1417,23 @@ vxl_status Engine::profile_read(uint32_t k, const char** name, double* ms, uint6
 
 // ---------------------------------------------------------------- stepping
 
+uint64_t Engine::boundary_total() const {
+  uint64_t nb = 0;
+  for (auto& s : scenes_) nb += s.nb;
+  return nb;
+}
+
+// Load of the density and force passes (team_lanes).
+uint64_t Engine::pass_load() const {
+  const uint64_t nb = boundary_total();
+  return used_ - nb + nb / 4;
+}
+
 void Engine::enqueue_substep(bool with_reactions) {
   cudaStream_t st = stream_;
   const uint32_t S = (uint32_t)scenes_.size();
   const uint32_t key_blocks = std::min<uint32_t>(std::max<uint32_t>(ntiles_, 1), 148 * 8);
-  uint64_t nb_total = 0;
-  for (auto& s : scenes_) nb_total += s.nb;
-  const uint64_t load = used_ - nb_total + nb_total / 4;  // of the density and force passes (team_lanes)
+  const uint64_t nb_total = boundary_total(), load = pass_load();
   const float4* p0 = (const float4*)pos_[0];
   const float4* v0 = (const float4*)vel_[0];
   const float4* p1 = (const float4*)pos_[1];
@@ -1756,12 +1766,21 @@ vxl_status Engine::autotune(float dt_tick, uint32_t trials, Tuning* best, float*
   const uint32_t blocks[2] = {128, 256};
   const uint32_t tile_mult[3] = {1, 2, 4};
   const uint32_t waves_c[3] = {0, 1, 2};
+  // small scenes: with team kernels in both passes only the tile matters; block and waves stay
+  const bool teams = !walls_any_ && team_lanes(pass_load(), kTeamDensity) > 1;
   for (uint32_t bi = 0; st == VXL_OK && bi < 2; ++bi)
     for (uint32_t ti = 0; st == VXL_OK && ti < 3; ++ti)
       for (uint32_t wi = 0; st == VXL_OK && wi < 3; ++wi) {
+        Tuning shape{blocks[bi], blocks[bi] * tile_mult[ti], waves_c[wi], was.density};
+        if (teams) {
+          if (wi || (bi == 0 && ti)) continue;  // tiles of 128 and of 256, 512 and 1,024 slots
+          if (shape.tile < was.block) continue;  // a tile is at least one block
+          shape.block = was.block;
+          shape.waves = was.waves;
+        }
         st = copy_all(false);
         if (st != VXL_OK) break;
-        set_tuning(Tuning{blocks[bi], blocks[bi] * tile_mult[ti], waves_c[wi], was.density});
+        set_tuning(shape);
         enqueue_substep(false);  // warm-up
         cudaEventRecord(e0, stream_);
         for (uint32_t r = 0; r < trials; ++r) enqueue_substep(false);

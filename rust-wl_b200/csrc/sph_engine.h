@@ -115,6 +115,8 @@ class Engine {
   bool record() const { return record_; }
   void set_use_graph(bool on) { use_graph_ = on; }
   void set_scan_wait(uint32_t looks);
+  uint64_t boundary_total() const;
+  uint64_t pass_load() const;
   void set_tuning(const Tuning& t);
   const Tuning& tuning() const { return tuning_; }
   vxl_status set_profile(bool on);

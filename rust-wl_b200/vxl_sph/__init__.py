@@ -733,7 +733,7 @@ class Batch:
         t = Tuning()
         t.hdr = header(Tuning)
         _check(self.lib.vxl_sph_autotune(self._h, dt_tick, trials, C.byref(t)))
-        return {"block": t.block, "tile": t.tile, "waves": t.waves, "density": ["walk", "grouped"][t.density],
+        return {"block": t.block, "tile": t.tile, "waves": t.waves, "density": "walk",
                 "ms_per_substep": t.ms_per_substep}
 
     def set_stream(self, stream_handle: int | None) -> None:

@@ -93,6 +93,19 @@ def test_autotune_restores_state_and_keeps_results(vxl):
         _assert_same(tuned.read_state(q)[0], plain.read_state(q)[0], f"scene {q}")
 
 
+@pytest.mark.parametrize("block,waves", [(128, 2), (256, 1), (128, 0)])
+def test_autotune_leaves_what_has_no_effect(vxl, block, waves):
+    """A small handle's passes follow the tile alone: the autotuner keeps the block and waves it was given (they count
+    when the handle grows), and names the one density kernel."""
+    b = vxl.Batch(_specs())
+    b.set_tuning(block, 256, waves, 1)
+    for _ in range(3):
+        best = b.autotune(DT_TICK, trials=1)
+        assert (best["block"], best["waves"], best["density"]) == (block, waves, "walk")
+        assert best["tile"] in (128, 256, 512, 1024) and best["tile"] >= block
+        assert b.tuning() == (block, best["tile"], waves, 1)
+
+
 def _alone(vxl, spec, ticks):
     g = vxl.Scene(spec.params, spec.pos, spec.vel, spec.pmass, spec.n_fluid)
     for _ in range(ticks):
