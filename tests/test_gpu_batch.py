@@ -59,9 +59,12 @@ def test_batch_equals_oracle_and_plain(vxl, oracle_mod):
         assert np.array_equal(items, og["items"]) and np.array_equal(start, og["start"])
 
 
-@pytest.mark.parametrize("shape", [(128, 128, 0, 0), (256, 1024, 0, 1), (128, 128, 1, 1), (256, 256, 2, 0),
-                                   (128, 4096, 1, 0), (256, 512, 1, 1)])
+SHAPES = [(128, 128, 0, 0), (256, 1024, 0, 1), (128, 128, 1, 1), (256, 256, 2, 0), (128, 4096, 1, 0), (256, 512, 1, 1)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
 def test_batch_launch_shape_does_not_change_results(vxl, shape):
+    """A small batch: several lanes per particle, whose shape follows the tile."""
     specs = _specs()
     ref = vxl.Batch(specs)
     alt = vxl.Batch(specs)
@@ -74,6 +77,32 @@ def test_batch_launch_shape_does_not_change_results(vxl, shape):
         a, _ = ref.read_state(q)
         b, _ = alt.read_state(q)
         _assert_same(a, b, f"scene {q}")
+
+
+@pytest.mark.parametrize("walls", [False, True])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_large_batch_launch_shape_does_not_change_results(vxl, shape, walls):
+    """The same scenes beside one that brings every pass to one lane per particle (over 36,000 fluid and 20,000
+    boundary particles), where block and waves choose the kernels and their grids; with provider walls the
+    variant with mirror ghosts. States and reactions of all scenes, bit for bit."""
+    from vxl_sph import scenes
+    specs = _specs()[:2] + [scenes.small_dam(n=(34, 34, 34), spacing=0.02, tank=(1.0, 0.9, 0.9), seed=15)]
+    assert specs[-1].n_fluid > 36000 and sum(s.n_boundary for s in specs) > 20000
+    ref = vxl.Batch(specs)
+    alt = vxl.Batch(specs)
+    alt.set_tuning(*shape)
+    if walls:
+        for b in (ref, alt):
+            b.set_providers([scenes.floor_provider(), scenes.box_obstacle((0.2, 0.05, 0.2), (0.08, 0.08, 0.08))], 0)
+            b.set_providers([scenes.floor_provider()], 2)
+    for t in range(2):
+        for (b1, f1, t1), (b2, f2, t2) in zip(ref.step_tick(DT_TICK), alt.step_tick(DT_TICK)):
+            assert b1 == b2 and f1.tobytes() == f2.tobytes() and t1.tobytes() == t2.tobytes(), (t, b1)
+    for q in range(len(specs)):
+        for a, b in zip(ref.read_state(q), alt.read_state(q)):
+            _assert_same(a, b, f"scene {q}")
+        for a, b in zip(ref.export_grid(q)[:3], alt.export_grid(q)[:3]):
+            assert np.array_equal(a, b), q
 
 
 def test_autotune_restores_state_and_keeps_results(vxl):

@@ -139,6 +139,21 @@ def test_pair_quotients_over_scales(vxl, oracle_mod, h, over):
     _run_both(vxl, oracle_mod, _custom(vxl, pos, vel=vel, h=h, spacing=s, boundary=b, **over), substeps=2)
 
 
+def test_reciprocals_and_quotients_on_the_device(tmp_path):
+    """recip_rn against 1 / b for every significand (it rests on rcp.approx being within 1 ulp), quot_rn against a / b
+    for every divisor's numerators nearest a rounding midpoint: every pair that the step could round wrongly."""
+    import subprocess
+    from pathlib import Path
+    from vxl_sph import build
+    exe = tmp_path / "quotients"
+    flags = [f for f in build.NVCC_FLAGS if f != "-shared"]
+    src = Path(__file__).resolve().parent / "c" / "quotients.cu"
+    subprocess.run([build.nvcc(), *flags, "-I", str(build.CSRC), "-o", str(exe), str(src)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert int(r.stdout.split()[3]) > 5e7, r.stdout
+
+
 def _edge_scenes(vxl):
     from vxl_sph import scenes
     rng = np.random.default_rng(17)

@@ -70,7 +70,7 @@ def test_filter_keeps_every_neighbour(bins, shift, span):
 @pytest.mark.parametrize("max_bins,shift", [(0, 0.0), (0, 300.0), (900, -2.0), (120, 0.0), (20, 50.0), (1, 0.0)])
 def test_density_walk_bit_exact_over_bin_sizes(vxl, oracle_mod, max_bins, shift):
     """A ragged cloud (dense core, sparse rim, walls through it) at bins of h, 2h, 4h, ... one cell,
-    near and far from the origin: rows past the window queue, windows cut at every word offset."""
+    near and far from the origin: windows cut at every word offset, with eight lanes per particle."""
     from vxl_sph import scenes
     from test_gpu_parity import _custom, _run_both
     rng = np.random.default_rng(max_bins + 5)
@@ -101,3 +101,58 @@ def test_density_walk_batch_of_bin_sizes(vxl):
             assert a.tobytes() == b.tobytes(), q
         for a, b in zip(bat.export_grid(q)[:3], g.export_grid()[:3]):
             assert np.array_equal(a, b), q
+
+
+def _cloud(vxl, name):
+    """Small scenes for the one-lane walk: name, rows with more windows than its queue of 18."""
+    from vxl_sph import scenes
+    from test_gpu_parity import _custom
+    rng = np.random.default_rng(12)
+    if name.startswith("lattice"):  # in random order in one cell or eight: some 38 windows of a row hold a few kept slots each
+        pos = scenes.jitter(scenes.fluid_block((0.0, 0.0, 0.0), (16, 16, 16), 0.05), 0.05, 3, 0.2)
+        return _custom(vxl, pos[rng.permutation(len(pos))], max_bins=int(name.split()[1]))
+    pos = np.concatenate([rng.uniform(0.26, 0.34, (2000, 3)), rng.uniform(0.0, 0.6, (700, 3))]).astype(F32)  # a crowded bin
+    b = scenes.body_particles([scenes.Body(0, (0.3, 0.05, 0.3), (0.25, -0.1, 0.25))], 0.05, 0.1, 1, 1000.0)
+    return _custom(vxl, pos, max_bins=int(name.split()[1]), boundary=b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("walls", [False, True])
+@pytest.mark.parametrize("cloud", ["lattice 1", "lattice 8", "crowd 0", "crowd 60", "crowd 1"])
+def test_one_lane_walk_past_its_queue(vxl, oracle_mod, cloud, walls):
+    """Rows of well over 18 windows of 32 slots (the queue is emptied in mid-row) at bins of h, 2h and more, beside a
+    block that brings the density pass to one lane per particle: table, state, density and lists bit for bit."""
+    import ctypes
+    from vxl_sph import scenes
+    from test_gpu_parity import _custom, assert_bits, f32_dt
+    spec = _cloud(vxl, cloud)
+    n = spec.n_total
+    g = vxl.Batch([spec, _custom(vxl, scenes.fluid_block((0.0, 0.0, 0.0), (34, 34, 34), 0.05))])
+    o = oracle_mod.OracleSystem.from_scene(spec, threads=8)
+    if walls:
+        for x in (g, o):
+            x.set_providers([scenes.floor_provider(), scenes.box_obstacle((0.1, 0.0, 0.1), (0.08, 0.05, 0.08))])
+    dt = f32_dt(400)
+    g.substep(dt)
+    o.substep(dt)
+    r, og = o.read_f32(), o.grid()
+    dens = np.empty(n, F32)
+    assert g.lib.vxl_sph_read_fields_scene(g._h, 0, vxl._fptr(dens), None, None, None, None) == vxl.OK
+    assert_bits(dens, r["dens"], "density")
+    items, start, _, info = g.export_grid(0)
+    assert list(info.dims) == list(og["dims"]) and np.array_equal(start, og["start"]) and np.array_equal(items, og["items"])
+    row = np.diff(start.astype(np.int64)).reshape(tuple(info.dims)).sum(0).max()
+    assert row > 18 * 32 * 1.5, row
+    p, v = g.read_state(0)
+    assert_bits(p, r["pos"], "pos")
+    assert_bits(v, r["vel"], "vel")
+    g.substep(dt)
+    off, tot = np.empty(n + 1, np.uint64), ctypes.c_uint64()
+    op = off.ctypes.data_as(ctypes.POINTER(ctypes.c_uint64))
+    assert g.lib.vxl_sph_export_neighbors(g._h, op, n + 1, None, 0, ctypes.byref(tot)) == vxl.OK
+    ent = np.empty(tot.value, np.uint32)
+    assert g.lib.vxl_sph_export_neighbors(g._h, op, n + 1, vxl._u32ptr(ent), tot.value, ctypes.byref(tot)) == vxl.OK
+    oo, oe = o.neighbors()
+    assert np.array_equal(off, oo) and np.array_equal(ent, oe)
+    if cloud.startswith("lattice"):
+        assert np.median(np.diff(oo.astype(np.int64))) <= 64  # lists that are recorded, not walked again
