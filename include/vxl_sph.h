@@ -516,8 +516,8 @@ vxl_status vxl_sph_serve_tick_times(vxl_sph_server* s, uint64_t id, double* out_
  * its stream), so no call may be made inside stream capture. Every call reuses the same
  * array (the counts it needs zeroed are cleared at the start of each call), so calls
  * that overlap on the GPU — from two streams or two host threads — race and must not be
- * made. Cells of any size are sorted in bounded time (warp, shared-memory rank, or a
- * bitmap of the particle indices for cells above 2,048 entries). */
+ * made. Cells of any size are sorted in bounded time (up to 2,048 entries each entry is
+ * ranked against its cell's, larger cells through a bitmap of the particle indices). */
 vxl_status vxl_sph_build_grid_static(const float* d_pos_xyz, uint32_t n, float h, uint32_t max_bins,
                                      uint32_t* d_items, uint32_t* d_start, uint64_t start_cap,
                                      vxl_sph_grid_info* info, void* cuda_stream);

@@ -113,9 +113,13 @@ __device__ __forceinline__ uint32_t sub_word(int bx, int by, int bz) {
 // elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990; also
 // Muller et al., Handbook of Floating-Point Arithmetic, division by Newton-Raphson), so a
 // denominator's reciprocal is formed once and each quotient by it takes three instructions. One
-// Newton step from an approximation within 1 ulp (rcp.approx) rounds 1 / b correctly unless
-// b's significand is all ones. That case and operands whose quotient or residual could leave
-// the normal range are the caller's to keep out (scene_safe, pair_safe).
+// Newton step from an approximation within 1 ulp (the documented bound of rcp.approx; from within 1.5
+// ulp 19 significands come out wrong) rounds 1 / b correctly unless b's significand is all ones. Where a's
+// significand lies below b's, q is only within 1.5 ulp and the theorem does not apply as it stands; but
+// the step can then round wrongly only quotients within 4 parts in 2^48 b of a rounding midpoint, and
+// tests/c/quotients.cu tries all of those for every b, and every reciprocal, on the device. The
+// all-ones case and operands whose quotient or residual could leave the normal range are the caller's
+// to keep out (scene_safe, pair_safe).
 __device__ __forceinline__ float recip_rn(float b) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));

@@ -1272,7 +1272,7 @@ vxl_status Engine::stage_spans() {
       sp.push_back(SpanDev{s.body, s.origin[0], s.origin[1], s.origin[2], gs, ge, rigid, scenes_[q].base + scenes_[q].nf,
                            bword});
       span_scene_.push_back(q);
-      if (ge - gs > kReactExactSpan) ch.push_back(LongSpan{idx, gs, ge, 0u});  // a block of its own
+      if (ge - gs > kReactExactSpan) ch.push_back(LongSpan{idx});  // a block of its own
     }
     bword += (scenes_[q].nb + kBoundaryTile - 1) / kBoundaryTile * (kBoundaryTile / 32);
   }

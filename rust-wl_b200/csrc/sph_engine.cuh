@@ -33,10 +33,9 @@
 #include "sph_device.cuh"
 
 // Resident threads per SM the density and force passes are compiled for (register
-// budget = 65536 / this). Force at 1024 / 1280 / 1536: 0.279 / 0.310 / 0.436 ms on the 1M dam
-// break, 2.5 / 2.7 / 3.8 ms on the 10M one (1024 does not spill). Density at 768 / 1024 / 1280: 0.352 / 0.291 / 0.288 ms on the 1M dam
-// break, 5.0 / 4.2 / 4.1 ms on the 10M one with queues of 12 windows (below), and 1280 has no
-// room for longer ones.
+// budget = 65536 / this). Force at 1280 / 1536 instead of 1024 (which does not spill) is 11% / 56%
+// slower on the 1M dam break, 8% / 52% on the 10M one. Density at 768 is 20% slower than at 1024; at 1280 it was
+// 1-2% faster with queues of 12 windows (kWalkQueue), but that has no room for longer ones.
 #ifndef VXL_DENSITY_THREADS_PER_SM
 #define VXL_DENSITY_THREADS_PER_SM 1024
 #endif
@@ -101,7 +100,7 @@ struct SpanDev {
 };
 
 struct LongSpan {  // a span above kReactExactSpan, summed by a block of its own
-  uint32_t span, begin, end, pad;
+  uint32_t span;
 };
 
 // Spans of at most this many particles (bodies) are summed by one warp each; larger ones
@@ -170,8 +169,8 @@ constexpr int kScanTile = 2048;
 constexpr int kScanThreads = 256;
 constexpr int kBGatherCap = 64;
 // Density walk: windows queued per thread. h-sized bins need 9 or 10 (a row each), 2h bins
-// about 20. 12 / 14 / 18 / 22 on the 10M dam break: 4.20 / 4.03 / 3.81 / 3.90 ms (shorter queues are
-// emptied more often, longer ones leave less L1); the 1M one 0.29 ms with each.
+// about 20. On the 10M dam break 12 / 14 / 22 are 10% / 6% / 2% slower than 18 (shorter queues are
+// emptied more often, longer ones leave less L1), on the 1M one all are the same.
 #ifndef VXL_WALK_QUEUE
 #define VXL_WALK_QUEUE 18
 #endif
@@ -334,10 +333,6 @@ __global__ void k_e_box_empty(SceneDev* __restrict__ S, int fluid, int boundary)
   if (a < 6 && boundary) S->bbox[a] = a < 3 ? 0xffffffffu : 0u;
 }
 
-// Move whole scenes to new bases (the served form's repack): slot ranges are copied into
-// the second buffer set, reference indices shifted by the move. from_base/to_base/count
-// per moved scene; one block row per scene (blockIdx.y).
-
 // set_boundary_particles on the device (crates/vxl-phys-fluid/src/fluid_step.rs:13-53): for
 // boundary particle k of a scene (reference order), with body-frame lattice point L and
 // its body's pose, world position p = body.pos + rotate(q, L) (Quat::rotate_vec3:
@@ -390,6 +385,9 @@ __global__ void k_e_body_rebuild(const float4* __restrict__ blocal, const Pose* 
   block_bbox_accumulate(bbox_acc, x, y, z, valid);
 }
 
+// Move whole scenes to new bases (the served form's repack): slot ranges are copied into
+// the second buffer set, reference indices shifted by the move. from_base/to_base/count
+// per moved scene; one block row per scene (blockIdx.y).
 __global__ void k_e_move(const float4* __restrict__ pos_in, const float4* __restrict__ vel_in,
                          const uint32_t* __restrict__ orig_in, const float4* __restrict__ bpos_in,
                          float4* __restrict__ pos_out, float4* __restrict__ vel_out, uint32_t* __restrict__ orig_out,
@@ -772,15 +770,14 @@ __device__ __forceinline__ ListRows list_rows(const GridBox& g, const uint32_t* 
 // (padded by 32 past the last slot), tested eight per step; what is left comes out a window at a
 // time, push(m, base, dy, dz): bit 31 - t of m (not 0) is slot base + t of row (dy, dz);
 // the first is found by one leading-zero count (find-first-set is two instructions of the
-// 16-lane unit: density 0.295 vs 0.27 ms on the 1M dam break).
+// 16-lane unit: 7% of the density pass on the 1M dam break).
 // Called by whole warps (`active`: this lane walks); row() follows each row, converged.
 // A candidate costs a dp4a and a funnel shift (39 pairs per clock and SM) instead of a 16-byte
 // gather and eight float operations; what binds the walk is its work per row, which is why
-// the rows are runs of slots and the words are kept per residue. Density pass, before (cells
-// one by one, every candidate gathered and tested exactly) and after: 0.475 -> 0.295 ms on the
-// 1M dam break (h-sized bins), 0.84 -> 0.58 ms on a 1.4M pool and 5.5 -> 3.8 ms on the 10M one
-// (2h bins), 75 -> 36 us at 16k particles. With the words of one frame per cell, 27 cells and a
-// window each, 0.43 / 0.65 / 4.2 ms.
+// the rows are runs of slots and the words are kept per residue: with one frame's words per
+// cell, 27 cells and a window each, the pass takes 10% (2h bins) to 45% (h-sized bins) longer. Density
+// pass with the cells one by one, every candidate gathered and tested exactly, and now: 0.475 -> 0.254 ms on the
+// 1M dam break (h-sized bins), 0.84 -> 0.53 ms on a 1.4M pool and 5.5 -> 3.45 ms on the 10M one (2h bins).
 template <class P, class R>
 __device__ __forceinline__ void walk27_q(const GridBox& g, const uint32_t* __restrict__ start,
                                          const uint32_t* __restrict__ words, float px, float py, float pz, uint32_t cx,
@@ -1027,7 +1024,7 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
   // length instead of waiting for one another in every window.
   __shared__ uint2 s_win[kWalkQueue][kBlock];
   // First slots of the particle's list planes (list_planes): read once a window, and three
-  // registers less in both loops (272 -> 253 us on the 1M dam break, 3.56 -> 3.44 ms on the 10M one).
+  // registers less in both loops (7% of the pass on the 1M dam break, 3% on the 10M one).
   __shared__ uint32_t s_plane[3][kBlock];
   for (uint32_t t = first_tile(&ctl->work[kWorkDensity], ntiles); t < ntiles; t = following_tile(&ctl->work[kWorkDensity], ntiles)) {
     const TileDev td = tiles[t];
@@ -1090,19 +1087,17 @@ __global__ void __launch_bounds__(kBlock, VXL_DENSITY_THREADS_PER_SM / kBlock) k
             if (fluid_i) {
               if (pj.w > 0.0f) sum += w;
               else sum_b += (-pj.w) * w;
-              if (kWalls) {
-                for (uint32_t q = 0; q < np; ++q) {
-                  const float qx = pi.x - dx, qy = pi.y - dy, qz = pi.z - dz;  // pj = pi - d
-                  const float dn = (qx - wpt[3 * q]) * wn[3 * q] + (qy - wpt[3 * q + 1]) * wn[3 * q + 1] +
-                                   (qz - wpt[3 * q + 2]) * wn[3 * q + 2];
-                  const float t2 = 2.0f * dn;
-                  const float ex = pi.x - (qx - wn[3 * q] * t2), ey = pi.y - (qy - wn[3 * q + 1] * t2),
-                              ez = pi.z - (qz - wn[3 * q + 2] * t2);
-                  const float rg2 = ex * ex + ey * ey + ez * ez;
-                  if (rg2 <= h2) {
-                    const float tg = h2 - rg2;
-                    sum += k6 * tg * tg * tg;
-                  }
+              for (uint32_t q = 0; q < np; ++q) {
+                const float qx = pi.x - dx, qy = pi.y - dy, qz = pi.z - dz;  // pj = pi - d
+                const float dn = (qx - wpt[3 * q]) * wn[3 * q] + (qy - wpt[3 * q + 1]) * wn[3 * q + 1] +
+                                 (qz - wpt[3 * q + 2]) * wn[3 * q + 2];
+                const float t2 = 2.0f * dn;
+                const float ex = pi.x - (qx - wn[3 * q] * t2), ey = pi.y - (qy - wn[3 * q + 1] * t2),
+                            ez = pi.z - (qz - wn[3 * q + 2] * t2);
+                const float rg2 = ex * ex + ey * ey + ez * ez;
+                if (rg2 <= h2) {
+                  const float tg = h2 - rg2;
+                  sum += k6 * tg * tg * tg;
                 }
               }
             } else if (pj.w > 0.0f) {

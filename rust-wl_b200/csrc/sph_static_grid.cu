@@ -241,7 +241,7 @@ __global__ void ks_place(const uint2* __restrict__ cellrank, const uint32_t* __r
 // The placed indices of each cell of at most kWideRank entries in ascending order, into
 // items: a thread per entry ranks it against its cell's entries (the lanes of a cell read the
 // same ones). A warp per cell, and a pass of blocks over all cells for those above 32 entries,
-// took most of a call's 182 us at 430k particles; it takes 79 now (62 -> 54 at 125: launches).
+// took most of a call's 182 us at 430k particles; a call takes 76 now (62 -> 54 at 125: launches).
 __global__ void __launch_bounds__(256) ks_canon(const uint32_t* __restrict__ tmp, const uint2* __restrict__ cellrank,
                                                 const uint32_t* __restrict__ start, uint32_t n,
                                                 uint32_t* __restrict__ items) {
