@@ -5,7 +5,7 @@ read) are exported through vxl_sph_export_neighbors and compared, entry for entr
 order, with the oracle's UniformGrid::for_neighbors_in walk
 (crates/vxl-phys-fluid/src/grid.rs:115-155) over the same positions: all neighbours of a
 fluid particle, the fluid ones of a boundary particle (fluid_density.rs:59-69). Cases: the
-16k dam break at h-sized bins, a doubled-bin tank (2h cells, half-cell culling), lists
+16k dam break at h-sized bins, a doubled-bin tank (2h cells), lists
 longer than the 64 recorded entries (walked again), and a flowing state after a few ticks.
 
 The 10M configuration (9,938,375 fluid particles in the 2.5 x 1.2 x 1.2 m tank, Akinci
@@ -43,7 +43,7 @@ def _compare_lists(g, o, label):
     return go, ge
 
 
-DENSITY = [0, 1]  # density kernels: per-particle walk, grouped segments
+DENSITY = [0, 1]  # the tuning's density: both accepted values run the one density pass
 
 
 def _lists_after(vxl, oracle_mod, spec, warm_ticks=0, substeps_before=0, density=0):
@@ -87,7 +87,7 @@ def test_neighbor_lists_flowing_state(vxl, oracle_mod, density):
 @pytest.mark.parametrize("density", DENSITY)
 def test_neighbor_lists_doubled_bins(vxl, oracle_mod, density):
     """The 10M tank's grid rule with a 40^3 block: the budget doubles the bins to 2h, so the
-    density pass culls half-cells and orders or groups particles by octant."""
+    density pass takes a cell's particles by octant."""
     from vxl_sph import scenes
     spec = scenes.dam10m_block(40)
     g, o = _lists_after(vxl, oracle_mod, spec, density=density)
@@ -199,7 +199,7 @@ def test_neighbor_lists_before_any_substep_is_not_ready(vxl):
 def test_dam10m_substep_bit_exact(vxl, oracle_mod):
     """The 10M configuration, one substep from identical state (doubled bins, walls, 64
     boxes, the configuration's constants): every per-particle quantity bit for bit, with
-    either density kernel."""
+    either value of the tuning's density."""
     from vxl_sph import scenes
     spec = scenes.dam10m()
     assert spec.n_fluid == 9938375 and len(spec.spans) == 69
@@ -215,13 +215,13 @@ def test_dam10m_substep_bit_exact(vxl, oracle_mod):
         g.substep(dt)
         _, _, _, info = g.export_grid()
         assert info.bin >= 2 * spec.params.smoothing_radius * 0.999, "the cell budget doubles the bins"
-        compare_grid(g, o, f"dam10m density kernel {density}")
+        compare_grid(g, o, f"dam10m density {density}")
         dens, press, acc, xsph, bf = g.read_fields()
         assert_bits(dens, r["dens"], "density")
         assert_bits(press, r["press"], "pressure")
         assert_bits(acc[:nf], r["acc"][:nf], "acceleration")
         assert_bits(xsph[:nf], r["xsph"][:nf], "xsph")
         assert_bits(bf, r["bforce"][nf:], "boundary reaction per particle")
-        compare_state(g, o, f"dam10m after one substep, density kernel {density}")
+        compare_state(g, o, f"dam10m after one substep, density {density}")
         g.close()
     o.close()

@@ -77,8 +77,8 @@ def test_backend_available(vxl):
 
 @pytest.mark.parametrize("density", [0, 1])
 def test_single_substep_bit_exact(vxl, oracle_mod, density):
-    """One substep from identical state: table, rho, p, a, xsph, bforce, pos, vel (with each
-    density kernel)."""
+    """One substep from identical state: table, rho, p, a, xsph, bforce, pos, vel (with either
+    value of the tuning's density)."""
     from vxl_sph import scenes
     spec = scenes.small_dam(n=(10, 12, 9), spacing=0.05, tank=(0.8, 0.7, 0.6))
     g, o = pair(vxl, oracle_mod, spec)
@@ -144,8 +144,7 @@ def test_published_hash_through_gpu(vxl, oracle_mod, case):
     """The reference's grid-probe scene run on the GPU: 5 + 1 ticks of the default
     config, then the FNV hash of the table of the last substep equals the published
     CPU hash (crates/vxl-phys-gpu/examples/gpu_grid_probe.rs:181-226) — for every published
-    case, up to the 9,938,375-particle lattice, whose 2^20 cell budget doubles the bins (the
-    half-culled density walk at full size)."""
+    case, up to the 9,938,375-particle lattice, whose 2^20 cell budget doubles the bins."""
     n = case["n"]
     s = F32(0.05)
     nf = F32(n)
@@ -231,29 +230,62 @@ def _custom(vxl, pos, vel=None, h=0.1, spacing=0.05, max_bins=0, boundary=None, 
     return scenes.SceneSpec("custom", p, pos, vel, pm, nf, spans, spacing, 1)
 
 
+_FILLER = []
+
+
+class _OneLane:
+    """Scene 0 of a batch whose other scene (39,304 fluid and 25,788 boundary particles) brings every pass to one
+    lane per particle; alone, the small scenes of these tests have eight."""
+
+    def __init__(self, vxl, spec):
+        from vxl_sph import scenes
+        if not _FILLER:
+            _FILLER.append(scenes.small_dam(n=(34, 34, 34), spacing=0.02, tank=(1.0, 0.9, 0.9), seed=15))
+        self.vxl, self.spec, self.batch = vxl, spec, vxl.Batch([spec, _FILLER[0]])
+        self.lib, self.h = self.batch.lib, self.batch._h
+
+    def set_record(self, on):
+        assert self.lib.vxl_sph_set_record(self.h, int(on)) == self.vxl.OK
+
+    def substep(self, dt):
+        self.batch.substep(dt)
+
+    def export_grid(self):
+        return self.batch.export_grid(0)
+
+    def read_state(self):
+        return self.batch.read_state(0)
+
+    def read_fields(self):
+        n, nb = self.spec.n_total, self.spec.n_boundary
+        out = [np.zeros(n, F32), np.zeros(n, F32), np.zeros((n, 3), F32), np.zeros((n, 3), F32), np.zeros((nb, 3), F32)]
+        assert self.lib.vxl_sph_read_fields_scene(self.h, 0, *(self.vxl._fptr(a) if a.size else None for a in out)) == self.vxl.OK
+        return out
+
+
 def _run_both(vxl, oracle_mod, spec, substeps=1):
-    """The oracle and the GPU with each density kernel (per-particle walk, grouped segments)
-    from identical state, `substeps` substeps, everything bit for bit."""
+    """The oracle and the GPU, with one lane per particle and with several, from identical state, `substeps`
+    substeps, everything bit for bit."""
     o = oracle_mod.OracleSystem.from_scene(spec, threads=8)
     dt = f32_dt(4)
     for _ in range(substeps):
         o.substep(dt)
     r = o.read_f32()
     nf = spec.n_fluid
-    for density in (0, 1):
-        g = vxl.Scene(spec.params, spec.pos, spec.vel, spec.pmass, spec.n_fluid)
-        g.set_tuning(256, 256, 0, density)
+    for lanes in ("one lane", "several lanes"):
+        g = (_OneLane(vxl, spec) if lanes == "one lane" else
+             vxl.Scene(spec.params, spec.pos, spec.vel, spec.pmass, spec.n_fluid))
         g.set_record(True)
         for _ in range(substeps):
             g.substep(dt)
-        compare_grid(g, o, f"density kernel {density}")
+        compare_grid(g, o, lanes)
         dens, press, acc, xsph, bf = g.read_fields()
-        assert_bits(dens, r["dens"], f"density (kernel {density})")
-        assert_bits(acc[:nf], r["acc"][:nf], f"acc (kernel {density})")
-        assert_bits(xsph[:nf], r["xsph"][:nf], f"xsph (kernel {density})")
+        assert_bits(dens, r["dens"], f"density ({lanes})")
+        assert_bits(acc[:nf], r["acc"][:nf], f"acc ({lanes})")
+        assert_bits(xsph[:nf], r["xsph"][:nf], f"xsph ({lanes})")
         if spec.n_boundary:
-            assert_bits(bf, r["bforce"][nf:], f"bforce (kernel {density})")
-        compare_state(g, o, f"density kernel {density}")
+            assert_bits(bf, r["bforce"][nf:], f"bforce ({lanes})")
+        compare_state(g, o, lanes)
     return g, o
 
 
@@ -262,8 +294,7 @@ def test_single_particle(vxl, oracle_mod):
 
 
 def test_one_crowded_cell_canon_paths(vxl, oracle_mod):
-    """Cells of > 32, > 512 and > 1024 particles take the shared-memory sort paths (keys and
-    source slots staged; keys only) and the global one."""
+    """One cell of 200, 800 and 1,500 particles: every entry is ranked against its cell's."""
     rng = np.random.default_rng(7)
     for n in (200, 800, 1500):
         pos = rng.uniform(0.0, 0.08, (n, 3)).astype(F32)
@@ -290,7 +321,7 @@ def test_clamped_edge_cell_with_doubled_bins(vxl, oracle_mod):
     """A 1 km long scene at h = 0.01: the budget quadruples the bin to 0.04 and the x axis
     still hits the 16,384-cell cap, so every particle beyond x = 655.32 is clamped into the
     last x cell. Two clusters there (x = 900 and x = 1000) find their neighbours in that
-    cell — the half-cell culling must not treat its upper face as a wall."""
+    cell — the walk must not treat its upper face as a wall."""
     from vxl_sph import scenes
     s = 0.005
     blocks = [scenes.fluid_block(o, (4, 4, 4), s) for o in ((0.0, 0.0, 0.0), (900.0, 0.1, 0.1),
@@ -408,7 +439,7 @@ def test_dam1_table_properties_and_determinism(vxl):
 
 def test_doubled_bins_many_per_cell(vxl, oracle_mod):
     """A cell budget that forces bins of 4h with ~500 particles per cell: the density pass
-    culls half-cells out of reach and must still accept the same neighbours in the same
+    filters out most candidates and must still accept the same neighbours in the same
     order (table, fields and state bit for bit over six substeps)."""
     from vxl_sph import scenes
     s = 0.01
@@ -631,9 +662,8 @@ def test_deferred_readback_and_vxld_dump(vxl, oracle_mod, tmp_path):
 
 
 def test_canon_window_at_its_limit(vxl, oracle_mod):
-    """Sixteen particles per cell (two interleaved lattices at spacing h/2): 32 consecutive
-    cells hold exactly 512 entries, the limit of the sort's window path, and cells at the
-    block's edges fall back to the per-cell path; the table, fields and state stay bit-exact."""
+    """Sixteen particles per cell (two interleaved lattices at spacing h/2), fewer at the block's
+    edges: the table, fields and state stay bit-exact."""
     from vxl_sph import scenes
     s = 0.025
     a = scenes.fluid_block((0.0, 0.0, 0.0), (12, 10, 32), s)

@@ -182,8 +182,8 @@ def test_coupled_loop_with_provider_floor(vxl, oracle_mod):
 
 
 def test_provider_walls_at_doubled_bins(vxl, oracle_mod):
-    """Provider walls with a cell budget that doubles the bins (the half-culled density walk
-    with mirror ghosts, and the x-half thread order): bitwise with the oracle."""
+    """Provider walls with a cell budget that doubles the bins (the filtered density walk
+    with mirror ghosts, in octant order): bitwise with the oracle."""
     from vxl_sph import scenes
     pos = scenes.jitter(scenes.fluid_block((-0.3, 0.05, -0.2), (12, 10, 8), 0.05), 0.05, 5)
     spec = _custom(vxl, pos, h=0.1, spacing=0.05, max_bins=64, xsph_viscosity=0.05)
