@@ -1111,7 +1111,7 @@ vxl_status Engine::read_fields(uint32_t q, float* dens, float* press, float* acc
   k_e_read_fields<<<blocks_for(n), kThreads, 0, stream_>>>((const float2*)rc_, press_, (const float4*)acc_,
                                                             (const float4*)xsph_, orig_, dens ? d_d : nullptr,
                                                             press ? d_p : nullptr, acc ? d_a : nullptr,
-                                                            xsph ? d_x : nullptr, si.base, n);
+                                                            xsph ? d_x : nullptr, si.base, n, si.nf);
   if (dens) CU(cudaMemcpyAsync(dens, d_d, (size_t)n * 4, cudaMemcpyDeviceToHost, stream_));
   if (press) CU(cudaMemcpyAsync(press, d_p, (size_t)n * 4, cudaMemcpyDeviceToHost, stream_));
   if (acc) CU(cudaMemcpyAsync(acc, d_a, (size_t)n * 12, cudaMemcpyDeviceToHost, stream_));

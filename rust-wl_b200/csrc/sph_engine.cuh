@@ -2629,7 +2629,7 @@ __global__ void k_e_read_scene(const float4* __restrict__ pos, const float4* __r
 __global__ void k_e_read_fields(const float2* __restrict__ rc, const float* __restrict__ press,
                                 const float4* __restrict__ acc, const float4* __restrict__ xsph,
                                 const uint32_t* __restrict__ orig, float* __restrict__ dout, float* __restrict__ pout,
-                                float* __restrict__ aout, float* __restrict__ xout, uint32_t base, uint32_t n) {
+                                float* __restrict__ aout, float* __restrict__ xout, uint32_t base, uint32_t n, uint32_t nf) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t s = base + i;
@@ -2637,13 +2637,13 @@ __global__ void k_e_read_fields(const float2* __restrict__ rc, const float* __re
   if (dout) dout[o] = rc[s].x;
   if (pout) pout[o] = press[s];
   if (aout) {
-    const float4 a = acc[s];
+    const float4 a = o < nf ? acc[s] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // the force pass records fluid slots only
     aout[3 * o] = a.x;
     aout[3 * o + 1] = a.y;
     aout[3 * o + 2] = a.z;
   }
   if (xout) {
-    const float4 x = xsph[s];
+    const float4 x = o < nf ? xsph[s] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     xout[3 * o] = x.x;
     xout[3 * o + 1] = x.y;
     xout[3 * o + 2] = x.z;

@@ -289,6 +289,23 @@ def _run_both(vxl, oracle_mod, spec, substeps=1):
     return g, o
 
 
+def test_recorded_fields_of_boundary_particles_are_zero(vxl, oracle_mod):
+    """Accelerations and XSPH sums of boundary particles are zero (the reference's), whatever fluid held their slots
+    in earlier substeps."""
+    from vxl_sph import scenes
+    spec = scenes.small_dam(n=(10, 12, 9), spacing=0.05, tank=(0.8, 0.7, 0.6))
+    g, o = pair(vxl, oracle_mod, spec)
+    g.set_record(True)
+    for _ in range(3):
+        g.step_tick(1.0 / 60.0, spec.spans)
+        o.step(float(F32(1.0) / F32(60.0)))
+    r = o.read_f32()
+    _, _, acc, xsph, _ = g.read_fields()
+    assert_bits(acc, r["acc"], "acc")
+    assert_bits(xsph, r["xsph"], "xsph")
+    assert not np.any(acc[spec.n_fluid:]) and not np.any(xsph[spec.n_fluid:])
+
+
 def test_single_particle(vxl, oracle_mod):
     _run_both(vxl, oracle_mod, _custom(vxl, [[0.1, 0.2, 0.3]]), substeps=5)
 
