@@ -23,7 +23,7 @@ struct GridBox {
   uint32_t nx, ny, nz;
   uint32_t total;
   uint32_t reach_q;  // candidate filter: the squared reach in cell units of 1/64 bin (sub_word below)
-  uint32_t rows;     // neighbour-list entries by rows (list_by_rows)
+  uint32_t rows;     // neighbour-list entries by rows (k_e_groups)
   uint32_t pad;
 };
 

@@ -1442,10 +1442,7 @@ void Engine::enqueue_substep(bool with_reactions) {
   // grids, cell table, sorted buffer, permutation, lists, work counters): join it first.
   // Its reaction sums read only bforce / bpos and go on beside this substep.
   join_side_only();
-  static_assert(kTeamForce.four >= kTeamDensity.four, "rows: one lane in the force pass means one lane in the density pass");
-  const bool rows = team_lanes(load, kTeamForce) == 1;
-  LAUNCH(KID_CELLOFF, k_e_celloff<<<1, S <= 32 ? 32 : kCelloffThreads, 0, st>>>(sc_d_, S, ctl_d_, (uint32_t)cell_cap_,
-                                                                                                 rows));
+  LAUNCH(KID_CELLOFF, k_e_celloff<<<1, S <= 32 ? 32 : kCelloffThreads, 0, st>>>(sc_d_, S, ctl_d_, (uint32_t)cell_cap_));
   LAUNCH(KID_KEYS, k_e_keys<<<key_blocks, kThreads, 0, st>>>(p0, sc_d_, tiles_d_, ntiles_, ctl_d_, counts_,
                                                              (uint2*)cellrank_, wet_));
   LAUNCH(KID_SCAN, k_e_scan<<<148 * 4, kScanThreads, 0, st>>>(counts_, ctl_d_, scan_, start_, scan_wait_));
@@ -1454,9 +1451,12 @@ void Engine::enqueue_substep(bool with_reactions) {
   LAUNCH(KID_CANON, k_e_canon<<<std::max<uint32_t>(blocks_for(used_), 1), 256, 0, st>>>(
                         (const uint2*)items_, order_, start_, (uint32_t)used_, ctl_d_, p0, v0, (float4*)pos_[1],
                         (float4*)vel_[1], orig_, slot_of_));
-  // the candidate-filter words, and at doubled bins the density pass's thread order
+  // the candidate-filter words, at doubled bins the density pass's thread order, and the scenes whose list
+  // entries go by rows (the team kernels of both passes, for a few ten thousand particles, know planes only)
+  static_assert(kTeamForce.four >= kTeamDensity.four, "one lane in the force pass means one lane in the density pass");
+  const bool rows = team_lanes(load, kTeamForce) == 1;
   LAUNCH(KID_GROUPS, k_e_groups<<<key_blocks, kGroupChunk, 0, st>>>(p1, sc_d_, tiles_d_, ntiles_, ctl_d_, order_, words_,
-                                                                    wstride_));
+                                                                    wstride_, rows ? start_ : nullptr));
   const uint32_t stride = (uint32_t)slot_cap_;
   const bool rec = record_;
   const uint32_t per_tile = std::max<uint32_t>(ntiles_, 1);

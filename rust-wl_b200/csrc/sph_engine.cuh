@@ -408,30 +408,16 @@ __global__ void k_e_slot_of(const uint32_t* __restrict__ orig, uint32_t* __restr
 
 // ---------------------------------------------------------------- substep kernels
 
-// Bits of a neighbour-list entry's distance, by planes and by rows (see "Compact neighbour-list entries").
-constexpr uint32_t kListOffBits = 14, kListRowBits = 12;
-constexpr uint32_t kListOffMask = (1u << kListOffBits) - 1u, kListRowMask = (1u << kListRowBits) - 1u;
-
-// Whether a scene's list entries go by rows: it has more slots than 14 bits hold, and two x rows
-// of cells over the fluid's length with three cells of a third, at rest density, do too (less a
-// window). Lists of a scene that is fuller than that fail one by one; one that is emptier pays
-// for loading the bases: a sixth of the force pass, a twentieth of the density pass.
-__device__ __forceinline__ bool list_by_rows(const SphConst& k, const GridBox& g, uint32_t count, float length) {
-  const float cells = 2.0f * fminf(length * g.inv, (float)g.nx) + 3.0f;
-  return count > kListOffMask && cells * (g.bin * g.bin * g.bin * k.rho0 / k.mass) > (float)(kListOffMask - 32u);
-}
-
 // Grid boxes and cell offsets (one block, any scene count): each scene's grid for this
 // substep (crates/vxl-phys-fluid/src/grid.rs:37-44 -> crates/vxl-phys-core/src/grid.rs:34-50)
 // from its AABB accumulators, which are then reset for the force pass's epilogue; then an
 // exclusive scan of the scenes' cell counts;
 // flags the substep when the total exceeds the cell capacity (every later kernel then
 // returns without touching memory).
-// A warp for up to 32 scenes, kCelloffThreads threads for more. rows: a scene's list
-// entries may go by rows (the team kernels of both passes, for a few ten thousand particles, know planes only).
+// A warp for up to 32 scenes, kCelloffThreads threads for more.
 constexpr uint32_t kCelloffThreads = 1024;
 __global__ void __launch_bounds__(kCelloffThreads) k_e_celloff(SceneDev* __restrict__ sc, uint32_t nscenes,
-                                                               EngineCtl* ctl, uint32_t cell_cap, bool rows) {
+                                                               EngineCtl* ctl, uint32_t cell_cap) {
   __shared__ uint32_t ws[32];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
   unsigned long long carry = 0;  // the same in every thread
@@ -452,7 +438,6 @@ __global__ void __launch_bounds__(kCelloffThreads) k_e_celloff(SceneDev* __restr
       GridBox g;
       if (!grid_box(lo[0], lo[1], lo[2], hi[0], hi[1], hi[2], s.k.h, s.k.max_bins, g))
         atomicOr(&ctl->err, kErrGridLoop);
-      g.rows = rows && list_by_rows(s.k, g, s.count, o2f(s.fbox[3]) - o2f(s.fbox[0]));
       s.g = g;
       s.cells = g.total;
       for (int a = 0; a < 3; ++a) {
@@ -722,14 +707,17 @@ __device__ __forceinline__ void walk27(const GridBox& g, const uint32_t* __restr
 // (max(cx - 1, 0), cy + dy, cz + dz); the rows of one z-plane dz follow one another. In most scenes
 // an entry is (dz + 1) << 14 | the slot's distance from the first slot of its plane's first row,
 // which spans two x rows of the grid: three bases decode it. Where two rows hold more than 14 bits
-// (scenes long in x; list_by_rows) it is (dz + 1) << 14 | (dy + 1) << 12 | the distance from the first slot
+// (scenes long in x; k_e_groups finds them) it is (dz + 1) << 14 | (dy + 1) << 12 | the distance from the first slot
 // of its own row, whose three cells hold 192 particles at rest at 2h bins; its base is loaded from
 // the cell table. A neighbour whose distance has more bits makes its list unusable (bit 31 of the
 // count): the consumers then walk the cells again. Tick of four substeps, 1.9M particles 1,200
 // long at 2h bins: 4.6 ms by rows (force 0.44 ms a substep), 16.4 with a z-plane's entries only (3.37).
-// By rows for every scene, with the nine bases in shared memory, density is 4% and force 3% slower
-// at all sizes, by the L1 cache they take.
+// A scene that could do with planes pays for loading the bases: a sixth of the force pass, a twentieth of
+// the density pass. By rows for every scene, with the nine bases in shared memory, density is 4% and
+// force 3% slower at all sizes, by the L1 cache they take.
 constexpr uint32_t kListBad = 0x80000000u;
+constexpr uint32_t kListOffBits = 14, kListRowBits = 12;
+constexpr uint32_t kListOffMask = (1u << kListOffBits) - 1u, kListRowMask = (1u << kListRowBits) - 1u;
 
 struct ListPlanes {
   uint32_t b0, b1, b2;  // first slot of plane cz - 1 (= b1 at the grid's edge), cz, cz + 1 (~0u if none)
@@ -839,6 +827,12 @@ __device__ __forceinline__ void walk27_q(const GridBox& g, const uint32_t* __res
 // one axis only (12 cells instead of 8; up to 27 for octants apart in all three). A chunk
 // holds 8 octant runs, 7 boundaries over kGroupChunk / 32 warps; chunks of 512 slots (tiles
 // of 512) let fewer warps straddle, but cost the grouping pass about as much as they save.
+//
+// It also finds the scenes whose lists go by rows (g.rows, zero before): the first slot of every eighth tile
+// looks up how many slots its own plane's entries span, and a span near the 14 bits marks the scene.
+// That is often enough: spans change little from cell to cell, a list that fails all the same is
+// walked again, and 512 slots less than the limit leave room for that. A slot of every warp cost 0.05 ms of the
+// 10M dam break's substep. (By the fluid's length and rest density a tank with splashes at both ends is full.)
 #ifndef VXL_GROUP_CHUNK
 #define VXL_GROUP_CHUNK 256
 #endif
@@ -847,10 +841,11 @@ static_assert(kGroupChunk % 128 == 0 && kGroupChunk <= 1024, "chunk: 128..1024 s
 
 __device__ __forceinline__ uint32_t octant_rank(uint32_t oct) { return oct ^ (oct >> 1) ^ (oct >> 2); }
 
-__global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restrict__ pos, const SceneDev* __restrict__ sc,
+__global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restrict__ pos, SceneDev* __restrict__ sc,
                                                           const TileDev* __restrict__ tiles, uint32_t ntiles,
                                                           const EngineCtl* __restrict__ ctl, uint32_t* __restrict__ order,
-                                                          uint32_t* __restrict__ words, uint32_t wstride) {
+                                                          uint32_t* __restrict__ words, uint32_t wstride,
+                                                          const uint32_t* __restrict__ start) {
   if (ctl->err & kErrCellCap) return;
   constexpr uint32_t kW = kGroupChunk / 32;  // warps
   constexpr uint32_t kV = 8 * kW / 32;       // (rank, warp) counts per lane of the scan
@@ -860,6 +855,7 @@ __global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restri
   // the block's chunks one after another, each one's positions loaded while the previous
   // one is sorted
   uint32_t t = blockIdx.x, c1 = 0;
+  uint32_t turn = blockIdx.x;  // tiles of this block, begun at its index: every block takes its eighth
   TileDev tn = t < ntiles ? tiles[t] : TileDev{};
   float4 pn = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (t < ntiles && threadIdx.x < tn.count) pn = pos[tn.first + threadIdx.x];
@@ -879,6 +875,7 @@ __global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restri
     const float hb = g.bin * 0.5f;
     const uint32_t i = threadIdx.x;
     const bool valid = i < min(kGroupChunk, td.count - c0);
+    if (c0 == 0) ++turn;
     uint32_t oct = 0;
     if (valid) {
       uint32_t cx, cy, cz;
@@ -890,6 +887,12 @@ __global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restri
       for (uint32_t q = 0; q < 3; ++q) {
         words[(size_t)q * wstride + td.first + c0 + i] = sub_word((int)(kSubUnits * side) + bx - 96, by, bz);
         side = side ? side - 1 : 2;
+      }
+      if (start && i == 0 && c0 == 0 && (turn & 7u) == 0 && !g.rows) {
+        const uint32_t* row = start + sc[td.scene].cell_off + cz * g.ny * g.nx;
+        const uint32_t first = row[(cy > 0 ? cy - 1 : 0) * g.nx + (cx > 0 ? cx - 1 : 0)];
+        const uint32_t end = row[min(cy + 1, g.ny - 1u) * g.nx + min(cx + 1, g.nx - 1u) + 1];
+        if (end - first > kListOffMask - 512u) sc[td.scene].g.rows = 1u;  // any number of writers, one value
       }
       if (half)
         oct = (p.x >= g.minx + (float)cx * g.bin + hb ? 1u : 0u) | (p.y >= g.miny + (float)cy * g.bin + hb ? 2u : 0u) |
