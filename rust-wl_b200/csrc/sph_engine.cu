@@ -1456,7 +1456,7 @@ void Engine::enqueue_substep(bool with_reactions) {
   static_assert(kTeamForce.four >= kTeamDensity.four, "one lane in the force pass means one lane in the density pass");
   const bool rows = team_lanes(load, kTeamForce) == 1;
   LAUNCH(KID_GROUPS, k_e_groups<<<key_blocks, kGroupChunk, 0, st>>>(p1, sc_d_, tiles_d_, ntiles_, ctl_d_, order_, words_,
-                                                                    wstride_, rows ? start_ : nullptr));
+                                                                    wstride_, rows ? start_ : nullptr, sc_d_));
   const uint32_t stride = (uint32_t)slot_cap_;
   const bool rec = record_;
   const uint32_t per_tile = std::max<uint32_t>(ntiles_, 1);

@@ -841,11 +841,11 @@ static_assert(kGroupChunk % 128 == 0 && kGroupChunk <= 1024, "chunk: 128..1024 s
 
 __device__ __forceinline__ uint32_t octant_rank(uint32_t oct) { return oct ^ (oct >> 1) ^ (oct >> 2); }
 
-__global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restrict__ pos, SceneDev* __restrict__ sc,
+__global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restrict__ pos, const SceneDev* __restrict__ sc,
                                                           const TileDev* __restrict__ tiles, uint32_t ntiles,
                                                           const EngineCtl* __restrict__ ctl, uint32_t* __restrict__ order,
                                                           uint32_t* __restrict__ words, uint32_t wstride,
-                                                          const uint32_t* __restrict__ start) {
+                                                          const uint32_t* __restrict__ start, SceneDev* mark) {
   if (ctl->err & kErrCellCap) return;
   constexpr uint32_t kW = kGroupChunk / 32;  // warps
   constexpr uint32_t kV = 8 * kW / 32;       // (rank, warp) counts per lane of the scan
@@ -888,11 +888,11 @@ __global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restri
         words[(size_t)q * wstride + td.first + c0 + i] = sub_word((int)(kSubUnits * side) + bx - 96, by, bz);
         side = side ? side - 1 : 2;
       }
-      if (start && i == 0 && c0 == 0 && (turn & 7u) == 0 && !g.rows) {
+      if (start && i == 0 && c0 == 0 && (turn & 7u) == 0) {
         const uint32_t* row = start + sc[td.scene].cell_off + cz * g.ny * g.nx;
         const uint32_t first = row[(cy > 0 ? cy - 1 : 0) * g.nx + (cx > 0 ? cx - 1 : 0)];
         const uint32_t end = row[min(cy + 1, g.ny - 1u) * g.nx + min(cx + 1, g.nx - 1u) + 1];
-        if (end - first > kListOffMask - 512u) sc[td.scene].g.rows = 1u;  // any number of writers, one value
+        if (end - first > kListOffMask - 512u) mark[td.scene].g.rows = 1u;  // any number of writers, one value; not read here
       }
       if (half)
         oct = (p.x >= g.minx + (float)cx * g.bin + hb ? 1u : 0u) | (p.y >= g.miny + (float)cy * g.bin + hb ? 2u : 0u) |
