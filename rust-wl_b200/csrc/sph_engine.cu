@@ -186,12 +186,11 @@ vxl_status Engine::alloc_all() {
   A(dalloc(&words_, 3ull * wstride_));
   A(dalloc(&bwet_, n / 32 + 4ull * scene_cap_ + 4));  // kBoundaryTile / 32 words per boundary tile
   A(dalloc(&stage_, 8 * n));
-  A(dalloc(&counts_, cell_cap_ + 1));
+  A(dalloc(&counts_, cell_cap_ + 1 + cell_cap_ / kExportTile + 1));  // and the tile sums of an export behind its cells
   A(dalloc(&wet_, cell_cap_ + 1));
   A(dalloc(&order_, slot_cap_));
   A(dalloc(&start_, cell_cap_ + 1));
   A(dalloc(&scan_, cell_cap_ / kScanTile + 2));
-  A(dalloc(&export_sums_, cell_cap_ / kExportTile + 2));
   A(dalloc(&sc_d_, scene_cap_));
   tiles_cap_ = (uint32_t)(n / 64 + 2ull * scene_cap_ + 2);  // particle tiles (>= 128 slots) + boundary tiles
   A(dalloc(&tiles_d_, tiles_cap_));
@@ -220,7 +219,7 @@ void Engine::free_all() {
   if (graph_) cudaGraphExecDestroy(graph_);
   graph_ = nullptr;
   void* d[] = {pos_[0], pos_[1], vel_[0], vel_[1], orig_, slot_of_, cellrank_, items_, rc_, press_, acc_, xsph_,
-               bforce_, bpos_, nbr_, nbr_n_, words_, bwet_, order_, stage_, counts_, wet_, start_, scan_, export_sums_, sc_d_, tiles_d_, ctl_d_, spans_d_,
+               bforce_, bpos_, nbr_, nbr_n_, words_, bwet_, order_, stage_, counts_, wet_, start_, scan_, sc_d_, tiles_d_, ctl_d_, spans_d_,
                longs_d_, breact_d_};
   for (void* p : d)
     if (p) cudaFree(p);
@@ -1157,8 +1156,9 @@ vxl_status Engine::export_grid(uint32_t q, uint32_t* items, uint32_t* start, uin
   uint32_t* d_items = (uint32_t*)stage_;
   uint32_t* d_bins = d_items + n;
   const uint32_t blocks = blocks_for(total + 1, kExportTile);
-  k_e_export_counts<<<blocks, kExportThreads, 0, stream_>>>(start_, sc_d_, q, ref_start, export_sums_);
-  k_e_export_table<<<blocks, kExportThreads, 0, stream_>>>(start_, orig_, sc_d_, q, ref_start, export_sums_,
+  uint32_t* sums = ref_start + total + 1;  // a word per tile
+  k_e_export_counts<<<blocks, kExportThreads, 0, stream_>>>(start_, sc_d_, q, ref_start, sums);
+  k_e_export_table<<<blocks, kExportThreads, 0, stream_>>>(start_, orig_, sc_d_, q, ref_start, sums,
                                                            items ? d_items : nullptr, bins ? d_bins : nullptr);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess && start)
@@ -1166,7 +1166,7 @@ vxl_status Engine::export_grid(uint32_t q, uint32_t* items, uint32_t* start, uin
   if (e == cudaSuccess && items && n) e = cudaMemcpyAsync(items, d_items, (size_t)n * 4, cudaMemcpyDeviceToHost, stream_);
   if (e == cudaSuccess && bins && n) e = cudaMemcpyAsync(bins, d_bins, (size_t)n * 4, cudaMemcpyDeviceToHost, stream_);
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
-  const cudaError_t z = cudaMemsetAsync(counts_, 0, (total + 1) * 4, stream_);  // the next substep is behind it
+  const cudaError_t z = cudaMemsetAsync(counts_, 0, (total + 1 + blocks) * 4, stream_);  // the next substep is behind it
   if (e == cudaSuccess) e = z;
   if (e != cudaSuccess) return set_error(VXL_CUDA_ERROR, std::string("export: ") + cudaGetErrorString(e));
   return VXL_OK;

@@ -2686,7 +2686,7 @@ __global__ void __launch_bounds__(kExportThreads) k_e_export_counts(const uint32
 
 // The tile's exclusive scan in place, from the sums of the tiles before it, and its cells'
 // particles. Tiles of 512 spread a small scene's cells over the SMs: 33k particles in 9k cells, a
-// call of 0.122 ms (0.144 with tiles of 2,048); 1.1M cells 0.60 ms, 1.86 when one block scanned them all.
+// call of 0.117 ms (0.14 with tiles of 2,048); 1.1M cells 0.60 ms, 1.86 when one block scanned them all.
 __global__ void __launch_bounds__(kExportThreads) k_e_export_table(const uint32_t* __restrict__ start,
                                                                    const uint32_t* __restrict__ orig,
                                                                    const SceneDev* __restrict__ sc, uint32_t scene,

@@ -240,7 +240,6 @@ class Engine {
   uint32_t* wet_ = nullptr;  // per cell: the substep epoch of the last substep it held fluid
   uint32_t* start_ = nullptr;
   unsigned long long* scan_ = nullptr;  // k_e_scan: a word per tile
-  uint32_t* export_sums_ = nullptr;     // k_e_export_counts: a word per tile
   // scenes / tiles / control
   SceneDev* sc_d_ = nullptr;
   SceneDev* sc_h_ = nullptr;  // pinned mirror (pushed when dt or membership changes)
