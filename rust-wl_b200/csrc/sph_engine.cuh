@@ -828,7 +828,7 @@ __device__ __forceinline__ void walk27_q(const GridBox& g, const uint32_t* __res
 // holds 8 octant runs, 7 boundaries over kGroupChunk / 32 warps; chunks of 512 slots (tiles
 // of 512) let fewer warps straddle, but cost the grouping pass about as much as they save.
 //
-// It also finds the scenes whose lists go by rows (g.rows, zero before): the first slot of every eighth tile
+// It also finds the scenes whose lists go by rows (g.rows, zero before): the first slot of every eighth chunk
 // looks up how many slots its own plane's entries span, and a span near the 14 bits marks the scene.
 // That is often enough: spans change little from cell to cell, a list that fails all the same is
 // walked again, and 512 slots less than the limit leave room for that. A slot of every warp cost 0.05 ms of the
@@ -841,11 +841,11 @@ static_assert(kGroupChunk % 128 == 0 && kGroupChunk <= 1024, "chunk: 128..1024 s
 
 __device__ __forceinline__ uint32_t octant_rank(uint32_t oct) { return oct ^ (oct >> 1) ^ (oct >> 2); }
 
-__global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restrict__ pos, const SceneDev* __restrict__ sc,
-                                                          const TileDev* __restrict__ tiles, uint32_t ntiles,
-                                                          const EngineCtl* __restrict__ ctl, uint32_t* __restrict__ order,
-                                                          uint32_t* __restrict__ words, uint32_t wstride,
-                                                          const uint32_t* __restrict__ start, SceneDev* mark) {
+// 1,280 threads per SM (48 registers): with 54 the pass is 10% slower.
+__global__ void __launch_bounds__(kGroupChunk, 1280 / kGroupChunk) k_e_groups(
+    const float4* __restrict__ pos, const SceneDev* __restrict__ sc, const TileDev* __restrict__ tiles, uint32_t ntiles,
+    const EngineCtl* __restrict__ ctl, uint32_t* __restrict__ order, uint32_t* __restrict__ words, uint32_t wstride,
+    const uint32_t* __restrict__ start, SceneDev* mark) {
   if (ctl->err & kErrCellCap) return;
   constexpr uint32_t kW = kGroupChunk / 32;  // warps
   constexpr uint32_t kV = 8 * kW / 32;       // (rank, warp) counts per lane of the scan
@@ -855,7 +855,7 @@ __global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restri
   // the block's chunks one after another, each one's positions loaded while the previous
   // one is sorted
   uint32_t t = blockIdx.x, c1 = 0;
-  uint32_t turn = blockIdx.x;  // tiles of this block, begun at its index: every block takes its eighth
+  uint32_t turn = blockIdx.x;  // chunks of this block, counted from its index: the blocks' eighths differ
   TileDev tn = t < ntiles ? tiles[t] : TileDev{};
   float4 pn = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (t < ntiles && threadIdx.x < tn.count) pn = pos[tn.first + threadIdx.x];
@@ -875,7 +875,7 @@ __global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restri
     const float hb = g.bin * 0.5f;
     const uint32_t i = threadIdx.x;
     const bool valid = i < min(kGroupChunk, td.count - c0);
-    if (c0 == 0) ++turn;
+    ++turn;
     uint32_t oct = 0;
     if (valid) {
       uint32_t cx, cy, cz;
@@ -888,7 +888,7 @@ __global__ void __launch_bounds__(kGroupChunk) k_e_groups(const float4* __restri
         words[(size_t)q * wstride + td.first + c0 + i] = sub_word((int)(kSubUnits * side) + bx - 96, by, bz);
         side = side ? side - 1 : 2;
       }
-      if (start && i == 0 && c0 == 0 && (turn & 7u) == 0) {
+      if (start && i == 0 && (turn & 7u) == 0) {
         const uint32_t* row = start + sc[td.scene].cell_off + cz * g.ny * g.nx;
         const uint32_t first = row[(cy > 0 ? cy - 1 : 0) * g.nx + (cx > 0 ? cx - 1 : 0)];
         const uint32_t end = row[min(cy + 1, g.ny - 1u) * g.nx + min(cx + 1, g.nx - 1u) + 1];

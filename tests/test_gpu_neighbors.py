@@ -167,16 +167,18 @@ def test_long_scene_beside_a_short_one(vxl):
                 assert x.tobytes() == y.tobytes(), (t, q)
 
 
-def test_force_pass_of_a_long_scene_is_no_slower_along_x(vxl):
-    """The lists hold whichever way a scene is long: the force pass of a block 900 long in x takes at most twice
-    that of the same block along z (walked again for want of lists it took eight times as long)."""
+@pytest.mark.parametrize("dims,max_bins,tile", [((900, 30, 30), 60000, 256), ((700, 12, 6), 1500, 16384)])
+def test_force_pass_of_a_long_scene_is_no_slower_along_x(vxl, dims, max_bins, tile):
+    """The lists hold whichever way a scene is long and however few tiles it has: the force pass of a block 900 long in
+    x takes at most twice that of the same block along z (walked again for want of lists it took six times as long)."""
     from vxl_sph import scenes
     ms = []
-    for dims in ((900, 30, 30), (30, 30, 900)):
+    for dims in (dims, dims[::-1]):
         s = 0.005
         pos = scenes.jitter(scenes.fluid_block((0.0, 0.0, 0.0), dims, s), s, 1)
-        spec = _custom(vxl, pos, h=2 * s, spacing=s, max_bins=60000)
-        g = vxl.Scene(spec.params, spec.pos, spec.vel, spec.pmass, spec.n_fluid)
+        spec = _custom(vxl, pos, h=2 * s, spacing=s, max_bins=max_bins)
+        g = vxl.Batch([spec])
+        g.set_tuning(256, tile, 0)
         g.substep(1e-5)
         g.set_profile(True)
         for _ in range(5):
