@@ -1499,7 +1499,8 @@ void Engine::enqueue_substep(bool with_reactions) {
       react_pending_ = false;
     }
     if (const uint32_t T = team_lanes(nb_total, kTeamBforce); bforce && T > 1) {
-      auto kernel = T == 8 ? k_e_bforce_team<8> : k_e_bforce_team<4>;
+      auto kernel = rows ? (T == 8 ? k_e_bforce_team<8, true> : k_e_bforce_team<4, true>)
+                         : (T == 8 ? k_e_bforce_team<8, false> : k_e_bforce_team<4, false>);
       LAUNCH_ON(KID_BFORCE, side_,
                 kernel<<<nbtiles_ * (kBoundaryTile / kTeams), kTeams * T, 0, side_>>>(
                     p1, v1, (const float2*)rc_, start_, orig_, nbr_, nbr_n_, nbr_cap_, stride, sc_d_, slot_of_,

@@ -2151,8 +2151,9 @@ __global__ void __launch_bounds__(128) k_e_bforce(
 // neighbours' reference indices are ranked against one another in shared memory instead of
 // inserted one by one, and the pairs' terms formed T at a time and subtracted in order by a lane per
 // component (x - 0 = x: the neutral term). A block is 32 consecutive boundary particles, a
-// word of the wet mask.
-template <uint32_t T>
+// word of the wet mask. kRows: some scene's list entries may go by rows (seven registers more, 1.2 us of a
+// small handle's 55 us substep).
+template <uint32_t T, bool kRows>
 __global__ void __launch_bounds__(kTeams * T) k_e_bforce_team(
     const float4* __restrict__ pos, const float4* __restrict__ vel, const float2* __restrict__ rc,
     const uint32_t* __restrict__ start, const uint32_t* __restrict__ orig, const uint16_t* __restrict__ nbr,
@@ -2195,7 +2196,7 @@ __global__ void __launch_bounds__(kTeams * T) k_e_bforce_team(
         s_key[team][q] = orig[ii];
       }
     };
-    if (g.rows) {
+    if (kRows && g.rows) {
       const ListRows rows = list_rows(g, cst, cx, cy, cz);
       gather([&](uint32_t e) { return rows.slot(e); });
     } else {
